@@ -21,7 +21,7 @@ CSRC = os.path.join(PKG, "csrc")
 LIBDIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIBDIR, "libharmgpu.so")
 SOURCES = ["harm_gpu.cu", "serve.cu", "rdump.cu", "flux_f32.cu"]
-HEADERS = ["harm_device.cuh", "weno5.cuh", "common.cuh", os.path.join(ROOT, "include", "harmgpu.h")]
+HEADERS = ["exact_div.cuh", "harm_device.cuh", "weno5.cuh", "common.cuh", os.path.join(ROOT, "include", "harmgpu.h")]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",

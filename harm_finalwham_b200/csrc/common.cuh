@@ -13,12 +13,14 @@
 namespace hg {
 
 // geometry component offsets
-constexpr int GLOC = 34;                  // per location: gcov 16, gcon 16, gcovpert_tt, gdet
+// per location: gcov 16, gcon 16, gcovpert_tt, gdet, then what derive_metric
+// makes of them: alpha, 1/alpha, beta^1..3, 1/gdet
+constexpr int GLOC = 40;
 constexpr int G_FACE1 = 0, G_FACE2 = 1, G_FACE3 = 2, G_CENT = 3;
 constexpr int G_CORN = 4 * GLOC;          // CORN1, CORN2, CORN3 gdet
 constexpr int G_CONN = G_CORN + 3;        // 64
 constexpr int G_FLOOR = G_CONN + 64;      // 2
-constexpr int G_NCOMP = G_FLOOR + 2;      // 205
+constexpr int G_NCOMP = G_FLOOR + 2;      // 229
 
 // reference location ids (global.h:948-955)
 constexpr int R_FACE1 = 0, R_FACE2 = 1, R_FACE3 = 2, R_CORN1 = 3, R_CORN2 = 4, R_CORN3 = 5, R_CENT = 7;
@@ -114,6 +116,11 @@ __device__ __forceinline__ void load_metric(const double *__restrict__ G, const 
   for (int q = 0; q < 16; q++) m.gcon[q] = __ldg(b + (long long)(16 + q) * d.nij);
   m.gcovpert_tt = __ldg(b + (long long)32 * d.nij);
   m.g = __ldg(b + (long long)33 * d.nij);
+  m.alpha = __ldg(b + (long long)34 * d.nij);
+  m.ralpha = __ldg(b + (long long)35 * d.nij);
+#pragma unroll
+  for (int q = 0; q < 3; q++) m.beta[q] = __ldg(b + (long long)(36 + q) * d.nij);
+  m.rg = __ldg(b + (long long)39 * d.nij);
 }
 
 __device__ __forceinline__ void load_prim(const double *__restrict__ P, const Dims &d, long long z, double *pr) {
@@ -217,14 +224,17 @@ __device__ __forceinline__ void para4(const T *y, T *lout, T *rout) {
 // per SM, B blocks of 128 threads cap a thread at 65536 / (128 B) registers:
 // 1-2 -> 255 (8 warps/SM), 3 -> 170 (12 warps), 4 -> 128 (16 warps), more
 // warps to hide FP64 latency at the price of spills to local memory.
-// Defaults from a B200 sweep (256x128x128 torus, 1/3/4/5 blocks for flux and
-// update): flux 4 (-11% WENO5, -21% MC); update is fastest unconstrained.
+// Measured on the B200, us per step: flux 4 against 3 blocks 3438 / 3679 on
+// the 256x128x128 WENO5 torus, 237 / 259 on 97x51x33 MC, 58 / 54 on 64x64
+// (there the few warps gain nothing from the fourth block and pay its
+// spills); update 4 against 3 blocks 2240 / 1505, 154 / 85, 36 / 27: its
+// spills sit in the contraction with the connection, so 3.
 // The WENO5 kernel runs blocks of 256 threads (W5_THREADS).
 #ifndef HG_MINB_FLUX
 #define HG_MINB_FLUX 4
 #endif
 #ifndef HG_MINB_UPDATE
-#define HG_MINB_UPDATE 4
+#define HG_MINB_UPDATE 3
 #endif
 #ifndef HG_MINB_INVERT
 #define HG_MINB_INVERT 1
@@ -252,7 +262,7 @@ template <> struct MinBlocks<float> {
 // for each heavy kernel; variant 0 is the default above)
 constexpr int kFluxMB[2] = {HG_MINB_FLUX, HG_MINB_FLUX - 1};
 constexpr int kWenoMB[2] = {HG_MINB_WENO, HG_MINB_WENO + 1};
-constexpr int kConserveMB[2] = {HG_MINB_UPDATE, 3};
+constexpr int kConserveMB[2] = {HG_MINB_UPDATE, HG_MINB_UPDATE + 1};
 constexpr int kInvertMB[2] = {HG_MINB_INVERT, 2};
 
 template <int DIR>
@@ -271,6 +281,11 @@ __device__ __forceinline__ void load_metric_t(const double *__restrict__ G, cons
   for (int q = 0; q < 16; q++) m.gcon[q] = (T)__ldg(b + (long long)(16 + q) * d.nij);
   m.gcovpert_tt = (T)__ldg(b + (long long)32 * d.nij);
   m.g = (T)__ldg(b + (long long)33 * d.nij);
+  m.alpha = (T)__ldg(b + (long long)34 * d.nij);
+  m.ralpha = (T)__ldg(b + (long long)35 * d.nij);
+#pragma unroll
+  for (int q = 0; q < 3; q++) m.beta[q] = (T)__ldg(b + (long long)(36 + q) * d.nij);
+  m.rg = (T)__ldg(b + (long long)39 * d.nij);
 }
 
 // ---------------------------------------------------------------------------
@@ -496,7 +511,11 @@ __global__ void __launch_bounds__(W5_THREADS, MB) weno5_kernel(Dims d, Params P,
 // ---------------------------------------------------------------------------
 // MIX = 1: the mixed-precision variant of the FP64 kernel (wave speeds in
 // FP32, vchar_f32; instantiated only in flux_f32.cu, whose FP64 arithmetic
-// may contract a*b+c into FMA)
+// may contract a*b+c into FMA).
+// Bound by FP64 issue and by the registers of two states.  On the
+// 256x128x128 WENO5 torus one direction takes 0.57 ms a launch, 1.14 ms
+// while every quotient was a division of its own and the tensors' zero
+// diagonals and the unit vectors of simplefast were multiplied out.
 template <int DIR, int RECON, typename T, int MB = MinBlocks<T>::flux, typename TR = T, int MIX = 0>
 __global__ void __launch_bounds__(128, MB) flux_kernel(Dims d, Params P, Box box,
                                                                  const double *__restrict__ pb,
@@ -566,9 +585,9 @@ __global__ void __launch_bounds__(128, MB) flux_kernel(Dims d, Params P, Box box
       else err |= vchar(p_l, q, DIR, m, gam, &cmaxl, &cminl);
       if (!ring) {
         EMT<T> e;
-        em_prepare(p_l, m, q, e);
-        primtoflux(p_l, q, e, DIR, m, gam, Fl);
-        primtoflux(p_l, q, e, 0, m, gam, Ul);
+        em_prepare<DIR>(p_l, m, q, e);
+        primtoflux<DIR>(p_l, q, e, m, gam, Fl);
+        primtoflux<0>(p_l, q, e, m, gam, Ul);
       }
     }
     {
@@ -578,9 +597,9 @@ __global__ void __launch_bounds__(128, MB) flux_kernel(Dims d, Params P, Box box
       else err |= vchar(p_r, q, DIR, m, gam, &cmaxr, &cminr);
       if (!ring) {
         EMT<T> e;
-        em_prepare(p_r, m, q, e);
-        primtoflux(p_r, q, e, DIR, m, gam, Fr);
-        primtoflux(p_r, q, e, 0, m, gam, Ur);
+        em_prepare<DIR>(p_r, m, q, e);
+        primtoflux<DIR>(p_r, q, e, m, gam, Fr);
+        primtoflux<0>(p_r, q, e, m, gam, Ur);
       }
     }
     // cminmax_calc (wavespeeds.c:325-385)
@@ -592,18 +611,23 @@ __global__ void __launch_bounds__(128, MB) flux_kernel(Dims d, Params P, Box box
     if (!ring) {
       double Fo[NPR];
       if (P.flux == HGPU_FLUX_HLL && (cmax + cmin != T(0.0))) {
+        T num[NPR], quo[NPR];
 #pragma unroll
-        for (int v = 0; v < NPR; v++)
-          Fo[v] = (double)(((cmax * Fl[v] + cmin * Fr[v]) - (cmax * cmin) * (Ur[v] - Ul[v])) / (cmax + cmin));
+        for (int v = 0; v < NPR; v++) num[v] = (cmax * Fl[v] + cmin * Fr[v]) - (cmax * cmin) * (Ur[v] - Ul[v]);
+        div_n<NPR>(num, make_divisor(cmax + cmin), quo);
+#pragma unroll
+        for (int v = 0; v < NPR; v++) Fo[v] = (double)quo[v];
       } else {
 #pragma unroll
         for (int v = 0; v < NPR; v++) Fo[v] = (double)(T(0.5) * ((Fl[v] + Fr[v]) - ctop * (Ur[v] - Ul[v])));
       }
       // flux_ct gdet strip (fluxct.c:74-96), in FP64 in both precision modes
-      const double gface = __ldg(G + (long long)((DIR - 1) * GLOC + 33) * d.nij + gix(d, i, j));
-      Fo[B1] /= gface;
-      Fo[B2] /= gface;
-      Fo[B3] /= gface;
+      const double *gf = G + (long long)((DIR - 1) * GLOC) * d.nij + gix(d, i, j);
+      double Fs[3];
+      div_n<3>(Fo + B1, known_divisor(__ldg(gf + 33 * d.nij), __ldg(gf + 39 * d.nij)), Fs);
+      Fo[B1] = Fs[0];
+      Fo[B2] = Fs[1];
+      Fo[B3] = Fs[2];
       store_prim(F, d, z, Fo);
     }
     double dxd = (DIR == 1) ? P.dx1 : ((DIR == 2) ? P.dx2 : P.dx3);

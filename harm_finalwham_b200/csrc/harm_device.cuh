@@ -14,6 +14,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "exact_div.cuh"
+
 namespace hg {
 
 constexpr int NPR = 8;
@@ -72,12 +74,19 @@ struct MetricT {
   T gcon[16];
   T gcovpert_tt;
   T g;
+  // functions of the above, formed once per location (derive_metric): the
+  // lapse 1/sqrt(-g^tt) and its reciprocal, the shift g^ti alpha alpha, the
+  // reciprocal of gdet (reciprocals as kept_rcp leaves them)
+  T alpha, ralpha;
+  T beta[3];
+  T rg;
 };
 using Metric = MetricT<double>;
 
 template <typename T>
 struct StateT {
   T ucon[4], ucov[4], bcon[4], bcov[4];
+  Divisor<T> d0;  // u^t, by which b^i, v^i and the Maxwell tensor divide
 };
 using State = StateT<double>;
 
@@ -95,6 +104,16 @@ using EM = EMT<double>;
 #define GCOV(m, a, b) ((m).gcov[(a) * 4 + (b)])
 #define GCON(m, a, b) ((m).gcon[(a) * 4 + (b)])
 
+// alpha and beta^i of ucon_calc_rel4vel (phys.c:983-1019) and the kept
+// reciprocals, from gcon and gdet
+__device__ __forceinline__ void derive_metric(Metric &m) {
+  m.alpha = 1. / sqrt(-GCON(m, 0, 0));
+  m.ralpha = kept_rcp(m.alpha);
+#pragma unroll
+  for (int j = 0; j < 3; j++) m.beta[j] = GCON(m, 0, j + 1) * m.alpha * m.alpha;
+  m.rg = kept_rcp(m.g);
+}
+
 template <typename T>
 __device__ __forceinline__ T dot4(const T *a, const T *b) {
   return a[0] * b[0] + a[1] * b[1] + a[2] * b[2] + a[3] * b[3];
@@ -107,15 +126,6 @@ __device__ __forceinline__ void lower_vec(const T *ucon, const MetricT<T> &m, T 
   ucov[1] = GCOV(m, 0, 1) * ucon[0] + GCOV(m, 1, 1) * ucon[1] + GCOV(m, 1, 2) * ucon[2] + GCOV(m, 1, 3) * ucon[3];
   ucov[2] = GCOV(m, 0, 2) * ucon[0] + GCOV(m, 1, 2) * ucon[1] + GCOV(m, 2, 2) * ucon[2] + GCOV(m, 2, 3) * ucon[3];
   ucov[3] = GCOV(m, 0, 3) * ucon[0] + GCOV(m, 1, 3) * ucon[1] + GCOV(m, 2, 3) * ucon[2] + GCOV(m, 3, 3) * ucon[3];
-}
-
-// raise_vec (phys.c:826-846)
-template <typename T>
-__device__ __forceinline__ void raise_vec(const T *ucov, const MetricT<T> &m, T *ucon) {
-  ucon[0] = GCON(m, 0, 0) * ucov[0] + GCON(m, 0, 1) * ucov[1] + GCON(m, 0, 2) * ucov[2] + GCON(m, 0, 3) * ucov[3];
-  ucon[1] = GCON(m, 0, 1) * ucov[0] + GCON(m, 1, 1) * ucov[1] + GCON(m, 1, 2) * ucov[2] + GCON(m, 1, 3) * ucov[3];
-  ucon[2] = GCON(m, 0, 2) * ucov[0] + GCON(m, 1, 2) * ucov[1] + GCON(m, 2, 2) * ucov[2] + GCON(m, 2, 3) * ucov[3];
-  ucon[3] = GCON(m, 0, 3) * ucov[0] + GCON(m, 1, 3) * ucov[1] + GCON(m, 2, 3) * ucov[2] + GCON(m, 3, 3) * ucov[3];
 }
 
 // qsq_calc (phys.c:1077-1090) on the relative 4-velocity u~^i
@@ -141,16 +151,12 @@ __device__ __forceinline__ int gamma_calc(const T *pr, const MetricT<T> &m, T *g
 // ucon_calc_rel4vel (phys.c:983-1019)
 template <typename T>
 __device__ __forceinline__ int ucon_calc(const T *pr, const MetricT<T> &m, T *ucon) {
-  T alpha = T(1.) / sqrt(-GCON(m, 0, 0));
-  T beta1 = GCON(m, 0, 1) * alpha * alpha;
-  T beta2 = GCON(m, 0, 2) * alpha * alpha;
-  T beta3 = GCON(m, 0, 3) * alpha * alpha;
   T gamma;
   if (gamma_calc(pr, m, &gamma)) return 1;
-  ucon[0] = gamma / alpha;
-  ucon[1] = pr[U1] - ucon[0] * beta1;
-  ucon[2] = pr[U2] - ucon[0] * beta2;
-  ucon[3] = pr[U3] - ucon[0] * beta3;
+  div_n<1>(&gamma, known_divisor(m.alpha, m.ralpha), ucon);
+  ucon[1] = pr[U1] - ucon[0] * m.beta[0];
+  ucon[2] = pr[U2] - ucon[0] * m.beta[1];
+  ucon[3] = pr[U3] - ucon[0] * m.beta[2];
   return 0;
 }
 
@@ -160,26 +166,26 @@ __device__ __forceinline__ int get_state(const T *pr, const MetricT<T> &m, State
   if (ucon_calc(pr, m, q.ucon)) return 1;
   lower_vec(q.ucon, m, q.ucov);
   q.bcon[0] = pr[B1] * q.ucov[1] + pr[B2] * q.ucov[2] + pr[B3] * q.ucov[3];
+  T num[3];
 #pragma unroll
-  for (int j = 1; j <= 3; j++) q.bcon[j] = (pr[B1 - 1 + j] + q.bcon[0] * q.ucon[j]) / q.ucon[0];
+  for (int j = 1; j <= 3; j++) num[j - 1] = pr[B1 - 1 + j] + q.bcon[0] * q.ucon[j];
+  q.d0 = make_divisor(q.ucon[0]);
+  div_n<3>(num, q.d0, q.bcon + 1);
   lower_vec(q.bcon, m, q.bcov);
   return 0;
 }
 
-// compute_1plusud0 (phys.c:541-575)
+// compute_1plusud0 (phys.c:541-575) from v^i = u^i / u^t
 template <typename T>
-__device__ __forceinline__ T compute_1plusud0(const MetricT<T> &m, const StateT<T> &q) {
-  T vcon[4];
-#pragma unroll
-  for (int j = 1; j < 4; j++) vcon[j] = q.ucon[j] / q.ucon[0];
+__device__ __forceinline__ T compute_1plusud0(const MetricT<T> &m, const StateT<T> &q, const T *v) {
   T plus1gv00 = m.gcovpert_tt;
   T vsq = m.gcovpert_tt;
 #pragma unroll
-  for (int j = 1; j < 4; j++) vsq += T(2.0) * GCOV(m, 0, j) * vcon[j];
+  for (int j = 1; j < 4; j++) vsq += T(2.0) * GCOV(m, 0, j) * v[j - 1];
 #pragma unroll
   for (int j = 1; j < 4; j++)
 #pragma unroll
-    for (int k = 1; k < 4; k++) vsq += GCOV(m, j, k) * vcon[j] * vcon[k];
+    for (int k = 1; k < 4; k++) vsq += GCOV(m, j, k) * v[j - 1] * v[k - 1];
   T gvtt = GCOV(m, 0, 0);
   T alpha = T(0.0);
 #pragma unroll
@@ -187,27 +193,49 @@ __device__ __forceinline__ T compute_1plusud0(const MetricT<T> &m, const StateT<
   T uu0 = q.ucon[0];
   return alpha + ((T(1.0) - gvtt) * plus1gv00 - uu0 * uu0 * vsq * gvtt * gvtt) / (T(1.0) - gvtt * uu0);
 }
+template <typename T>
+__device__ __forceinline__ T compute_1plusud0(const MetricT<T> &m, const StateT<T> &q) {
+  T v[3];
+  div_n<3>(q.ucon + 1, q.d0, v);
+  return compute_1plusud0(m, q, v);
+}
 
 // Mcon_calc PRIMMAXWELL (phys.c:178-210), lower_A (phys.ffde.c:1707-1735),
-// Msq (phys.ffde.c:1507) and 1+u_t
-template <typename T>
+// Msq (phys.ffde.c:1507) and 1+u_t.
+// The reference's 4x4 loops run over the zero diagonals of both tensors and
+// form each spatial pair twice.  Here the diagonal terms, which add +-0 to
+// sums that hold no -0, are left out, and a pair is divided once: the other
+// order is its exact negative.  The pairs are formed as (j, DIR), the order
+// in which the induction flux of direction DIR takes them, so that its zeros
+// keep their sign; the sums below do not depend on the sign of a zero.
+template <int DIR, typename T>
 __device__ __forceinline__ void em_prepare(const T *pr, const MetricT<T> &m, const StateT<T> &q, EMT<T> &e) {
-#pragma unroll
-  for (int j = 0; j < 4; j++) e.Mcon[j][j] = T(0.0);
 #pragma unroll
   for (int k = 1; k < 4; k++) {
     e.Mcon[k][0] = pr[B1 + k - 1];
     e.Mcon[0][k] = -e.Mcon[k][0];
   }
+  // numerators over u^t: the three pairs, then u^i
+  constexpr int PJ[3] = {DIR == 1 ? 2 : 1, DIR == 1 ? 3 : (DIR == 2 ? 3 : (DIR == 3 ? 2 : 1)), DIR == 3 ? 1 : (DIR == 2 ? 1 : 2)};
+  constexpr int PK[3] = {DIR == 1 ? 1 : (DIR == 2 ? 2 : (DIR == 3 ? 3 : 2)), DIR == 1 ? 1 : (DIR == 2 ? 2 : 3), DIR == 3 ? 2 : 3};
+  T num[6], quo[6];
 #pragma unroll
-  for (int j = 1; j < 4; j++)
+  for (int c = 0; c < 3; c++) {
+    num[c] = pr[B1 + PJ[c] - 1] * q.ucon[PK[c]] - pr[B1 + PK[c] - 1] * q.ucon[PJ[c]];
+    num[3 + c] = q.ucon[1 + c];
+  }
+  div_n<6>(num, q.d0, quo);
 #pragma unroll
-    for (int k = 1; k < 4; k++) e.Mcon[j][k] = (pr[B1 + j - 1] * q.ucon[k] - pr[B1 + k - 1] * q.ucon[j]) / q.ucon[0];
+  for (int c = 0; c < 3; c++) {
+    e.Mcon[PJ[c]][PK[c]] = quo[c];
+    e.Mcon[PK[c]][PJ[c]] = -quo[c];
+  }
   T a01 = T(0.), a02 = T(0.), a03 = T(0.), a12 = T(0.), a23 = T(0.), a31 = T(0.);
 #pragma unroll
   for (int j = 0; j < 4; j++)
 #pragma unroll
     for (int k = 0; k < 4; k++) {
+      if (j == k) continue;
       T A = e.Mcon[j][k];
       a01 += (GCOV(m, 0, j)) * (GCOV(m, 1, k)) * A;
       a02 += (GCOV(m, 0, j)) * (GCOV(m, 2, k)) * A;
@@ -216,10 +244,6 @@ __device__ __forceinline__ void em_prepare(const T *pr, const MetricT<T> &m, con
       a23 += (GCOV(m, 2, j)) * (GCOV(m, 3, k)) * A;
       a31 += (GCOV(m, 3, j)) * (GCOV(m, 1, k)) * A;
     }
-  e.Mcov[0][0] = T(0.);
-  e.Mcov[1][1] = T(0.);
-  e.Mcov[2][2] = T(0.);
-  e.Mcov[3][3] = T(0.);
   e.Mcov[0][1] = a01;
   e.Mcov[0][2] = a02;
   e.Mcov[0][3] = a03;
@@ -236,28 +260,32 @@ __device__ __forceinline__ void em_prepare(const T *pr, const MetricT<T> &m, con
 #pragma unroll
   for (int j = 0; j < 4; j++)
 #pragma unroll
-    for (int k = 0; k < 4; k++) Msq += e.Mcov[j][k] * e.Mcon[j][k];
+    for (int k = 0; k < 4; k++)
+      if (j != k) Msq += e.Mcov[j][k] * e.Mcon[j][k];
   e.Msq = Msq;
-  e.plus1ud0 = compute_1plusud0(m, q);
+  e.plus1ud0 = compute_1plusud0(m, q, quo + 3);
 }
 
 // mhd_calc_norestmass (phys.c:442-506) + ffdestresstensor_dir
-// (phys.ffde.c:1483-1515): one row T^dir_mu without rest mass
+// (phys.ffde.c:1483-1515): one row T^dir_mu without rest mass (the terms
+// with a Kronecker delta or a zero diagonal only where they are not zero)
 template <typename T>
 __device__ __forceinline__ void mhd_row(const T *pr, int dir, T gam, const StateT<T> &q, const EMT<T> &e, T *mhd) {
   T rho = pr[RHO], u = pr[UU];
   T P = (gam - T(1.)) * u;
   T w = P + rho + u;
   T eta = w, ptot = P;
-  mhd[0] = (P + u) * q.ucon[dir] * q.ucov[0] + rho * q.ucon[dir] * e.plus1ud0 + ptot * ((dir == 0) ? T(1.) : T(0.));
+  mhd[0] = (P + u) * q.ucon[dir] * q.ucov[0] + rho * q.ucon[dir] * e.plus1ud0;
 #pragma unroll
-  for (int j = 1; j < 4; j++) mhd[j] = eta * q.ucon[dir] * q.ucov[j] + ptot * ((dir == j) ? T(1.) : T(0.));
+  for (int j = 1; j < 4; j++) mhd[j] = eta * q.ucon[dir] * q.ucov[j];
+  mhd[dir] += ptot;
   T TEM[4];
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     TEM[j] = T(0.);
 #pragma unroll
-    for (int i = 0; i < 4; i++) TEM[j] += e.Mcon[dir][i] * e.Mcov[j][i];
+    for (int i = 0; i < 4; i++)
+      if (i != dir && i != j) TEM[j] += e.Mcon[dir][i] * e.Mcov[j][i];
   }
   TEM[dir] -= T(0.25) * e.Msq;
 #pragma unroll
@@ -265,16 +293,17 @@ __device__ __forceinline__ void mhd_row(const T *pr, int dir, T gam, const State
 }
 
 // primtoflux (phys.c:16-55), UEVOLVE, every EOM factor = gdet
-template <typename T>
-__device__ __forceinline__ void primtoflux(const T *pr, const StateT<T> &q, const EMT<T> &e, int dir,
-                                           const MetricT<T> &m, T gam, T *flux) {
+// (the induction flux of direction dir is the column (j, dir) of Mcon, for
+// which e is prepared; its own component is u^dir B^dir - u^dir B^dir)
+template <int dir, typename T>
+__device__ __forceinline__ void primtoflux(const T *pr, const StateT<T> &q, const EMT<T> &e, const MetricT<T> &m,
+                                           T gam, T *flux) {
   T fin[NPR];
   fin[RHO] = pr[RHO] * q.ucon[dir];
   mhd_row(pr, dir, gam, q, e, &fin[UU]);
   if (dir > 0) {
-    fin[B1] = (pr[B1] * q.ucon[dir] - pr[B1 + dir - 1] * q.ucon[1]) / q.ucon[0];
-    fin[B2] = (pr[B2] * q.ucon[dir] - pr[B1 + dir - 1] * q.ucon[2]) / q.ucon[0];
-    fin[B3] = (pr[B3] * q.ucon[dir] - pr[B1 + dir - 1] * q.ucon[3]) / q.ucon[0];
+#pragma unroll
+    for (int j = 1; j < 4; j++) fin[B1 + j - 1] = (j == dir) ? T(0.) : e.Mcon[j][dir];
   } else {
     fin[B1] = pr[B1];
     fin[B2] = pr[B2];
@@ -288,16 +317,12 @@ __device__ __forceinline__ void primtoflux(const T *pr, const StateT<T> &q, cons
 template <typename T>
 __device__ __forceinline__ int simplefast(int dir, const MetricT<T> &m, const StateT<T> &q, T cms2, T *vmin,
                                           T *vmax) {
-  T Acov[4] = {T(0.), T(0.), T(0.), T(0.)}, Bcov[4] = {T(0.), T(0.), T(0.), T(0.)}, Acon[4], Bcon[4];
-  Acov[dir] = T(1.);
-  raise_vec(Acov, m, Acon);
-  Bcov[0] = T(1.);
-  raise_vec(Bcov, m, Bcon);
-  T Asq = dot4(Acon, Acov);
-  T Bsq = dot4(Bcon, Bcov);
-  T Au = dot4(Acov, q.ucon);
-  T Bu = dot4(Bcov, q.ucon);
-  T AB = dot4(Acon, Bcov);
+  // raise_vec and dot4 of the unit vectors
+  T Asq = GCON(m, dir, dir);
+  T Bsq = GCON(m, 0, 0);
+  T Au = q.ucon[dir];
+  T Bu = q.ucon[0];
+  T AB = GCON(m, 0, dir);
   T Au2 = Au * Au;
   T Bu2 = Bu * Bu;
   T AuBu = Au * Bu;
@@ -308,8 +333,9 @@ __device__ __forceinline__ int simplefast(int dir, const MetricT<T> &m, const St
   if ((discr < T(0.0)) && (discr > -Tol<T>::discr)) discr = T(0.0);
   else if (discr < T(0.0)) return ERR_VCHAR_DISCR;
   discr = sqrt(discr);
-  T vm = -(-B + discr) / (T(2.) * A);
-  T vp = -(-B - discr) / (T(2.) * A);
+  T num[2] = {-(-B + discr), -(-B - discr)}, v[2];
+  div_n<2>(num, make_divisor(T(2.) * A), v);
+  const T vm = v[0], vp = v[1];
   if ((!isfinite(vm)) || (!isfinite(vp))) return ERR_NONFINITE_SPEED;
   if (vp < vm) {
     *vmax = vm;
@@ -437,10 +463,9 @@ __device__ __forceinline__ void func_vsq2(const U2P &c, double W, double vsq, do
   double wmrho0 = (Wp / gammasq - D * vsq / (1.0 + gamma));
   double igr = (c.gam - 1.0) / c.gam;
   double p_tmp = igr * wmrho0;
-  double dPdW = 0.0 * 0.0 + (1.0 - vsq) * igr;
+  double dPdW = (1.0 - vsq) * igr;
   double dwmrho0dvsq = (D * (gamma * 0.5 - 1.0) - Wp);
-  double drho0dvsq = -D * gamma * 0.5;
-  double dPdvsq = drho0dvsq * 0.0 + dwmrho0dvsq * igr;
+  double dPdvsq = dwmrho0dvsq * igr;
   double Bsq = c.Bsq, QdotBsq = c.QdotBsq, Qtsq = c.Qtsq, Qdotn = c.Qdotn;
   double t2 = -0.5 * Bsq + dPdvsq;
   double t3 = Bsq + W;
@@ -477,27 +502,25 @@ __device__ __forceinline__ int utoprimgen(const double *U, const Metric &m, doub
   c.vsq_too_big = (c.gammasq_too_big - 1.0) / (c.gammasq_too_big);
   double Ugf[NPR], Ut[NPR];
   // UtoU(UEVOLVE->UNOTHING) and rest-mass convention (utoprimgen.c:55,76-85)
-#pragma unroll
-  for (int pl = 0; pl < NPR; pl++) Ugf[pl] = U[pl] / m.g;
+  div_n<NPR>(U, known_divisor(m.g, m.rg), Ugf);
   Ugf[UU] -= Ugf[RHO];
   // Utoprim_2d_final (utoprim_2d_final.c:34-117)
   prim[B1] = Ugf[B1];
   prim[B2] = Ugf[B2];
   prim[B3] = Ugf[B3];
-  double alpha = 1.0 / sqrt(-GCON(m, 0, 0));
 #pragma unroll
-  for (int i = 0; i < NPR; i++) Ut[i] = alpha * Ugf[i];
+  for (int i = 0; i < NPR; i++) Ut[i] = m.alpha * Ugf[i];
   // Utoprim_new_body (:152-453)
-  double Bcon[4], Bcov[4], Qcov[4], Qcon[4], ncov[4], ncon[4];
+  double Bcon[4], Bcov[4], Qcov[4], Qcon[4], ncov[1], ncon[4];
   Bcon[0] = 0.;
   Bcon[1] = Ut[B1];
   Bcon[2] = Ut[B2];
   Bcon[3] = Ut[B3];
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
+  for (int i = 1; i < 4; i++) {
     double s = 0.;
 #pragma unroll
-    for (int j = 0; j < 4; j++) s += GCOV(m, i, j) * Bcon[j];
+    for (int j = 1; j < 4; j++) s += GCOV(m, i, j) * Bcon[j];
     Bcov[i] = s;
   }
 #pragma unroll
@@ -515,20 +538,12 @@ __device__ __forceinline__ int utoprimgen(const double *U, const Metric &m, doub
   c.Bsq = Bsq;
   double QdotB = 0.;
 #pragma unroll
-  for (int i = 0; i < 4; i++) QdotB += Qcov[i] * Bcon[i];
+  for (int i = 1; i < 4; i++) QdotB += Qcov[i] * Bcon[i];
   c.QdotBsq = QdotB * QdotB;
   double lapse = sqrt(-1. / GCON(m, 0, 0));
   ncov[0] = -lapse;
-  ncov[1] = 0.;
-  ncov[2] = 0.;
-  ncov[3] = 0.;
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    double s = 0.;
-#pragma unroll
-    for (int j = 0; j < 4; j++) s += GCON(m, i, j) * ncov[j];
-    ncon[i] = s;
-  }
+  for (int i = 0; i < 4; i++) ncon[i] = 0. + GCON(m, i, 0) * ncov[0];
   c.Qdotn = Qcon[0] * ncov[0];
   double Qsq = 0.;
 #pragma unroll
@@ -669,8 +684,8 @@ __device__ __forceinline__ void jon_func(const JonU2P &c, double Wp, double *res
   const double W3 = Wsq * W;
   const double X3v = Xv * Xv * Xv;
   const double dvsq = -2. * (c.Qtsq / X3v + c.QdotBsq * (3.0 * W * Xv + c.Bsq * c.Bsq) / (W3 * X3v));
-  const double dp1 = 0.0 * 0.0 + (1.0 / gammasq) * c.igammar;
-  const double dp2 = (-D * gamma * 0.5) * 0.0 + (D * (gamma * 0.5 - 1.0) - Wp) * c.igammar;
+  const double dp1 = (1.0 / gammasq) * c.igammar;
+  const double dp2 = (D * (gamma * 0.5 - 1.0) - Wp) * c.igammar;
   const double dpdWp = dp1 + dp2 * dvsq;
   const double X3 = X * X * X;
   const double drdW = (1.0 - dpdWp) - (c.Bsq * c.Qtsq - c.QdotBsq) / X3;
@@ -703,30 +718,28 @@ __device__ __forceinline__ int utoprimgen_jon(const double *U, const Metric &m, 
   double Ut[NPR], pt[NPR];
   // UtoU(UEVOLVE->UNOTHING); U[UU] stays without rest mass (utoprimgen.c:76-85)
   double Ugf[NPR];
-#pragma unroll
-  for (int pl = 0; pl < NPR; pl++) Ugf[pl] = U[pl] / m.g;
+  div_n<NPR>(U, known_divisor(m.g, m.rg), Ugf);
   prim[B1] = Ugf[B1];
   prim[B2] = Ugf[B2];
   prim[B3] = Ugf[B3];
-  const double alpha = 1.0 / sqrt(-GCON(m, 0, 0));
 #pragma unroll
-  for (int i = 0; i < NPR; i++) Ut[i] = alpha * Ugf[i];
+  for (int i = 0; i < NPR; i++) Ut[i] = m.alpha * Ugf[i];
 #pragma unroll
   for (int i = 0; i < B1; i++) pt[i] = prim[i];
 #pragma unroll
   for (int i = B1; i <= B3; i++) pt[i] = Ut[i];
   // compute_setup_quantities (:494-636)
   c.D = Ut[RHO];
-  double Bcon[4], Bcov[4], ncov[4], ncon[4], Qconp[4], Qcov[4], Qtcon[4];
+  double Bcon[4], Bcov[4], ncov[1], ncon[4], Qconp[4], Qcov[4], Qtcon[4];
   Bcon[0] = 0.;
   Bcon[1] = Ut[B1];
   Bcon[2] = Ut[B2];
   Bcon[3] = Ut[B3];
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
+  for (int i = 1; i < 4; i++) {
     double s = 0.;
 #pragma unroll
-    for (int j = 0; j < 4; j++) s += GCOV(m, i, j) * Bcon[j];
+    for (int j = 1; j < 4; j++) s += GCOV(m, i, j) * Bcon[j];
     Bcov[i] = s;
   }
   double Bsq = 0.;
@@ -735,16 +748,8 @@ __device__ __forceinline__ int utoprimgen_jon(const double *U, const Metric &m, 
   c.Bsq = Bsq;
   const double lapse = sqrt(-1. / GCON(m, 0, 0));
   ncov[0] = -lapse;
-  ncov[1] = 0.;
-  ncov[2] = 0.;
-  ncov[3] = 0.;
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    double s = 0.;
-#pragma unroll
-    for (int j = 0; j < 4; j++) s += GCON(m, i, j) * ncov[j];
-    ncon[i] = s;
-  }
+  for (int i = 0; i < 4; i++) ncon[i] = 0. + GCON(m, i, 0) * ncov[0];
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     double s = 0.;

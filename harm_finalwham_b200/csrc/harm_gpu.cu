@@ -5,8 +5,9 @@
 //   primitives, conserved accumulators, fluxes: SoA planes [8][nt1][nt2][nt3]
 //     with x3 fastest, so that the 32 threads of a warp walk x3 at one (i,j)
 //     and read one metric row (broadcast) -- the metric depends on (i,j) only.
-//   geometry: SoA [component][gt1*gt2], 205 doubles per (i,j):
-//     4 locations (FACE1, FACE2, FACE3, CENT) x {gcov 16, gcon 16, gcovpert_tt, gdet},
+//   geometry: SoA [component][gt1*gt2], 229 doubles per (i,j):
+//     4 locations (FACE1, FACE2, FACE3, CENT) x {gcov 16, gcon 16, gcovpert_tt, gdet,
+//     lapse, 1/lapse, shift 3, 1/gdet},
 //     CORN1..3 gdet, conn[64] at CENT, floors[2].
 //
 // Work per RK substep (the reference's advance(), step_ch.c:94-186):
@@ -35,6 +36,7 @@
 
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -182,8 +184,8 @@ __device__ __forceinline__ void fv_diag_fixup(const double *pr0, const double *p
       *err |= ERR_UTCALC_DISCR;
       return;
     }
-    em_prepare(pr0, m, q, e);
-    primtoflux(pr0, q, e, 0, m, gam, Ui);
+    em_prepare<0>(pr0, m, q, e);
+    primtoflux<0>(pr0, q, e, m, gam, Ui);
   }
   {
     State q;
@@ -192,8 +194,8 @@ __device__ __forceinline__ void fv_diag_fixup(const double *pr0, const double *p
       *err |= ERR_UTCALC_DISCR;
       return;
     }
-    em_prepare(pr, m, q, e);
-    primtoflux(pr, q, e, 0, m, gam, Uf);
+    em_prepare<0>(pr, m, q, e);
+    primtoflux<0>(pr, q, e, m, gam, Uf);
   }
 #pragma unroll
   for (int pl = 0; pl < NPR; pl++) {
@@ -227,8 +229,8 @@ __global__ void pi2u_kernel(Dims d, Params P, const double *__restrict__ p, cons
     atomicOr(&sc->err, ERR_UTCALC_DISCR);
     return;
   }
-  em_prepare(pr, m, q, e);
-  primtoflux(pr, q, e, 0, m, P.gam, U);
+  em_prepare<0>(pr, m, q, e);
+  primtoflux<0>(pr, q, e, m, P.gam, U);
 #pragma unroll
   for (int pl = 0; pl < NPR; pl++) u[pl * d.nz + z] = U[pl];
 }
@@ -264,23 +266,19 @@ __device__ __forceinline__ void source_conn(const Dims &d, const double *__restr
   // dU = sum of the NUMSOURCES components; only GEOMSOURCE is nonzero
   double full[NPR] = {0., dUconn[0], dUconn[1], dUconn[2], dUconn[3], 0., 0., 0.};
 #pragma unroll
-  for (int pl = 0; pl < NPR; pl++) {
-    double comp0 = 0. + m.g * full[pl];
-    double acc = 0.;
-    acc += comp0;
-#pragma unroll
-    for (int l = 1; l < 7; l++) acc += 0.0;
-    dUg[pl] = acc;
-  }
+  for (int pl = 0; pl < NPR; pl++) dUg[pl] = (pl >= UU && pl <= U3) ? 0. + m.g * full[pl] : 0.;
 }
 
+// Bound by FP64 issue and registers: 0.75 ms a launch on 256x128x128 (RK2),
+// 1.37 ms with the tensors' zero diagonals multiplied out, every quotient a
+// division, 4 blocks per SM and both accumulators moved in each stage.
 template <int MB>
 __global__ void __launch_bounds__(128, MB) conserve_kernel(
     Dims d, Params P, Box box, const double *pi, const double *pb, double *__restrict__ uf,
     double *__restrict__ ucum, const double *__restrict__ F1, const double *__restrict__ F2,
     const double *__restrict__ F3, const double *__restrict__ E, const double *__restrict__ G, Scalars *sc,
     double CUf0, double CUf1, double CUf2, double Cunew0, double Cunew1, double Cunew2, int timeorder,
-    double *__restrict__ ui, int fv) {
+    double *__restrict__ ui, int fv, int read_uf, int read_ucum, int write_uf) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= box.size()) return;
   int i, j, k;
@@ -350,7 +348,7 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
       State q;
       EM e;
       if (get_state(pbz, m, q)) err |= ERR_UTCALC_DISCR;
-      em_prepare(pbz, m, q, e);
+      em_prepare<0>(pbz, m, q, e);
       source_conn(d, G, ij, pbz, q, e, m, gam, dUg);
     } else if (pi == pb) {
       // a first substep: U(pi) and the source read the same state, whose
@@ -360,8 +358,8 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
       State q;
       EM e;
       if (get_state(pbz, m, q)) err |= ERR_UTCALC_DISCR;
-      em_prepare(pbz, m, q, e);
-      primtoflux(pbz, q, e, 0, m, gam, Ui);
+      em_prepare<0>(pbz, m, q, e);
+      primtoflux<0>(pbz, q, e, m, gam, Ui);
       source_conn(d, G, ij, pbz, q, e, m, gam, dUg);
     } else {
       {
@@ -370,33 +368,38 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
         State qi;
         EM ei;
         if (get_state(pr, m, qi)) err |= ERR_UTCALC_DISCR;
-        em_prepare(pr, m, qi, ei);
-        primtoflux(pr, qi, ei, 0, m, gam, Ui);
+        em_prepare<0>(pr, m, qi, ei);
+        primtoflux<0>(pr, qi, ei, m, gam, Ui);
       }
       double pbz[NPR];
       load_prim(pb, d, z, pbz);
       State q;
       EM e;
       if (get_state(pbz, m, q)) err |= ERR_UTCALC_DISCR;
-      em_prepare(pbz, m, q, e);
+      em_prepare<0>(pbz, m, q, e);
       source_conn(d, G, ij, pbz, q, e, m, gam, dUg);
     }
     // dUtoU (advance.c:922-949)
     double Uf[NPR], Ucum[NPR];
 #pragma unroll
     for (int pl = 0; pl < NPR; pl++) {
-      double ufo = (timeorder == 0) ? 0.0 : uf[pl * nz + z];
-      double uco = (timeorder == 0) ? 0.0 : ucum[pl * nz + z];
+      const double ufo = read_uf ? uf[pl * nz + z] : 0.0;
+      const double uco = read_ucum ? ucum[pl * nz + z] : 0.0;
       Uf[pl] = CUf0 * Ui[pl] + CUf1 * ufo + CUf2 * dt * (dUr[pl] + dUg[pl]);
       Ucum[pl] = uco + (Cunew0 * Ui[pl] + Cunew1 * dt * (dUr[pl] + dUg[pl]) + Cunew2 * Uf[pl]);
-      uf[pl * nz + z] = Uf[pl];
+      if (write_uf) uf[pl * nz + z] = Uf[pl];
       ucum[pl * nz + z] = Ucum[pl];
     }
     if (err) atomicOr(&sc->err, err);
 }
 
-template <int UV, int MB>
-__global__ void __launch_bounds__(128, MB) invert_kernel(Dims d, Params P, Box box, const double *pb,
+// FV: the finite-volume scheme, whose diag_fixup forms two more conserved
+// states.  Inlined for every scheme it held the kernel at 246 registers
+// (8 warps per SM) where the inversion itself needs about 120: 0.70 -> 0.36
+// ms a launch on 256x128x128.  With it, 3 blocks spill 140 B in the branch
+// of the floored zones: 83 -> 58 us a launch on 128x64x32 (RK4, Jon).
+template <int UV, int MB, bool FV>
+__global__ void __launch_bounds__(128, FV ? 3 : MB) invert_kernel(Dims d, Params P, Box box, const double *pb,
                                                                      double *pf, const double *__restrict__ uf,
                                                                      const double *__restrict__ ucum,
                                                                      const double *__restrict__ G,
@@ -449,7 +452,7 @@ __global__ void __launch_bounds__(128, MB) invert_kernel(Dims d, Params P, Box b
       if (lg == -1) ffc_count(P, nz, z, CNT_LIMITGAMMAACT);
       if (lg < 1 && (floored || lg == -1)) ffc_count(P, nz, z, CNT_FLOORACT);
       // diag_fixup (fixup.c:443) when fixup1zone changed the primitives
-      if (ufv && lg < 1 && (floored || lg == -1)) fv_diag_fixup(pr0, pr, m, gam, ufv, z, nz, &err);
+      if (FV && ufv && lg < 1 && (floored || lg == -1)) fv_diag_fixup(pr0, pr, m, gam, ufv, z, nz, &err);
     }
     store_prim(pf, d, z, pr);
     pflag[z] = flag;
@@ -1331,6 +1334,16 @@ __global__ void pack_geometry_kernel(const double *__restrict__ raw, long long n
     }
     G[(long long)(s * GLOC + 32) * nij + ij] = rpert[(ij * 8 + L) * 4 + 0];
     G[(long long)(s * GLOC + 33) * nij + ij] = rgdet[ij * 8 + L];
+    Metric m;
+#pragma unroll
+    for (int q = 0; q < 4; q++) m.gcon[q] = rcon[(ij * 8 + L) * 16 + q];
+    m.g = rgdet[ij * 8 + L];
+    derive_metric(m);
+    G[(long long)(s * GLOC + 34) * nij + ij] = m.alpha;
+    G[(long long)(s * GLOC + 35) * nij + ij] = m.ralpha;
+#pragma unroll
+    for (int q = 0; q < 3; q++) G[(long long)(s * GLOC + 36 + q) * nij + ij] = m.beta[q];
+    G[(long long)(s * GLOC + 39) * nij + ij] = m.rg;
   }
   G[(long long)(G_CORN + 0) * nij + ij] = rgdet[ij * 8 + R_CORN1];
   G[(long long)(G_CORN + 1) * nij + ij] = rgdet[ij * 8 + R_CORN2];
@@ -1359,6 +1372,7 @@ __global__ void utoprim_batch_kernel(const double *__restrict__ U, const double 
     }
     m.gcovpert_tt = 0.0;
     m.g = gdet[t];
+    derive_metric(m);
     double u[NPR], p[NPR];
 #pragma unroll
     for (int v = 0; v < NPR; v++) {
@@ -2212,29 +2226,30 @@ static void launch_stage_advance(hgpu_ctx *x, int timeorder) {
   launch_fluxes(x, pb);
   const int fv = (x->cfg.doenoflux == HGPU_ENOFINITEVOLUME);
   double *ufv = (fv && finalstep) ? x->ucum : nullptr;
-  if (x->tune.conserve)
-    LAUNCH(x, K_UPDATE, conserve_kernel<kConserveMB[1]>, grid_for(x->active_box.size(), 128), 128, d, x->P,
-           x->active_box, pi, pb, x->uf, x->ucum, x->F[1], x->F[2], x->F[3], x->E, x->G, x->sc, CUf0, CUf1, CUf2, Cn0,
-           Cn1, Cn2, timeorder, x->ui, fv);
-  else
-    LAUNCH(x, K_UPDATE, conserve_kernel<kConserveMB[0]>, grid_for(x->active_box.size(), 128), 128, d, x->P,
-           x->active_box, pi, pb, x->uf, x->ucum, x->F[1], x->F[2], x->F[3], x->E, x->G, x->sc, CUf0, CUf1, CUf2, Cn0,
-           Cn1, Cn2, timeorder, x->ui, fv);
+  // ulast and ucum enter a stage only where an earlier one left them other
+  // than zero, and uf is read by later stages and the intermediate inversion
+  // alone: what no one reads is not moved (RK2: 128 of 256 bytes a zone and step)
+  bool read_ucum = false;
+  for (int o = 0; o < timeorder; o++) {
+    const RKStage &E = rk_stage(x, o);
+    read_ucum |= E.cun[0] != 0.0 || E.cun[1] != 0.0 || E.cun[2] != 0.0;
+  }
+  const int read_uf = timeorder > 0 && CUf1 != 0.0, write_uf = !finalstep;
+  auto update = x->tune.conserve ? conserve_kernel<kConserveMB[1]> : conserve_kernel<kConserveMB[0]>;
+  LAUNCH(x, K_UPDATE, update, grid_for(x->active_box.size(), 128), 128, d, x->P, x->active_box, pi, pb, x->uf, x->ucum,
+         x->F[1], x->F[2], x->F[3], x->E, x->G, x->sc, CUf0, CUf1, CUf2, Cn0, Cn1, Cn2, timeorder, x->ui, fv, read_uf,
+         (int)read_ucum, write_uf);
   {
     const unsigned gi = grid_for(x->active_box.size(), 128);
     const bool jon = x->cfg.utoprimversion == HGPU_UTOPRIMJONNONRELCOMPAT;
-    if (jon && x->tune.invert)
-      LAUNCH(x, K_INVERT, (invert_kernel<8, kInvertMB[1]>), gi, 128, d, x->P, x->active_box, pb, pf, x->uf, x->ucum,
-             x->G, x->pflag, x->sc, finalstep, ufv);
-    else if (jon)
-      LAUNCH(x, K_INVERT, (invert_kernel<8, kInvertMB[0]>), gi, 128, d, x->P, x->active_box, pb, pf, x->uf, x->ucum,
-             x->G, x->pflag, x->sc, finalstep, ufv);
-    else if (x->tune.invert)
-      LAUNCH(x, K_INVERT, (invert_kernel<6, kInvertMB[1]>), gi, 128, d, x->P, x->active_box, pb, pf, x->uf, x->ucum,
-             x->G, x->pflag, x->sc, finalstep, ufv);
-    else
-      LAUNCH(x, K_INVERT, (invert_kernel<6, kInvertMB[0]>), gi, 128, d, x->P, x->active_box, pb, pf, x->uf, x->ucum,
-             x->G, x->pflag, x->sc, finalstep, ufv);
+    auto pick = [&](auto fvc) {
+      constexpr bool FV = decltype(fvc)::value;
+      if (jon) return x->tune.invert ? invert_kernel<8, kInvertMB[1], FV> : invert_kernel<8, kInvertMB[0], FV>;
+      return x->tune.invert ? invert_kernel<6, kInvertMB[1], FV> : invert_kernel<6, kInvertMB[0], FV>;
+    };
+    auto invert = fv ? pick(std::true_type{}) : pick(std::false_type{});
+    LAUNCH(x, K_INVERT, invert, gi, 128, d, x->P, x->active_box, pb, pf, x->uf, x->ucum, x->G, x->pflag, x->sc, finalstep,
+           ufv);
   }
   launch_bound(x, pf);
   // post_fixup (fixup.c:37-96)
@@ -2635,8 +2650,8 @@ __global__ void __launch_bounds__(DIAG_BLOCK) diag_kernel(Dims d, Params P, Box 
       State q;
       EM e;
       get_state(pr, m, q);
-      em_prepare(pr, m, q, e);
-      primtoflux(pr, q, e, 0, m, P.gam, U);
+      em_prepare<0>(pr, m, q, e);
+      primtoflux<0>(pr, q, e, m, P.gam, U);
     }
     double dV = P.dx1 * P.dx2 * P.dx3;
 #pragma unroll
