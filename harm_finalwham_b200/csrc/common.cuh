@@ -229,7 +229,6 @@ __device__ __forceinline__ void para4(const T *y, T *lout, T *rout) {
 // (there the few warps gain nothing from the fourth block and pay its
 // spills); update 4 against 3 blocks 2240 / 1505, 154 / 85, 36 / 27: its
 // spills sit in the contraction with the connection, so 3.
-// The WENO5 kernel runs blocks of 256 threads (W5_THREADS).
 #ifndef HG_MINB_FLUX
 #define HG_MINB_FLUX 4
 #endif
@@ -240,7 +239,7 @@ __device__ __forceinline__ void para4(const T *y, T *lout, T *rout) {
 #define HG_MINB_INVERT 1
 #endif
 #ifndef HG_MINB_WENO
-#define HG_MINB_WENO 3
+#define HG_MINB_WENO 4
 #endif
 // the same for the FP32 kernels of the mixed-precision path (B200 sweep of
 // 4/6/8 for flux: 8 -4%)
@@ -261,7 +260,7 @@ template <> struct MinBlocks<float> {
 // the FP64 variants the autotuner chooses between (resident blocks per SM
 // for each heavy kernel; variant 0 is the default above)
 constexpr int kFluxMB[2] = {HG_MINB_FLUX, HG_MINB_FLUX - 1};
-constexpr int kWenoMB[2] = {HG_MINB_WENO, HG_MINB_WENO + 1};
+constexpr int kWenoMB[2] = {HG_MINB_WENO, HG_MINB_WENO - 1};
 constexpr int kConserveMB[2] = {HG_MINB_UPDATE, HG_MINB_UPDATE + 1};
 constexpr int kInvertMB[2] = {HG_MINB_INVERT, 2};
 
@@ -291,42 +290,45 @@ __device__ __forceinline__ void load_metric_t(const double *__restrict__ G, cons
 // ---------------------------------------------------------------------------
 // WENO5 line reconstruction (slope_lim_linetype_c2e, interpline.c:517-678),
 // one kernel per direction.  The reference sweeps whole lines serially; here
-// a block owns a tile: `lb` consecutive output cells along the direction on
-// `w` lines, and stages what the cells of the tile share in shared memory so
-// that every per-cell quantity is computed once:
-//   S  per output cell: the post/pre-shock reduction factor of
-//      apply_additional_reduction_to_weights (reconstructeno.c:650-700) from
-//      the dP/P jump of compute_df_line_new (interpline.c:2148-2222) over
-//      cells -1, 0, +1, whose state pieces w5_state_kernel formed once per
-//      zone for all three directions
-//   for each primitive v:
-//   Y  the line of v, cells -5..lb+4
-//   A  per cell -3..lb+2: SMONO cusp test and indicator, unoptimised order-3
+// one thread marches one primitive along a segment of `lb` output cells of
+// one line, keeping in registers what neighbouring cells share, so that every
+// per-cell quantity is formed once (but for six cells where a segment starts):
+//   y  the line at cells s-7..s
+//   A  cell s-2: SMONO class (cusp test and indicator) and unoptimised order-3
 //      weights (compute_cf_stencil_weights + mono_adjust_unoptimized_weights)
-//   R  per cell -1..lb: lower-order fraction of compute_weights_ratios
-//   F  per output cell: the final fraction (the cell's own, and the shock
+//   R  cell s-4: lower-order fraction of compute_weights_ratios from the
+//      weights of cells s-6, s-4, s-2
+//   F  output cell s-5: the final fraction (the cell's own, and the shock
 //      factor times its neighbours'), optimised and order-2 weights and the
 //      two face values -> pL, pR
+// The shock factor, the post/pre-shock reduction of
+// apply_additional_reduction_to_weights (reconstructeno.c:650-700) from the
+// dP/P jump of compute_df_line_new (interpline.c:2148-2222), is the same for
+// the eight primitives: w5_state_kernel and w5_shock_kernel form it once per
+// zone and direction.
 // The output cells of a direction are the line cells -1..n (the box), every
-// line across it that the flux loop covers.  Every quantity is formed by the
-// same device functions, in the same operation order, as before tiling, so
-// the FP64 results stay bit-identical to the reference.  T = float is the
-// reconstruction of the mixed-precision path: its line is kept in FP64, it
-// works on differences from each cell's own value and writes FP64 face
-// values (the cell's value plus the FP32 offset), which the FP64 Riemann
-// kernel reads.
+// line across it that the flux loop covers.  Every quantity has the bits of
+// the reference's expressions in FP64.  T = float is the reconstruction of
+// the mixed-precision path: its line is kept in FP64, it works on differences
+// from each cell's own value and writes FP64 face values (the cell's value
+// plus the FP32 offset), which the FP64 Riemann kernel reads.
+//
+// Bound by instruction issue, FP64 first.  The form before this one staged
+// tiles of a line in shared memory, one stage at a time between barriers, and
+// held 1.7 other instructions (addresses, shared memory, selects, the
+// branches of its divisions) to an FP64 one.
 // ---------------------------------------------------------------------------
-constexpr int W5_THREADS = 256;
+constexpr int W5_THREADS = 128;
+constexpr int W5_CHUNK = 8;               // FS: line cells staged per warp and turn
+constexpr int W5_PITCH = W5_CHUNK + 1;    // odd, so that lanes on different rows meet different banks
 
 struct W5Tile {
   Box box;      // output cells
-  int lb;       // output cells per tile along the direction
-  int w;        // lines per tile (a power of two, at most 32)
-  int wshift;   // log2(w)
-  int nseg;     // tiles along the direction
-  int ntile;    // tiles across (ceil(nlines / w))
+  int lb;       // output cells per segment
+  int w;        // lines a caller chose for a tile (kept for hgpu_tuning; rows fill the warps by themselves)
+  int nseg;     // segments along the direction
   int nlines;   // lines of the box
-  int fast_s;   // 1: threads walk along the line (its cells are contiguous in memory), 0: across lines
+  int fast_s;   // 1: a line's cells are contiguous in memory, 0: neighbouring lines are
 };
 
 // The dP/P pieces of compute_df_line_new (interpline.c:2148-2222) of one
@@ -354,11 +356,29 @@ __global__ void __launch_bounds__(128) w5_state_kernel(Dims d, Params P, Box box
   PU[d.nz + z] = gam * pc[UU] * (q.ucon[0] * q.ucov[0]) + (gam - T(1.0)) * pc[UU];
 }
 
-// shared-memory bytes of a tile with lb output cells on w lines: per line
-// Y (lb+10) in FP64, and in the arithmetic type (tsize bytes) A 4 (lb+6),
-// R (lb+2) and the shock factor lb
-__host__ __device__ inline long long w5_smem_bytes(int lb, int w, int tsize) {
-  return (long long)w * (8LL * (lb + 10) + (long long)tsize * (6LL * lb + 26));
+// The shock factor of every output cell along each direction, SS[dir-1][z],
+// from the state pieces of cells -1, 0, +1 (five planes read, up to three
+// written: HBM).  A zone outside a direction's cells -1..n has none there.
+template <typename T>
+__global__ void __launch_bounds__(256) w5_shock_kernel(Dims d, Box box, const double *__restrict__ pb,
+                                                       const T *__restrict__ PU, T *__restrict__ SS) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= box.size()) return;
+  int ijk[3];
+  box_ijk(box, t, ijk[0], ijk[1], ijk[2]);
+  const long long z = zix(d, ijk[0], ijk[1], ijk[2]);
+  const long long o[3] = {(long long)d.nt2 * d.nt3, d.nt3, 1};
+  const int n[3] = {d.n1, d.n2, d.n3};
+  const T r0 = (T)pb[z], par = PU[z], upar = PU[d.nz + z];
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    if (n[q] == 1 || ijk[q] < -1 || ijk[q] > n[q]) continue;
+    const T parl = PU[z - o[q]], parr = PU[z + o[q]];
+    const T uparl = PU[d.nz + z - o[q]], uparr = PU[d.nz + z + o[q]];
+    const T dP = (fabs(r0 * (parr - parl)) + fabs(uparr - uparl)) / (fabs(r0 * par) + fabs(upar) + w5::K<T>::tiny);
+    // (x / 0.25 is the exact multiplication by 4)
+    SS[q * d.nz + z] = w5::wmin((fabs(dP) - T(0.5 * w5::kDpFrac)) * T(1.0 / (0.5 * w5::kDpFrac)), T(1.));
+  }
 }
 
 // zone index of cell 0 of line `line` of box b (along the line the index
@@ -379,128 +399,147 @@ __device__ __forceinline__ long long w5_line(const Dims &d, const Box &b, int li
   return zix(d, i, j, k);
 }
 
+// FS (a line's cells are contiguous): a warp's 32 rows (segments of lines) lie
+// far apart, so it brings W5_CHUNK cells of each at a time through shared
+// memory, a row's cells by neighbouring lanes, and the face values back the
+// same way; otherwise neighbouring lanes are neighbouring lines and read and
+// write the planes directly.
 template <int DIR, bool FS, typename T, int MB = MinBlocks<T>::weno>
-__global__ void __launch_bounds__(W5_THREADS, MB) weno5_kernel(Dims d, Params P, W5Tile tl,
-                                                               const double *__restrict__ pb,
-                                                               const T *__restrict__ PU, double *__restrict__ pL,
+__global__ void __launch_bounds__(W5_THREADS, MB) weno5_kernel(Dims d, W5Tile tl, const double *__restrict__ pb,
+                                                               const T *__restrict__ SS, double *__restrict__ pL,
                                                                double *__restrict__ pR) {
-  extern __shared__ __align__(16) unsigned char w5_smem[];
-  __shared__ long long zb[32];
-  const int W = tl.w;
-  const int seg = blockIdx.x % tl.nseg;
-  const int line0 = (blockIdx.x / tl.nseg) * W;
-  const int nl = min(W, tl.nlines - line0);
+  __shared__ double stage[FS ? W5_THREADS / 32 : 1][FS ? 4 : 1][FS ? 32 * W5_PITCH : 1];
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned rows = (unsigned)tl.nlines * tl.nseg;
+  unsigned t = blockIdx.x * W5_THREADS + threadIdx.x;
+  const bool on = t < rows * NPR;
+  if (!on) t = rows * NPR - 1;
+  const int v = (int)(t / rows);
+  const unsigned r = t - v * rows;
+  const int seg = FS ? (int)(r % tl.nseg) : (int)(r / tl.nlines);
+  const int line = FS ? (int)(r / tl.nseg) : (int)(r % tl.nlines);
   const int nout = (DIR == 1) ? tl.box.ni : ((DIR == 2) ? tl.box.nj : tl.box.nk);
-  const int c0 = ((DIR == 1) ? tl.box.i0 : ((DIR == 2) ? tl.box.j0 : tl.box.k0)) + seg * tl.lb;
-  const int nv = min(tl.lb, nout - seg * tl.lb);  // output cells of this tile
-  const int NS = nv + 10, NA = nv + 6, NL = nv + 2;
+  const int nv = on ? min(tl.lb, nout - seg * tl.lb) : 0;  // output cells of this thread
   const long long o = dir_stride<DIR>(d);
-  // this thread's line w and first cell r; it steps along the line by TL
-  const int TL = W5_THREADS >> tl.wshift;
-  const int w = FS ? (int)(threadIdx.x / TL) : (int)(threadIdx.x & (W - 1));
-  const int r = FS ? (int)(threadIdx.x & (TL - 1)) : (int)(threadIdx.x >> tl.wshift);
-  const bool on = w < nl;
-  if (threadIdx.x < nl) zb[threadIdx.x] = w5_line<DIR>(d, tl.box, line0 + threadIdx.x);
-  double *Y = reinterpret_cast<double *>(w5_smem);                  // cells -5 .. nv+4
-  T *A = reinterpret_cast<T *>(Y + (long long)NS * W);  // 4 planes, cells -3 .. nv+2: code (indicator, -1 at a cusp), w0, w1, w2
-  T *R = A + 4LL * NA * W;          // cells -1 .. nv: lower-order fraction
-  T *SS = R + (long long)NL * W;    // output cells: shock reduction factor
-  // element s of this thread's line in a plane with n cells per line
-  auto at = [&](T *plane, int n, int s) -> T & { return FS ? plane[w * n + s] : plane[s * W + w]; };
-  auto aty = [&](int s) -> double & { return FS ? Y[w * NS + s] : Y[s * W + w]; };
-  // the stencil of the cell at Y index sc: yd[] for differences and linear
-  // combinations, yn[] for magnitudes (the same values in FP64; in FP32 the
-  // offsets from the cell's own value and the values)
-  auto stencil = [&](int sc, T *yd, T *yn, double &yc) {
-    yc = aty(sc);
+  const long long zc = w5_line<DIR>(d, tl.box, line) +
+                       (((DIR == 1) ? tl.box.i0 : ((DIR == 2) ? tl.box.j0 : tl.box.k0)) + seg * tl.lb) * o;
+  const long long zv = zc + (long long)v * d.nz;
+  const double *src = pb + zv;
+  const T *ssrc = SS + (long long)(DIR - 1) * d.nz + zc;
+  const int slast = nv + 4;  // the last cell this thread's output reads
+  double *Ys = stage[FS ? threadIdx.x >> 5 : 0][0];
+  double *Ss = stage[FS ? threadIdx.x >> 5 : 0][FS ? 1 : 0];
+  double *Ls = stage[FS ? threadIdx.x >> 5 : 0][FS ? 2 : 0];
+  double *Rs = stage[FS ? threadIdx.x >> 5 : 0][FS ? 3 : 0];
+
+  double y[8];  // the line at cells s-7 .. s
+  T w0[5], w1[4], w2[4];  // weights of cells s-6 .. s-2 (w0), s-5 .. s-2
+  T Rm = T(0.), Rc = T(0.), Rp = T(0.);  // lower-order fractions of cells s-6, s-5, s-4
+  unsigned codes = 0;     // classes, two bits a cell, s-2 lowest
 #pragma unroll
-    for (int q = 0; q < 5; q++) {
-      const double yq = aty(sc - 2 + q);
-      if constexpr (sizeof(T) == 4) {
-        yd[q] = (T)(yq - yc);
-        yn[q] = (T)yq;
-      } else {
-        yd[q] = yq;
-        yn[q] = yq;
-      }
-    }
-  };
-  __syncthreads();
-  const long long zl = on ? zb[w] : 0;
+  for (int q = 0; q < 8; q++) y[q] = 0.;
+#pragma unroll
+  for (int q = 0; q < 5; q++) w0[q] = T(0.);
+#pragma unroll
+  for (int q = 0; q < 4; q++) w1[q] = w2[q] = T(0.);
+  double ynext = 0.;
+  if (!FS) ynext = __ldg(src + (long long)min(-5, slast) * o);
 
-  // S: the reduction factor of each output cell from the state pieces of
-  // cells -1, 0, +1 (no barrier needed before stage Y: different planes)
-  if (on)
-    for (int s = r; s < nv; s += TL) {
-      const long long z = zl + (long long)(c0 + s) * o;
-      const T parl = __ldg(PU + z - o), par = __ldg(PU + z), parr = __ldg(PU + z + o);
-      const T uparl = __ldg(PU + d.nz + z - o), upar = __ldg(PU + d.nz + z), uparr = __ldg(PU + d.nz + z + o);
-      const T r0 = (T)__ldg(pb + z);
-      const T dP =
-          (fabs(r0 * (parr - parl)) + fabs(uparr - uparl)) / (fabs(r0 * par) + fabs(upar) + w5::K<T>::tiny);
-      // (x / 0.25 is the exact multiplication by 4)
-      at(SS, nv, s) = w5::wmin((fabs(dP) - T(0.5 * w5::kDpFrac)) * T(1.0 / (0.5 * w5::kDpFrac)), T(1.));
+  for (int s = -5; s < tl.lb + 5; s++) {
+    const int slot = (s + 5) % W5_CHUNK;
+    if (FS && slot == 0) {
+      // cells s .. s+CHUNK-1 of the line and s-5 .. of the shock factor
+      __syncwarp();
+#pragma unroll
+      for (int it = 0; it < W5_CHUNK; it++) {
+        const int row = it * (32 / W5_CHUNK) + (int)(lane / W5_CHUNK), c = (int)(lane % W5_CHUNK);
+        const double *rs = (const double *)__shfl_sync(0xffffffffu, (unsigned long long)src, row);
+        const T *rss = (const T *)__shfl_sync(0xffffffffu, (unsigned long long)ssrc, row);
+        const int last = __shfl_sync(0xffffffffu, slast, row);
+        Ys[row * W5_PITCH + c] = __ldg(rs + min(s + c, last));
+        if (s + c >= 5) Ss[row * W5_PITCH + c] = (double)__ldg(rss + min(s + c - 5, max(last - 5, 0)));
+      }
+      __syncwarp();
     }
-
-  T *CODE = A, *W0 = A + (long long)NA * W, *W1 = A + 2LL * NA * W, *W2 = A + 3LL * NA * W;
-  for (int v = 0; v < NPR; v++) {
-    const double *pv = pb + (long long)v * d.nz + zl;
-    // Y: the line of primitive v
-    if (on)
-      for (int s = r; s < NS; s += TL) aty(s) = __ldg(pv + (long long)(c0 - 5 + s) * o);
-    __syncthreads();
-    // A: cusp test, SMONO indicator, unoptimised weights of cells -3..nv+2
-    if (on)
-      for (int s = r; s < NA; s += TL) {
-        T ya[5], yb[5];
-        double yc;
-        stencil(s + 2, ya, yb, yc);
-        const T *y = ya + 2, *yn = yb + 2;
-        const bool c = w5::cusp(y, yn);
-        const T m0 = c ? T(0.0) : w5::mono(y, yn);
-        T wt[3];
-        w5::unopt3(m0, y, yn, wt);
-        at(CODE, NA, s) = c ? T(-1.0) : m0;
-        at(W0, NA, s) = wt[0];
-        at(W1, NA, s) = wt[1];
-        at(W2, NA, s) = wt[2];
-      }
-    __syncthreads();
-    // R: lower-order fraction of cells -1..nv from the weights of cells -3..nv+2
-    if (on)
-      for (int s = r; s < NL; s += TL) {
-        const int a = s + 2;  // cell s-1 in the A planes
-        const T wc[3] = {at(W0, NA, a), T(0.0), at(W2, NA, a)};
-        at(R, NL, s) =
-            w5::ratio_lof(wc, at(W0, NA, a - 2), at(W2, NA, a + 2), at(CODE, NA, a) == T(-1.0) ? T(1.0) : T(0.0));
-      }
-    __syncthreads();
-    // F: face values of the output cells
-    if (on)
-      for (int s = r; s < nv; s += TL) {
-        const T ss = at(SS, nv, s);
-        T lof = at(R, NL, s + 1);
-        lof = w5::wmax(lof, ss * at(R, NL, s + 2));
-        lof = w5::wmax(lof, ss * at(R, NL, s));
-        const int a = s + 3;
-        const T c0v = at(CODE, NA, a);
-        const T wc[3] = {at(W0, NA, a), at(W1, NA, a), at(W2, NA, a)};
-        T ya[5], yb[5];
-        double yc;
-        stencil(s + 5, ya, yb, yc);
-        const bool cu = (c0v == T(-1.0));
-        T yl, yr;
-        w5::faces(ya + 2, yb + 2, cu ? T(0.0) : c0v, cu, wc, lof, &yl, &yr);
-        const long long z = zl + (long long)(c0 + s) * o + (long long)v * d.nz;
+#pragma unroll
+    for (int q = 0; q < 7; q++) y[q] = y[q + 1];
+    T ss = T(0.);
+    if (FS) {
+      y[7] = Ys[lane * W5_PITCH + slot];
+      if (s >= 5) ss = (T)Ss[lane * W5_PITCH + slot];
+    } else {
+      y[7] = ynext;
+      ynext = __ldg(src + (long long)min(s + 1, slast) * o);
+      if (s >= 5) ss = __ldg(ssrc + (long long)min(s - 5, max(nv - 1, 0)) * o);
+    }
+    // the stencil of the cell at y[q]: values for FP64; in FP32 offsets from
+    // the cell's own value, and the values for magnitudes
+    auto stencil = [&](int q, T *yd, T *yn) {
+#pragma unroll
+      for (int e = 0; e < 5; e++) {
         if constexpr (sizeof(T) == 4) {
-          pL[z] = yc + (double)yl;
-          pR[z] = yc + (double)yr;
+          yd[e] = (T)(y[q - 2 + e] - y[q]);
+          yn[e] = (T)y[q - 2 + e];
         } else {
-          pL[z] = yl;
-          pR[z] = yr;
+          yd[e] = yn[e] = y[q - 2 + e];
         }
       }
-    __syncthreads();
+    };
+    if (s >= -1) {
+      T ya[5], yb[5], w[3];
+      stencil(5, ya, yb);
+      const int code = w5::code_of(ya + 2, yb + 2);
+      w5::weights3(code, ya + 2, yb + 2, w);
+      codes = (codes << 2) | (unsigned)code;
+#pragma unroll
+      for (int q = 0; q < 4; q++) w0[q] = w0[q + 1];
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        w1[q] = w1[q + 1];
+        w2[q] = w2[q + 1];
+      }
+      w0[4] = w[0];
+      w1[3] = w[1];
+      w2[3] = w[2];
+    }
+    if (s >= 3) {
+      Rm = Rc;
+      Rc = Rp;
+      Rp = w5::lower_fraction((int)(codes >> 4) & 3, w0[2], w2[1], w0[0], w2[3]);
+    }
+    if (s >= 5) {
+      T lof = Rc;
+      lof = w5::wmax(lof, ss * Rp);
+      lof = w5::wmax(lof, ss * Rm);
+      T ya[5], yb[5], yl, yr;
+      stencil(2, ya, yb);
+      const T w[3] = {w0[1], w1[0], w2[0]};
+      w5::face_values((int)(codes >> 6) & 3, ya + 2, yb + 2, w, lof, &yl, &yr);
+      const double fl = sizeof(T) == 4 ? y[2] + (double)yl : (double)yl;
+      const double fr = sizeof(T) == 4 ? y[2] + (double)yr : (double)yr;
+      if (FS) {
+        Ls[lane * W5_PITCH + slot] = fl;
+        Rs[lane * W5_PITCH + slot] = fr;
+      } else if (s - 5 < nv) {
+        pL[zv + (long long)(s - 5) * o] = fl;
+        pR[zv + (long long)(s - 5) * o] = fr;
+      }
+    }
+    if (FS && (slot == W5_CHUNK - 1 || s == tl.lb + 4)) {
+      // the face values of this turn's output cells, s-5-slot ..
+      __syncwarp();
+#pragma unroll
+      for (int it = 0; it < W5_CHUNK; it++) {
+        const int row = it * (32 / W5_CHUNK) + (int)(lane / W5_CHUNK), c = (int)(lane % W5_CHUNK);
+        const long long rz = __shfl_sync(0xffffffffu, zv, row);
+        const int rnv = __shfl_sync(0xffffffffu, nv, row);
+        const int cell = s - 5 - slot + c;
+        if (c <= slot && cell >= 0 && cell < rnv) {
+          pL[rz + cell] = Ls[row * W5_PITCH + c];
+          pR[rz + cell] = Rs[row * W5_PITCH + c];
+        }
+      }
+    }
   }
 }
 

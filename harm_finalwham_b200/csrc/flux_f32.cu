@@ -13,9 +13,9 @@
 namespace hg {
 
 #define HG_F32_INSTANCES(DIR)                                                                                      \
-  template __global__ void weno5_kernel<DIR, true, float>(Dims, Params, W5Tile, const double *, const float *,    \
+  template __global__ void weno5_kernel<DIR, true, float>(Dims, W5Tile, const double *, const float *,            \
                                                           double *, double *);                                      \
-  template __global__ void weno5_kernel<DIR, false, float>(Dims, Params, W5Tile, const double *, const float *,   \
+  template __global__ void weno5_kernel<DIR, false, float>(Dims, W5Tile, const double *, const float *,           \
                                                            double *, double *);                                     \
   template __global__ void flux_kernel<DIR, 0, float>(Dims, Params, Box, const double *, const float *,           \
                                                       const float *, const double *, double *, Scalars *);          \
@@ -30,5 +30,6 @@ HG_F32_INSTANCES(1)
 HG_F32_INSTANCES(2)
 HG_F32_INSTANCES(3)
 template __global__ void w5_state_kernel<float>(Dims, Params, Box, const double *, const double *, float *);
+template __global__ void w5_shock_kernel<float>(Dims, Box, const double *, const float *, float *);
 
 }  // namespace hg

@@ -12,8 +12,8 @@
 //
 // Work per RK substep (the reference's advance(), step_ch.c:94-186):
 //   weno5_kernel<dir> WENO5 line reconstruction (interpline.c:517-678), one
-//                     kernel per direction over tiles staged in shared
-//                     memory (lim = WENO5 only; weno5.cuh, common.cuh)
+//                     kernel per direction, a thread per segment of a line
+//                     and primitive (lim = WENO5 only; weno5.cuh, common.cuh)
 //   flux_kernel<dir>  fluxcalc_standard (flux.c:469-680) fused with the
 //                     MC/PARA reconstruction (or reading the WENO5 face
 //                     values), both Riemann states, vchar, HLL/LaxF, the gdet
@@ -51,10 +51,10 @@ using namespace hg;
 // flux_f32.cu (FMA and fast FP32 division there; this unit keeps -fmad=false)
 namespace hg {
 #define HG_F32_EXTERN(DIR)                                                                                         \
-  extern template __global__ void weno5_kernel<DIR, true, float>(Dims, Params, W5Tile, const double *,            \
-                                                                 const float *, double *, double *);              \
-  extern template __global__ void weno5_kernel<DIR, false, float>(Dims, Params, W5Tile, const double *,           \
-                                                                  const float *, double *, double *);             \
+  extern template __global__ void weno5_kernel<DIR, true, float>(Dims, W5Tile, const double *, const float *,       \
+                                                                double *, double *);                             \
+  extern template __global__ void weno5_kernel<DIR, false, float>(Dims, W5Tile, const double *, const float *,      \
+                                                                double *, double *);                             \
   extern template __global__ void flux_kernel<DIR, 0, float>(Dims, Params, Box, const double *, const float *,    \
                                                              const float *, const double *, double *, Scalars *);   \
   extern template __global__ void flux_kernel<DIR, 2, float>(Dims, Params, Box, const double *, const float *,    \
@@ -67,6 +67,7 @@ HG_F32_EXTERN(1)
 HG_F32_EXTERN(2)
 HG_F32_EXTERN(3)
 extern template __global__ void w5_state_kernel<float>(Dims, Params, Box, const double *, const double *, float *);
+extern template __global__ void w5_shock_kernel<float>(Dims, Box, const double *, const float *, float *);
 }  // namespace hg
 
 namespace {
@@ -1392,85 +1393,55 @@ __global__ void utoprim_batch_kernel(const double *__restrict__ U, const double 
 
 inline unsigned grid_for(long long n, int block) { return (unsigned)((n + block - 1) / block); }
 
-// Dynamic shared memory the WENO5 kernel may use per block (its tilings are
-// sized to fit, for FP64 elements)
-constexpr size_t W5_SMEM_MAX = 72 * 1024;
-
-// Cost of a WENO5 tiling in block rounds (a stage's items over the 256
-// threads, whole rounds), weighted by each stage's work per item, plus the
-// barriers: S (shock factor) once, then per primitive Y (line loads), A
-// (SMONO + weights), R (ratios), F (face values) and four barriers.
-double w5_cost(int nout, long long nlines, int lb, int w, bool fs) {
-  const int nseg = (nout + lb - 1) / lb;
-  const long long ntile = (nlines + w - 1) / w;
-  const int tl = W5_THREADS / w;
-  auto rounds = [&](int n) {
-    return fs ? (double)((n + tl - 1) / tl) : (double)(((long long)n * w + W5_THREADS - 1) / W5_THREADS);
-  };
-  double per = 0.0;
-  for (int sgi = 0; sgi < 2; sgi++) {
-    const int nv = sgi == 0 ? lb : nout - (nseg - 1) * lb;  // full tiles, then the last one
-    const double count = sgi == 0 ? (double)(nseg - 1) : 1.0;
-    per += count * (rounds(nv) +
-                    8.0 * (0.3 * rounds(nv + 10) + 2.0 * rounds(nv + 6) + 0.3 * rounds(nv + 2) + 1.5 * rounds(nv) + 2.0));
-  }
-  return per * (double)ntile;
+// Time of a WENO5 pass with segments of lb cells, in steps of one thread
+// along its line.  A thread takes lb + 10 steps, of which lb do the whole
+// work and the first ten about as much as five.  While an SM holds one block
+// its four schedulers wait on the results of a warp each; further blocks fill
+// them and cost about 0.6 of a block's time apiece (up to four resident, the
+// rest in turn).
+double w5_cost(int nout, long long nlines, int lb) {
+  const long long nseg = (nout + lb - 1) / lb;
+  const long long blocks = (nlines * nseg * NPR + W5_THREADS - 1) / W5_THREADS;
+  const double per_sm = (double)((blocks + 147) / 148);
+  return (lb + 5.0) * (per_sm <= 1.0 ? 1.0 : 0.4 + 0.6 * per_sm);
 }
 
-// WENO5 tilings of the output box b along direction dir, best first (at
-// most `max` of them, one per line count).  Lines whose cells are contiguous
-// in memory (x3, or any direction of a domain flat across it) are walked
-// along by consecutive threads, a warp or more per line; the others across,
-// consecutive threads on neighbouring lines (x3 fastest), at least 8 of them
-// for 64-byte rows.  Every tiling fits the shared-memory budget.
+// WENO5 segmentings of the output box b along direction dir, best first (at
+// most `max`, at most 4): every segment count whose last segment is not
+// mostly empty, by the cost above.  Lines whose cells are contiguous in
+// memory (x3, or any direction of a domain flat across it) are staged.
 int w5_candidates(const Dims &d, const Box &b, int dir, W5Tile *out, int max) {
   const int nout = dir == 1 ? b.ni : (dir == 2 ? b.nj : b.nk);
   const long long nlines = dir == 1 ? (long long)b.nj * b.nk : (dir == 2 ? (long long)b.ni * b.nk : (long long)b.ni * b.nj);
   const long long stride = dir == 1 ? (long long)d.nt2 * d.nt3 : (dir == 2 ? (long long)d.nt3 : 1LL);
-  const bool fs = stride == 1;
-  double cost[6];
-  W5Tile cand[6];
-  int n = 0;
-  const int ws[] = {1, 2, 4, 8, 16, 32};
-  for (int w : ws) {
-    if (w > nlines && w > 1) break;
-    if (!fs && w < 8 && nlines >= 8) continue;
-    if (fs && w > 8 && nout >= 32) continue;
-    double best = -1.0;
-    int blb = 0;
-    for (int nseg = 1; nseg <= nout; nseg++) {
-      const int lb = (nout + nseg - 1) / nseg;
-      if (w5_smem_bytes(lb, w, 8) > (long long)W5_SMEM_MAX) continue;
-      if (lb < 8 && nseg > 1) break;
-      const double c = w5_cost(nout, nlines, lb, w, fs);
-      if (best < 0.0 || c < best) {
-        best = c;
-        blb = lb;
-      }
-      if (nseg > 64 && lb < 256) break;
+  double cost[5];
+  int lbs[5], n = 0;
+  int last = 0;
+  for (int nseg = 1; nseg <= nout; nseg++) {
+    const int lb = (nout + nseg - 1) / nseg;
+    if (lb == last) continue;
+    last = lb;
+    if (lb < 4 && nseg > 1) break;
+    // the best four so far, in order
+    const double c = w5_cost(nout, nlines, lb);
+    int at = n < 4 ? n++ : 4;
+    cost[at] = c;
+    lbs[at] = lb;
+    for (; at > 0 && cost[at] < cost[at - 1]; at--) {
+      std::swap(cost[at], cost[at - 1]);
+      std::swap(lbs[at], lbs[at - 1]);
     }
-    if (blb == 0) continue;
-    W5Tile t;
+  }
+  if (n > max) n = max;
+  for (int i = 0; i < n; i++) {
+    W5Tile &t = out[i];
     t.box = b;
     t.nlines = (int)nlines;
-    t.fast_s = fs;
-    t.lb = blb;
-    t.w = w;
-    t.nseg = (nout + blb - 1) / blb;
-    t.ntile = (int)((nlines + w - 1) / w);
-    t.wshift = 0;
-    while ((1 << t.wshift) < w) t.wshift++;
-    cost[n] = best;
-    cand[n++] = t;
+    t.fast_s = stride == 1;
+    t.lb = lbs[i];
+    t.w = 32;
+    t.nseg = (nout + t.lb - 1) / t.lb;
   }
-  // best first
-  for (int i = 1; i < n; i++)
-    for (int j = i; j > 0 && cost[j] < cost[j - 1]; j--) {
-      std::swap(cost[j], cost[j - 1]);
-      std::swap(cand[j], cand[j - 1]);
-    }
-  if (n > max) n = max;
-  for (int i = 0; i < n; i++) out[i] = cand[i];
   return n;
 }
 
@@ -1480,29 +1451,10 @@ W5Tile w5_tiling(const Dims &d, const Box &b, int dir) {
   return t[0];
 }
 
-// the WENO5 kernels may use up to W5_SMEM_MAX of dynamic shared memory
-void w5_allow_smem_all() {
-  static std::once_flag once;
-  std::call_once(once, [] {
-    const int m = (int)W5_SMEM_MAX;
-    const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaFuncSetAttribute(weno5_kernel<1, false, double, kWenoMB[0]>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<1, true, double, kWenoMB[0]>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<2, false, double, kWenoMB[0]>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<2, true, double, kWenoMB[0]>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<3, true, double, kWenoMB[0]>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<1, false, double, kWenoMB[1]>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<1, true, double, kWenoMB[1]>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<2, false, double, kWenoMB[1]>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<2, true, double, kWenoMB[1]>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<3, true, double, kWenoMB[1]>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<1, false, float>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<1, true, float>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<2, false, float>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<2, true, float>, a, m);
-    cudaFuncSetAttribute(weno5_kernel<3, true, float>, a, m);
-    cudaGetLastError();
-  });
+// What hgpu_set_tuning accepts as a tile of lb cells on w lines: the shared
+// memory that the tiled form of the kernel took for it, up to 72 KB.
+bool w5_tile_accepted(int lb, int w) {
+  return (long long)w * (8LL * (lb + 10) + 8 * (6LL * lb + 26)) <= 72 * 1024;
 }
 
 }  // namespace
@@ -1556,12 +1508,14 @@ struct hgpu_ctx {
   double *staging = nullptr;  // AoS staging for uploads/downloads
   double *pL = nullptr, *pR = nullptr;  // WENO5 face values
   double *w5pu = nullptr;               // WENO5: per-zone dP/P state pieces (2 planes)
+  double *w5ss = nullptr;               // WENO5: shock factor per direction (3 planes)
   unsigned char *bsqf = nullptr;        // FLAGBSQORHO | FLAGBSQOU << 2 per zone
   unsigned int *ffc = nullptr;          // failure/floor counters, NFFC planes
   double *bondi_tab = nullptr;          // Bondi-integral boundaries' coordinate data
   double *progress = nullptr;                          // 4 doubles for hg_progress_async
   W5Tile w5[4];  // WENO5 tiling per direction
   Box w5_state_box;  // zones whose dP/P state pieces some direction reads
+  Box w5_shock_box;  // zones whose shock factors some direction reads
   int *istaging = nullptr;
   // batch of 1D instances (hgpu_create_batch)
   int *cell_inst = nullptr;
@@ -1681,7 +1635,7 @@ void hgpu_destroy(hgpu_ctx *x) {
   for (cudaEvent_t e : x->freelist) cudaEventDestroy(e);
   void *ptrs[] = {x->p, x->pk, x->uf, x->ucum, x->F[1], x->F[2], x->F[3], x->E, x->G, x->pflag, x->gammacheck,
                   x->cand, x->fixlist, x->cand_orig, x->cand_dec, x->cand_bits, x->cand_deplist, x->candmap, x->fixvals, x->sc, x->staging, x->istaging,
-                  x->pL, x->pR, x->w5pu, x->bsqf, x->ffc, x->bondi_tab, x->cell_inst, x->inst, x->progress, x->pk1, x->ui};
+                  x->pL, x->pR, x->w5pu, x->w5ss, x->bsqf, x->ffc, x->bondi_tab, x->cell_inst, x->inst, x->progress, x->pk1, x->ui};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   cudaStreamDestroy(x->stream);
@@ -1801,8 +1755,8 @@ int hgpu_create(const hgpu_config *cfg, hgpu_ctx **out) {
     const int fvg = cfg->doenoflux == HGPU_ENOFINITEVOLUME;
     const int e1 = fvg ? d.g1 : 2 * d.s1, e2 = fvg ? d.g2 : 2 * d.s2, e3 = fvg ? d.g3 : 2 * d.s3;
     x->w5_state_box = Box{-e1, -e2, -e3, d.n1 + 2 * e1, d.n2 + 2 * e2, d.n3 + 2 * e3};
+    x->w5_shock_box = fvg ? x->w5_state_box : x->dq_box;
   }
-  if (cfg->lim == HGPU_LIM_WENO5) w5_allow_smem_all();
   long long nz = d.nz;
   x->cap = (int)((long long)d.n1 * d.n2 * d.n3 < (1LL << 22) ? (long long)d.n1 * d.n2 * d.n3 : (1LL << 22));
   if (cudaStreamCreateWithFlags(&x->stream, cudaStreamNonBlocking) != cudaSuccess) {
@@ -1836,7 +1790,8 @@ int hgpu_create(const hgpu_config *cfg, hgpu_ctx **out) {
          cudaMemset(x->ucum, 0, pb) == cudaSuccess;
   if (ok && cfg->lim == HGPU_LIM_WENO5)
     ok = cudaMalloc(&x->pL, pb) == cudaSuccess && cudaMalloc(&x->pR, pb) == cudaSuccess &&
-         cudaMalloc(&x->w5pu, sizeof(double) * 2 * nz) == cudaSuccess;
+         cudaMalloc(&x->w5pu, sizeof(double) * 2 * nz) == cudaSuccess &&
+         cudaMalloc(&x->w5ss, sizeof(double) * 3 * nz) == cudaSuccess;
   if (!ok) {
     hgpu_destroy(x);
     set_err("device allocation failed");
@@ -2053,21 +2008,28 @@ extern "C++" {
 template <int DIR, typename TW, int BMB>
 static void launch_w5(hgpu_ctx *x, const double *pb) {
   const Dims &d = x->d;
-  const Params &P = x->P;
   const W5Tile &tl = x->w5[DIR];
-  const size_t smem = (size_t)w5_smem_bytes(tl.lb, tl.w, (int)sizeof(TW));
-  const TW *PU = (const TW *)x->w5pu;
+  const TW *SS = (const TW *)x->w5ss;
   double *pL = x->pL, *pR = x->pR;
   ProfScope ps__(x, K_WENO5);
-  const unsigned grid = (unsigned)tl.nseg * tl.ntile;
+  const unsigned grid = grid_for((long long)tl.nlines * tl.nseg * NPR, W5_THREADS);
   if constexpr (DIR == 3) {
-    weno5_kernel<3, true, TW, BMB><<<grid, W5_THREADS, smem, x->stream>>>(d, P, tl, pb, PU, pL, pR);
+    weno5_kernel<3, true, TW, BMB><<<grid, W5_THREADS, 0, x->stream>>>(d, tl, pb, SS, pL, pR);
   } else {
     if (tl.fast_s)
-      weno5_kernel<DIR, true, TW, BMB><<<grid, W5_THREADS, smem, x->stream>>>(d, P, tl, pb, PU, pL, pR);
+      weno5_kernel<DIR, true, TW, BMB><<<grid, W5_THREADS, 0, x->stream>>>(d, tl, pb, SS, pL, pR);
     else
-      weno5_kernel<DIR, false, TW, BMB><<<grid, W5_THREADS, smem, x->stream>>>(d, P, tl, pb, PU, pL, pR);
+      weno5_kernel<DIR, false, TW, BMB><<<grid, W5_THREADS, 0, x->stream>>>(d, tl, pb, SS, pL, pR);
   }
+}
+
+// the WENO5 state pieces and shock factors, for every direction
+template <typename TW>
+static void launch_w5_state(hgpu_ctx *x, const double *pb) {
+  LAUNCH(x, K_W5STATE, w5_state_kernel<TW>, grid_for(x->w5_state_box.size(), 128), 128, x->d, x->P, x->w5_state_box,
+         pb, x->G, (TW *)x->w5pu);
+  LAUNCH(x, K_W5STATE, w5_shock_kernel<TW>, grid_for(x->w5_shock_box.size(), 256), 256, x->d, x->w5_shock_box, pb,
+         (const TW *)x->w5pu, (TW *)x->w5ss);
 }
 
 template <int DIR, typename TW, typename TF, int FMB, int BMB, int MIX = 0>
@@ -2092,9 +2054,7 @@ static void launch_dir(hgpu_ctx *x, const double *pb) {
 template <typename TW, typename TF, int FMB, int BMB, int MIX = 0>
 static void launch_fluxes_t(hgpu_ctx *x, const double *pb) {
   const Dims &d = x->d;
-  if (x->P.lim == HGPU_LIM_WENO5)
-    LAUNCH(x, K_W5STATE, w5_state_kernel<TW>, grid_for(x->w5_state_box.size(), 128), 128, d, x->P, x->w5_state_box,
-           pb, x->G, (TW *)x->w5pu);
+  if (x->P.lim == HGPU_LIM_WENO5) launch_w5_state<TW>(x, pb);
   if (d.n1 > 1) launch_dir<1, TW, TF, FMB, BMB, MIX>(x, pb);
   if (d.n2 > 1) launch_dir<2, TW, TF, FMB, BMB, MIX>(x, pb);
   if (d.n3 > 1) launch_dir<3, TW, TF, FMB, BMB, MIX>(x, pb);
@@ -2103,16 +2063,11 @@ static void launch_fluxes_t(hgpu_ctx *x, const double *pb) {
 // context's precision and WENO5 variant (for timing tilings)
 template <int DIR>
 static void launch_w5_any(hgpu_ctx *x, const double *pb, bool state) {
-  const Dims &d = x->d;
   if (x->cfg.precision == HGPU_PREC_MIXED) {
-    if (state)
-      w5_state_kernel<float><<<grid_for(x->w5_state_box.size(), 128), 128, 0, x->stream>>>(d, x->P, x->w5_state_box,
-                                                                                          pb, x->G, (float *)x->w5pu);
+    if (state) launch_w5_state<float>(x, pb);
     launch_w5<DIR, float, MinBlocks<float>::weno>(x, pb);
   } else {
-    if (state)
-      w5_state_kernel<double><<<grid_for(x->w5_state_box.size(), 128), 128, 0, x->stream>>>(d, x->P, x->w5_state_box,
-                                                                                           pb, x->G, x->w5pu);
+    if (state) launch_w5_state<double>(x, pb);
     if (x->tune.weno == 0) launch_w5<DIR, double, kWenoMB[0]>(x, pb);
     else launch_w5<DIR, double, kWenoMB[1]>(x, pb);
   }
@@ -2935,16 +2890,13 @@ int hgpu_set_tuning(hgpu_ctx *x, const hgpu_tuning *t) {
     if (lb <= 0 || x->P.lim != HGPU_LIM_WENO5) continue;
     const Box &bx = x->w5[q].box;
     const int nout = q == 1 ? bx.ni : (q == 2 ? bx.nj : bx.nk);
-    if (w < 1 || w > 32 || (w & (w - 1)) || lb > nout || w5_smem_bytes(lb, w, 8) > (long long)W5_SMEM_MAX) {
+    if (w < 1 || w > 32 || (w & (w - 1)) || lb > nout || !w5_tile_accepted(lb, w)) {
       set_err("hgpu_set_tuning: invalid WENO5 tiling");
       return HGPU_E_INVALID;
     }
     w5[q].lb = lb;
     w5[q].w = w;
     w5[q].nseg = (nout + lb - 1) / lb;
-    w5[q].ntile = (w5[q].nlines + w - 1) / w;
-    w5[q].wshift = 0;
-    while ((1 << w5[q].wshift) < w) w5[q].wshift++;
   }
   CUDA_TRY(cudaStreamSynchronize(x->stream));
   for (int q = 1; q <= 3; q++) x->w5[q] = w5[q];
@@ -3211,7 +3163,7 @@ extern "C" size_t hgpu_context_bytes(const hgpu_config *c) {
              + sizeof(double) * nz            // gamma check
              + cap * (2 * sizeof(long long) + 4 * sizeof(int) + 5 * sizeof(double))
              + plane;                         // staging for uploads and downloads
-  if (c->lim == HGPU_LIM_WENO5) b += 2 * plane + sizeof(double) * 2 * nz;  // pL, pR, dP/P state pieces
+  if (c->lim == HGPU_LIM_WENO5) b += 2 * plane + sizeof(double) * 5 * nz;  // pL, pR, dP/P state pieces, shock factors
   if (c->timeorder >= 3) b += plane;                     // pk1
   if (c->doenoflux == HGPU_ENOFINITEVOLUME) b += plane;  // ui
   if (c->bc[0] == HGPU_BC_BONDIMDOTOUTFLOW || c->bc[1] == HGPU_BC_BONDIINTOUTFLOW)

@@ -10,7 +10,7 @@
 // c depends only on the line from c-5 to c+5 (for the reference's MAXBND=11
 // lines no stencil reaches a line end, so its boundary-truncation branches
 // are dead).  These are the per-cell pieces; weno5_kernel (common.cuh)
-// stages them over tiles of a line in shared memory:
+// marches them along the lines:
 //   per cell, per primitive: SMONO cusp test and indicator, and the
 //          unoptimised order-3 weights (compute_cf_stencil_weights +
 //          mono_adjust_unoptimized_weights)
@@ -21,6 +21,7 @@
 // Every expression keeps the reference's operation order; the library is
 // compiled with -fmad=false, so results are bit-identical to the reference.
 #pragma once
+#include "exact_div.cuh"
 
 namespace hg {
 namespace w5 {
@@ -397,6 +398,228 @@ __device__ __forceinline__ void faces(const T *u, const T *un, T m0, bool is_cus
     if (right) *yr = prev;
     else *yl = prev;
   }
+}
+
+// ---------------------------------------------------------------------------
+// The pieces as weno5_kernel calls them: a cell's SMONO class, its
+// unoptimised weights, the lower-order fraction and the face values.  T =
+// float goes through the routines above.  FP64 gives their bits with less
+// work: most SMONO indicators are exactly 0 or 1 and are told from signs and
+// exponents, quotients share reciprocals (exact_div.cuh), and a quotient that
+// is only compared or clamped is formed where a product cannot decide it.
+// Whatever falls outside (indicators in between, magnitudes near the ends of
+// the range, significands that exact_div excludes) takes the routines above.
+// ---------------------------------------------------------------------------
+
+enum { kZero = 0, kOne = 1, kBlend = 2, kCusp = 3 };  // monoindicator 0, 1, in between; cusp (indicator 0)
+
+template <typename T>
+__device__ __forceinline__ int code_of(const T *y, const T *yn) {
+  if (cusp(y, yn)) return kCusp;
+  const T m0 = mono(y, yn);
+  return m0 == T(0.0) ? kZero : (m0 == T(1.0) ? kOne : kBlend);
+}
+
+// the sign of s put on x as a factor +-1 would
+__device__ __forceinline__ double times_sign(double x, uint32_t hs) {
+  return __hiloint2double(__double2hiint(x) ^ (int)(hs & 0x80000000u), __double2loint(x));
+}
+
+// check_for_cusp_new with its differences against norm as comparisons (a -
+// norm > 0 and a > norm agree in IEEE arithmetic), then the indicator:
+//   0 where a pair of estimates differs in sign or the outer difference of
+//     either side is 0 (minmod gives 0);
+//   1 where every estimate is above the cut (they are compared by exponent
+//     word; x/12 > x/16, and the cusp test's norm is not below mono's cut but
+//     for rounding, which the word after the next covers);
+//   otherwise mono decides.
+template <>
+__device__ __forceinline__ int code_of<double>(const double *y, const double *) {
+  const double df_m1 = y[-1] - y[-2], df0 = y[0] - y[-1], df1 = y[1] - y[0], df2 = y[2] - y[1];
+  const double ddf_m1 = df0 - df_m1, ddf0 = df1 - df0, ddf1 = df2 - df1;
+  const double norm = (fabs(y[-2]) + fabs(y[-1]) + fabs(y[0]) + fabs(y[1]) + fabs(y[2]) + K<double>::small) * K<double>::smono;
+  const uint32_t h0 = hi_word(df0), h1 = hi_word(df1);
+  if (fabs(df0) > norm && times_sign(ddf_m1, h0) > norm && -times_sign(ddf0, h0) > norm &&
+      ((-times_sign(df2, h0) > norm && fabs(df2 + df0) > 0.25 * (fabs(df2) + fabs(df0))) ||
+       (-times_sign(df1, h0) > norm && fabs(df1 + df0) > 0.25 * (fabs(df1) + fabs(df0)))))
+    return kCusp;
+  if (fabs(df1) > norm && -times_sign(ddf1, h1) > norm && times_sign(ddf0, h1) > norm &&
+      ((-times_sign(df_m1, h1) > norm && fabs(df_m1 + df1) > 0.25 * (fabs(df_m1) + fabs(df1))) ||
+       (-times_sign(df0, h1) > norm && fabs(df0 + df1) > 0.25 * (fabs(df0) + fabs(df1)))))
+    return kCusp;
+  // the numerators of mono's estimates
+  const uint32_t l1 = hi_word(((-3 * y[-2] + y[2]) + (-10 * y[-1] - 6 * y[1])) + 18 * y[0]);
+  const uint32_t l2 = hi_word(((11 * y[-2] - y[2]) + (-20 * y[-1] + 4 * y[1])) + 6 * y[0]);
+  const uint32_t l3 = hi_word(((-3 * y[-2] - y[2]) + (10 * y[-1] + 6 * y[1])) - 12 * y[0]);
+  const uint32_t r1 = hi_word(((-y[-2] + 3 * y[2]) + (6 * y[-1] + 10 * y[1])) - 18 * y[0]);
+  const uint32_t r2 = hi_word(((-y[-2] + 11 * y[2]) + (4 * y[-1] - 20 * y[1])) + 6 * y[0]);
+  const uint32_t r3 = hi_word(((y[-2] + 3 * y[2]) - (6 * y[-1] + 10 * y[1])) + 12 * y[0]);
+  const uint32_t dl = hi_word(df_m1), dr = hi_word(df2);
+  const uint32_t diff = (l1 ^ dl) | (l1 ^ r1) | (l1 ^ dr) | (l2 ^ r2) | (l3 ^ r3);
+  if ((int)diff < 0 || df_m1 == 0.0 || df2 == 0.0) return kZero;
+  const uint32_t m = 0x7fffffffu;
+  const int e12 = (int)min(min(l1 & m, r1 & m), min(l2 & m, r2 & m)) - (4 << 20);
+  const int e2 = (int)min(l3 & m, r3 & m) - (1 << 20);
+  const int e1 = (int)min(dl & m, dr & m);
+  if (min(min(e12, e2), e1) > (int)hi_word(norm) + 2) return kOne;
+  const double m0 = mono(y, y);
+  return m0 == 0.0 ? kZero : (m0 == 1.0 ? kOne : kBlend);
+}
+
+template <typename T>
+__device__ __forceinline__ void weights3(int code, const T *u, const T *un, T w[3]) {
+  const T m0 = code == kBlend ? mono(u, un) : (code == kOne ? T(1.0) : T(0.0));
+  unopt3(m0, u, un, w);
+}
+
+// whether a divisor of the smoothness terms, or the square of a normalised
+// one, has a reciprocal by rcp_rn: each numerator is at least 1e-28 of it, so
+// [2^-700, 2^700] leaves the remainders exact
+__device__ __forceinline__ bool w_rcp_ok(double s) {
+  return (hi_word(s) << 1) - exp_word2(-700) < exp_word2(700) - exp_word2(-700) && lo_word(s) != 0xffffffffu;
+}
+
+template <>
+__device__ __forceinline__ void weights3<double>(int code, const double *u, const double *un, double w[3]) {
+  if (code == kOne) {
+    w[0] = w[1] = w[2] = 1.0 / 3;
+    return;
+  }
+  bool ok = code != kBlend;
+  {
+    const double u3 = 3 * u[0], u4p = 4 * u[1], u4m = 4 * u[-1], t0 = 2 * u[0];
+    const double fd0 = -(u3 + u[2]) + u4p;
+    const double fd1 = u[1] - u[-1];
+    const double fd2 = (u3 + u[-2]) - u4m;
+    const double sd0 = (u[0] + u[2]) - 2 * u[1];
+    const double sd1 = (u[-1] + u[1]) - t0;
+    const double sd2 = (u[0] + u[-2]) - 2 * u[-1];
+    const double e = (((u[-2] * u[-2] + u[2] * u[2]) + (u[-1] * u[-1] + u[1] * u[1])) + u[0] * u[0]) * K<double>::eps;
+    const double si0 = (13. / 12. * sd0 * sd0 + 1. / 4. * fd0 * fd0) + e;
+    const double si1 = (13. / 12. * sd1 * sd1 + 1. / 4. * fd1 * fd1) + e;
+    const double si2 = (13. / 12. * sd2 * sd2 + 1. / 4. * fd2 * fd2) + e;
+    const double s = (si0 + si2) + si1;
+    // a line of zeros: 0 / DBL_MIN = 0, as 0 times 0 gives
+    const bool z = s == 0.0;
+    ok = ok && (z || w_rcp_ok(s));
+    const double y = z ? 0.0 : rcp_rn(s);
+    double t0q = quot(si0, s, y) + K<double>::eps, t1q = quot(si1, s, y) + K<double>::eps,
+           t2q = quot(si2, s, y) + K<double>::eps;
+    t0q *= t0q;
+    t1q *= t1q;
+    t2q *= t2q;
+    ok = ok && lo_word(t0q) != 0xffffffffu && lo_word(t1q) != 0xffffffffu && lo_word(t2q) != 0xffffffffu;
+    const double w0 = rcp_rn(t0q), w1 = rcp_rn(t1q), w2 = rcp_rn(t2q);
+    const double sw = (w0 + w2) + w1;
+    ok = ok && lo_word(sw) != 0xffffffffu;
+    const double yw = rcp_rn(sw);
+    w[0] = quot(w0, sw, yw);
+    w[1] = quot(w1, sw, yw);
+    w[2] = quot(w2, sw, yw);
+  }
+  if (!ok) unopt3(code == kBlend ? mono(u, un) : 0.0, u, un, w);
+}
+
+// lower-order fraction of a cell from its weights, weights[0] of cell-2 and
+// weights[2] of cell+2 (ratio_lof)
+template <typename T>
+__device__ __forceinline__ T lower_fraction(int code, T wc0, T wc2, T wl0, T wr2) {
+  const T wc[3] = {wc0, T(0.0), wc2};
+  return ratio_lof(wc, wl0, wr2, code == kCusp ? T(1.0) : T(0.0));
+}
+// FP64: a ratio below 1.3 gives 0 and both above 1.6 give 1; the quotients
+// are formed in between (the margins are far wider than a rounding).  The
+// reference's MIN takes the second ratio when the first is NaN, and a NaN
+// second ratio makes the fraction 1: the ordered comparisons follow that.
+template <>
+__device__ __forceinline__ double lower_fraction<double>(int code, double wc0, double wc2, double wl0, double wr2) {
+  if (code == kCusp) return 1.0;
+  const double na = wc2 + K<double>::eps, nb = wl0 + K<double>::eps;
+  const double ma = wc0 + K<double>::eps, mb = wr2 + K<double>::eps;
+  const double lo2 = 1.2999 * mb;
+  if (ma < lo2 || (na < 1.2999 * nb && ma >= lo2)) return 0.0;
+  if (na > 1.6001 * nb && ma > 1.6001 * mb) return 1.0;
+  const double wc[3] = {wc0, 0.0, wc2};
+  return ratio_lof(wc, wl0, wr2, 0.0);
+}
+
+template <typename T>
+__device__ __forceinline__ void face_values(int code, const T *u, const T *un, const T w[3], T lof, T *yl, T *yr) {
+  const T m0 = code == kBlend ? mono(u, un) : (code == kOne ? T(1.0) : T(0.0));
+  faces(u, un, m0, code == kCusp, w, lof, yl, yr);
+}
+template <>
+__device__ __forceinline__ void face_values<double>(int code, const double *u, const double *un, const double w[3],
+                                                    double lof, double *yl, double *yr) {
+  if (code == kOne) {
+    *yl = eno5(false, u);
+    *yr = eno5(true, u);
+    return;
+  }
+  bool ok = code != kBlend;
+  // optimised order-3 weights (their sum is at least 1/16)
+  double l0 = w[0] * (1. / 16.), m1 = w[1] * (5. / 8.), l2 = w[2] * (5. / 16.);
+  double r0 = w[0] * (5. / 16.), r2 = w[2] * (1. / 16.);
+  const double sl = (l0 + l2) + m1, sr = (r0 + r2) + m1;
+  ok = ok && lo_word(sl) != 0xffffffffu && lo_word(sr) != 0xffffffffu;
+  const double ysl = rcp_rn(sl), ysr = rcp_rn(sr);
+  l0 = quot(l0, sl, ysl);
+  double l1 = quot(m1, sl, ysl);
+  l2 = quot(l2, sl, ysl);
+  r0 = quot(r0, sr, ysr);
+  double r1 = quot(m1, sr, ysr);
+  r2 = quot(r2, sr, ysr);
+  const double dm = u[-1], d0 = u[0], dp = u[1];
+  double vl2 = 0.0, vr2 = 0.0;
+  if (0.0 < lof) {
+    const double f = 1. - lof;
+    l0 *= f;
+    l1 *= f;
+    l2 *= f;
+    r0 *= f;
+    r1 *= f;
+    r2 *= f;
+    // unopt2 and its optimised weights
+    const double fd0 = dp - d0, fd1 = d0 - dm;
+    const double e = ((dm * dm + dp * dp) + d0 * d0) * K<double>::eps;
+    const double si0 = fd0 * fd0 + e, si1 = fd1 * fd1 + e;
+    const double s = si0 + si1;
+    const bool z = s == 0.0;
+    ok = ok && (z || w_rcp_ok(s));
+    const double y = z ? 0.0 : rcp_rn(s);
+    double t0 = quot(si0, s, y) + K<double>::eps, t1 = quot(si1, s, y) + K<double>::eps;
+    t0 *= t0;
+    t1 *= t1;
+    ok = ok && lo_word(t0) != 0xffffffffu && lo_word(t1) != 0xffffffffu;
+    double w0 = rcp_rn(t0), w1 = rcp_rn(t1);
+    const double sw = w0 + w1;
+    ok = ok && lo_word(sw) != 0xffffffffu;
+    const double yw = rcp_rn(sw);
+    w0 = quot(w0, sw, yw);
+    w1 = quot(w1, sw, yw);
+    double a0 = w0 * (1. / 4.), a1 = w1 * (3. / 4), b0 = w0 * (3. / 4.), b1 = w1 * (1. / 4.);
+    const double sa = a0 + a1, sb = b0 + b1;
+    ok = ok && lo_word(sa) != 0xffffffffu && lo_word(sb) != 0xffffffffu;
+    const double ya = rcp_rn(sa), yb = rcp_rn(sb);
+    a0 = quot(a0, sa, ya) * lof;
+    a1 = quot(a1, sa, ya) * lof;
+    b0 = quot(b0, sb, yb) * lof;
+    b1 = quot(b1, sb, yb) * lof;
+    const double h0 = (1. / 2.) * d0;
+    vl2 = a0 * ((3. / 2.) * d0 + (-1. / 2.) * dp) + a1 * ((1. / 2.) * dm + h0);
+    vr2 = b0 * (h0 + (1. / 2.) * dp) + b1 * ((-1. / 2.) * dm + (3. / 2.) * d0);
+  }
+  const double p38 = (3. / 8.) * d0, p34 = (3. / 4.) * d0, p158 = (15. / 8.) * d0;
+  const double q38 = (3. / 8.) * dp, q34 = (3. / 4.) * dp, q54 = (-5. / 4.) * dp, q18 = (-1. / 8.) * dp;
+  const double s38 = (3. / 8.) * dm, s34 = (3. / 4.) * dm, s54 = (-5. / 4.) * dm, s18 = (-1. / 8.) * dm;
+  const double vl = (l0 * ((p158 + (3. / 8.) * u[2]) + q54) + l2 * (((-1. / 8.) * u[-2] + p38) + s34)) +
+                    l1 * ((s38 + q18) + p34);
+  const double vr = (r0 * ((p38 + (-1. / 8.) * u[2]) + q34) + r2 * (((3. / 8.) * u[-2] + p158) + s54)) +
+                    r1 * ((s18 + q38) + p34);
+  *yl = vl + vl2;
+  *yr = vr + vr2;
+  if (!ok)
+    faces(u, un, code == kBlend ? mono(u, un) : 0.0, code == kCusp, w, lof, yl, yr);
 }
 
 }  // namespace w5
