@@ -802,6 +802,9 @@ def algorithmic_bytes(kernel, n1, n2, n3, lim="MC", tx=1):
     t = 2 * tx
     faces = {"flux_x1": (n1 + 1) * (n2 + t) * (n3 + t), "flux_x2": (n1 + t) * (n2 + 1) * (n3 + t),
              "flux_x3": (n1 + t) * (n2 + t) * (n3 + 1)}
+    if kernel == "flux":
+        # every direction of a point reconstruction in one launch
+        return sum(f for f, n in zip(faces.values(), (n1, n2, n3)) if n > 1) * (64 + 64)
     if kernel in faces:
         if lim == "WENO5":
             return faces[kernel] * (128 + 64)     # read the two face states (16 doubles), write 8 fluxes

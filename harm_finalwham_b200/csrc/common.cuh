@@ -13,14 +13,18 @@
 namespace hg {
 
 // geometry component offsets
-// per location: gcov 16, gcon 16, gcovpert_tt, gdet, then what derive_metric
-// makes of them: alpha, 1/alpha, beta^1..3, 1/gdet
-constexpr int GLOC = 40;
+constexpr int GLOC = 34;                  // per location: gcov 16, gcon 16, gcovpert_tt, gdet
+// What derive_metric forms at upload.  The face kernels read gcon's upper
+// triangle alone, so at the faces its lower triangle (planes 16 + 4a + b, b <
+// a) holds alpha, 1/alpha, beta^1..3, 1/gdet; the inversion reads all of gcon
+// at CENT, where alpha and 1/alpha have planes of their own.
+__host__ __device__ constexpr int g_derived(int q) { return 16 + (q == 0 ? 4 : (q == 1 ? 8 : (q == 2 ? 9 : 9 + q))); }
 constexpr int G_FACE1 = 0, G_FACE2 = 1, G_FACE3 = 2, G_CENT = 3;
 constexpr int G_CORN = 4 * GLOC;          // CORN1, CORN2, CORN3 gdet
 constexpr int G_CONN = G_CORN + 3;        // 64
 constexpr int G_FLOOR = G_CONN + 64;      // 2
-constexpr int G_NCOMP = G_FLOOR + 2;      // 229
+constexpr int G_LAPSE = G_FLOOR + 2;      // CENT: alpha, 1/alpha
+constexpr int G_NCOMP = G_LAPSE + 2;      // 207
 
 // reference location ids (global.h:948-955)
 constexpr int R_FACE1 = 0, R_FACE2 = 1, R_FACE3 = 2, R_CORN1 = 3, R_CORN2 = 4, R_CORN3 = 5, R_CENT = 7;
@@ -98,6 +102,7 @@ struct Scalars {
   int done;                        // t reached tf: later steps leave the state unchanged
   int nsteps;                      // time steps taken since the last upload
   unsigned long long nfloor;       // zone floorings by fixup1zone (summed over a call's final substeps)
+  unsigned int blocks_done;        // blocks of a bound kernel that are through (wraps to 0 with the last)
 };
 
 __device__ __forceinline__ long long zix(const Dims &d, int i, int j, int k) {
@@ -107,20 +112,34 @@ __device__ __forceinline__ long long gix(const Dims &d, int i, int j) {
   return (long long)(i + d.g1) * d.gt2 + (j + d.g2);
 }
 
-__device__ __forceinline__ void load_metric(const double *__restrict__ G, const Dims &d, long long ij, int slot,
-                                            Metric &m) {
+// metric of one location converted to the arithmetic type of a kernel
+template <typename T>
+__device__ __forceinline__ void load_metric_t(const double *__restrict__ G, const Dims &d, long long ij, int slot,
+                                              MetricT<T> &m) {
   const double *b = G + (long long)slot * GLOC * d.nij + ij;
 #pragma unroll
-  for (int q = 0; q < 16; q++) m.gcov[q] = __ldg(b + (long long)q * d.nij);
+  for (int q = 0; q < 16; q++) m.gcov[q] = (T)__ldg(b + (long long)q * d.nij);
 #pragma unroll
-  for (int q = 0; q < 16; q++) m.gcon[q] = __ldg(b + (long long)(16 + q) * d.nij);
-  m.gcovpert_tt = __ldg(b + (long long)32 * d.nij);
-  m.g = __ldg(b + (long long)33 * d.nij);
-  m.alpha = __ldg(b + (long long)34 * d.nij);
-  m.ralpha = __ldg(b + (long long)35 * d.nij);
+  for (int q = 0; q < 16; q++)
+    if (slot == G_CENT || (q & 3) >= (q >> 2)) m.gcon[q] = (T)__ldg(b + (long long)(16 + q) * d.nij);
+  m.gcovpert_tt = (T)__ldg(b + (long long)32 * d.nij);
+  m.g = (T)__ldg(b + (long long)33 * d.nij);
+  if (slot == G_CENT) {
+    m.alpha = (T)__ldg(G + (long long)G_LAPSE * d.nij + ij);
+    m.ralpha = (T)__ldg(G + (long long)(G_LAPSE + 1) * d.nij + ij);
+    derive_shift(m);
+    m.rg = kept_rcp(m.g);
+  } else {
+    m.alpha = (T)__ldg(b + (long long)g_derived(0) * d.nij);
+    m.ralpha = (T)__ldg(b + (long long)g_derived(1) * d.nij);
 #pragma unroll
-  for (int q = 0; q < 3; q++) m.beta[q] = __ldg(b + (long long)(36 + q) * d.nij);
-  m.rg = __ldg(b + (long long)39 * d.nij);
+    for (int q = 0; q < 3; q++) m.beta[q] = (T)__ldg(b + (long long)g_derived(2 + q) * d.nij);
+    m.rg = (T)__ldg(b + (long long)g_derived(5) * d.nij);
+  }
+}
+__device__ __forceinline__ void load_metric(const double *__restrict__ G, const Dims &d, long long ij, int slot,
+                                            Metric &m) {
+  load_metric_t(G, d, ij, slot, m);
 }
 
 __device__ __forceinline__ void load_prim(const double *__restrict__ P, const Dims &d, long long z, double *pr) {
@@ -227,7 +246,8 @@ __device__ __forceinline__ void para4(const T *y, T *lout, T *rout) {
 // Measured on the B200, us per step: flux 4 against 3 blocks 3438 / 3679 on
 // the 256x128x128 WENO5 torus, 237 / 259 on 97x51x33 MC, 58 / 54 on 64x64
 // (there the few warps gain nothing from the fourth block and pay its
-// spills); update 4 against 3 blocks 2240 / 1505, 154 / 85, 36 / 27: its
+// spills); WENO5 4 against 3 blocks 8921 / 9716 on 256x128x128, 1008 / 1100 on
+// 128x64x32; update 4 against 3 blocks 2240 / 1505, 154 / 85, 36 / 27: its
 // spills sit in the contraction with the connection, so 3.
 #ifndef HG_MINB_FLUX
 #define HG_MINB_FLUX 4
@@ -269,24 +289,6 @@ __device__ __forceinline__ long long dir_stride(const Dims &d) {
   return (DIR == 1) ? (long long)d.nt2 * d.nt3 : ((DIR == 2) ? (long long)d.nt3 : 1);
 }
 
-// metric of one location converted to the arithmetic type of a kernel
-template <typename T>
-__device__ __forceinline__ void load_metric_t(const double *__restrict__ G, const Dims &d, long long ij, int slot,
-                                              MetricT<T> &m) {
-  const double *b = G + (long long)slot * GLOC * d.nij + ij;
-#pragma unroll
-  for (int q = 0; q < 16; q++) m.gcov[q] = (T)__ldg(b + (long long)q * d.nij);
-#pragma unroll
-  for (int q = 0; q < 16; q++) m.gcon[q] = (T)__ldg(b + (long long)(16 + q) * d.nij);
-  m.gcovpert_tt = (T)__ldg(b + (long long)32 * d.nij);
-  m.g = (T)__ldg(b + (long long)33 * d.nij);
-  m.alpha = (T)__ldg(b + (long long)34 * d.nij);
-  m.ralpha = (T)__ldg(b + (long long)35 * d.nij);
-#pragma unroll
-  for (int q = 0; q < 3; q++) m.beta[q] = (T)__ldg(b + (long long)(36 + q) * d.nij);
-  m.rg = (T)__ldg(b + (long long)39 * d.nij);
-}
-
 // ---------------------------------------------------------------------------
 // WENO5 line reconstruction (slope_lim_linetype_c2e, interpline.c:517-678),
 // one kernel per direction.  The reference sweeps whole lines serially; here
@@ -313,10 +315,11 @@ __device__ __forceinline__ void load_metric_t(const double *__restrict__ G, cons
 // from each cell's own value and writes FP64 face values (the cell's value
 // plus the FP32 offset), which the FP64 Riemann kernel reads.
 //
-// Bound by instruction issue, FP64 first.  The form before this one staged
-// tiles of a line in shared memory, one stage at a time between barriers, and
-// held 1.7 other instructions (addresses, shared memory, selects, the
-// branches of its divisions) to an FP64 one.
+// Bound by instruction issue, FP64 first (FP64 pipe 51-59% active, 250 FP64
+// instructions a cell and primitive).  The form before this one staged tiles
+// of a line in shared memory, one stage at a time between barriers, and held
+// 1.7 other instructions (addresses, shared memory, selects, the branches of
+// its divisions) to an FP64 one: 2.63 -> 1.49 ms a launch on 256x128x128.
 // ---------------------------------------------------------------------------
 constexpr int W5_THREADS = 128;
 constexpr int W5_CHUNK = 8;               // FS: line cells staged per warp and turn
@@ -555,13 +558,12 @@ __global__ void __launch_bounds__(W5_THREADS, MB) weno5_kernel(Dims d, W5Tile tl
 // 256x128x128 WENO5 torus one direction takes 0.57 ms a launch, 1.14 ms
 // while every quotient was a division of its own and the tensors' zero
 // diagonals and the unit vectors of simplefast were multiplied out.
-template <int DIR, int RECON, typename T, int MB = MinBlocks<T>::flux, typename TR = T, int MIX = 0>
-__global__ void __launch_bounds__(128, MB) flux_kernel(Dims d, Params P, Box box,
-                                                                 const double *__restrict__ pb,
-                                                                 const TR *__restrict__ pL, const TR *__restrict__ pR,
-                                                                 const double *__restrict__ G, double *__restrict__ F,
-                                                                 Scalars *sc) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+template <int DIR, int RECON, typename T, typename TR, int MIX>
+__device__ __forceinline__ void flux_block(unsigned block, const Dims &d, const Params &P, const Box &box,
+                                           const double *__restrict__ pb, const TR *__restrict__ pL,
+                                           const TR *__restrict__ pR, const double *__restrict__ G,
+                                           double *__restrict__ F, Scalars *sc) {
+  long long t = (long long)block * blockDim.x + threadIdx.x;
   bool active = t < box.size();
   double dtij = 0.0;
   if (active) {
@@ -663,7 +665,7 @@ __global__ void __launch_bounds__(128, MB) flux_kernel(Dims d, Params P, Box box
       // flux_ct gdet strip (fluxct.c:74-96), in FP64 in both precision modes
       const double *gf = G + (long long)((DIR - 1) * GLOC) * d.nij + gix(d, i, j);
       double Fs[3];
-      div_n<3>(Fo + B1, known_divisor(__ldg(gf + 33 * d.nij), __ldg(gf + 39 * d.nij)), Fs);
+      div_n<3>(Fo + B1, known_divisor(__ldg(gf + 33 * d.nij), __ldg(gf + g_derived(5) * d.nij)), Fs);
       Fo[B1] = Fs[0];
       Fo[B2] = Fs[1];
       Fo[B3] = Fs[2];
@@ -686,6 +688,80 @@ __global__ void __launch_bounds__(128, MB) flux_kernel(Dims d, Params P, Box box
     }
   }
   warp_min_atomic(&sc->ndtbits[DIR], dtij, active);
+}
+
+template <int DIR, int RECON, typename T, int MB = MinBlocks<T>::flux, typename TR = T, int MIX = 0>
+__global__ void __launch_bounds__(128, MB) flux_kernel(Dims d, Params P, Box box,
+                                                                 const double *__restrict__ pb,
+                                                                 const TR *__restrict__ pL, const TR *__restrict__ pR,
+                                                                 const double *__restrict__ G, double *__restrict__ F,
+                                                                 Scalars *sc) {
+  flux_block<DIR, RECON, T, TR, MIX>(blockIdx.x, d, P, box, pb, pL, pR, G, F, sc);
+}
+
+// get_bsqflags (fixup.c:1751-1849), which pre_fixup runs on the stage's
+// input state at the start of every RK stage (step_ch.c:117-120): per zone,
+// with the CENT metric, b^2/rho against BSQORHOLIMIT and b^2/u against
+// BSQOULIMIT (initbase.c:465-466), 2 above the limit, 1 above 0.9 of it,
+// else 0: the FLAGBSQORHO and FLAGBSQOU slots of pflag, packed as
+// FLAGBSQORHO | FLAGBSQOU << 2.  With LIMADJUST = FLUXADJUST = 0 they change
+// no state; the last stage's values are what the reference leaves in pflag.
+// A state whose u^t has no real solution sets ERR_UTCALC_DISCR, as the
+// reference's FAILSTATEMENT ends the step.
+constexpr double BSQORHOLIMIT = 20.0, BSQOULIMIT = 100.0;
+__device__ __forceinline__ void bsqflags_zone(long long z, const Dims &d, const double *__restrict__ pv,
+                                              const double *__restrict__ G, unsigned char *__restrict__ bf,
+                                              Scalars *sc) {
+  if (z >= d.nz) return;
+  const long long r = z / d.nt3;
+  const int j = (int)(r % d.nt2) - d.g2;
+  const int i = (int)(r / d.nt2) - d.g1;
+  double pr[NPR];
+  load_prim(pv, d, z, pr);
+  Metric m;
+  load_metric(G, d, gix(d, i, j), G_CENT, m);
+  State q;
+  if (get_state(pr, m, q)) {
+    atomicOr(&sc->err, ERR_UTCALC_DISCR);
+    bf[z] = 0;
+    return;
+  }
+  const double bsq = dot4(q.bcon, q.bcov);
+  int f0, f3;
+  if (bsq / pr[RHO] > BSQORHOLIMIT) f0 = 2;
+  else if (bsq / pr[RHO] > 0.9 * BSQORHOLIMIT) f0 = 1;
+  else f0 = 0;
+  if (bsq / pr[UU] > BSQOULIMIT) f3 = 2;
+  else if (bsq / pr[UU] > 0.9 * BSQOULIMIT) f3 = 1;
+  else f3 = 0;
+  bf[z] = (unsigned char)(f0 | (f3 << 2));
+}
+
+// The faces of every direction in one launch (point reconstructions, whose
+// states need no pass of their own), and behind them, on the last RK stage,
+// the b^2 flags of the state pi.  The directions and the flags do not depend
+// on one another: on a 64x64 grid one direction's 33 blocks take 11 us on 148
+// SMs, all of it latency, so that two directions at once cost the time of
+// one; on large grids the last wave of one direction fills with the next.
+struct FluxJob {
+  Box box[4];             // faces per direction
+  unsigned first[5];      // first block of direction 1, 2, 3, of the flags, and the number of blocks
+  double *F[4];
+  const double *pi;
+  unsigned char *bsqf;
+};
+template <int RECON, typename T, int MB = MinBlocks<T>::flux>
+__global__ void __launch_bounds__(128, MB) fluxes_kernel(Dims d, Params P, FluxJob J, const double *__restrict__ pb,
+                                                         const double *__restrict__ G, Scalars *sc) {
+  const unsigned b = blockIdx.x;
+  if (b < J.first[1])
+    flux_block<1, RECON, T, T, 0>(b, d, P, J.box[1], pb, nullptr, nullptr, G, J.F[1], sc);
+  else if (b < J.first[2])
+    flux_block<2, RECON, T, T, 0>(b - J.first[1], d, P, J.box[2], pb, nullptr, nullptr, G, J.F[2], sc);
+  else if (b < J.first[3])
+    flux_block<3, RECON, T, T, 0>(b - J.first[2], d, P, J.box[3], pb, nullptr, nullptr, G, J.F[3], sc);
+  else
+    bsqflags_zone((long long)(b - J.first[3]) * blockDim.x + threadIdx.x, d, J.pi, G, J.bsqf, sc);
 }
 
 

@@ -110,6 +110,7 @@ HG_HD Divisor<double> known_divisor(double b, double y) { return Divisor<double>
 HG_HD Divisor<float> known_divisor(float b, float) { return Divisor<float>{b}; }
 // the reciprocal to keep for known_divisor
 HG_HD double kept_rcp(double b) { return rcp_ok(b) ? rcp_rn(b) : 0.0; }
+HG_HD float kept_rcp(float) { return 0.f; }
 
 // q[i] = a[i] / d, i < N.  One maximum over the exponent words tells whether
 // every numerator is in range; zeros fail it and are let through by the

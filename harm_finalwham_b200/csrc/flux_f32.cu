@@ -17,10 +17,6 @@ namespace hg {
                                                           double *, double *);                                      \
   template __global__ void weno5_kernel<DIR, false, float>(Dims, W5Tile, const double *, const float *,           \
                                                            double *, double *);                                     \
-  template __global__ void flux_kernel<DIR, 0, float>(Dims, Params, Box, const double *, const float *,           \
-                                                      const float *, const double *, double *, Scalars *);          \
-  template __global__ void flux_kernel<DIR, 2, float>(Dims, Params, Box, const double *, const float *,           \
-                                                      const float *, const double *, double *, Scalars *);          \
   template __global__ void flux_kernel<DIR, 1, double, kFluxMB[0], double, 1>(                                    \
       Dims, Params, Box, const double *, const double *, const double *, const double *, double *, Scalars *);      \
   template __global__ void flux_kernel<DIR, 1, double, kFluxMB[1], double, 1>(                                    \
@@ -29,6 +25,8 @@ namespace hg {
 HG_F32_INSTANCES(1)
 HG_F32_INSTANCES(2)
 HG_F32_INSTANCES(3)
+template __global__ void fluxes_kernel<0, float>(Dims, Params, FluxJob, const double *, const double *, Scalars *);
+template __global__ void fluxes_kernel<2, float>(Dims, Params, FluxJob, const double *, const double *, Scalars *);
 template __global__ void w5_state_kernel<float>(Dims, Params, Box, const double *, const double *, float *);
 template __global__ void w5_shock_kernel<float>(Dims, Box, const double *, const float *, float *);
 

@@ -106,11 +106,15 @@ using EM = EMT<double>;
 
 // alpha and beta^i of ucon_calc_rel4vel (phys.c:983-1019) and the kept
 // reciprocals, from gcon and gdet
+template <typename T>
+__device__ __forceinline__ void derive_shift(MetricT<T> &m) {
+#pragma unroll
+  for (int j = 0; j < 3; j++) m.beta[j] = GCON(m, 0, j + 1) * m.alpha * m.alpha;
+}
 __device__ __forceinline__ void derive_metric(Metric &m) {
   m.alpha = 1. / sqrt(-GCON(m, 0, 0));
   m.ralpha = kept_rcp(m.alpha);
-#pragma unroll
-  for (int j = 0; j < 3; j++) m.beta[j] = GCON(m, 0, j + 1) * m.alpha * m.alpha;
+  derive_shift(m);
   m.rg = kept_rcp(m.g);
 }
 

@@ -5,9 +5,8 @@
 //   primitives, conserved accumulators, fluxes: SoA planes [8][nt1][nt2][nt3]
 //     with x3 fastest, so that the 32 threads of a warp walk x3 at one (i,j)
 //     and read one metric row (broadcast) -- the metric depends on (i,j) only.
-//   geometry: SoA [component][gt1*gt2], 229 doubles per (i,j):
-//     4 locations (FACE1, FACE2, FACE3, CENT) x {gcov 16, gcon 16, gcovpert_tt, gdet,
-//     lapse, 1/lapse, shift 3, 1/gdet},
+//   geometry: SoA [component][gt1*gt2], 207 doubles per (i,j):
+//     4 locations (FACE1, FACE2, FACE3, CENT) x {gcov 16, gcon 16, gcovpert_tt, gdet},
 //     CORN1..3 gdet, conn[64] at CENT, floors[2].
 //
 // Work per RK substep (the reference's advance(), step_ch.c:94-186):
@@ -29,6 +28,7 @@
 //                     formulation that reproduces the reference's sequential
 //                     sweep exactly (see checksol_resolve / fixup_compute)
 //   finalize_kernel   ndt combine (advance.c:231) and dt update (step_ch.c:236-247)
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -55,10 +55,6 @@ namespace hg {
                                                                 double *, double *);                             \
   extern template __global__ void weno5_kernel<DIR, false, float>(Dims, W5Tile, const double *, const float *,      \
                                                                 double *, double *);                             \
-  extern template __global__ void flux_kernel<DIR, 0, float>(Dims, Params, Box, const double *, const float *,    \
-                                                             const float *, const double *, double *, Scalars *);   \
-  extern template __global__ void flux_kernel<DIR, 2, float>(Dims, Params, Box, const double *, const float *,    \
-                                                             const float *, const double *, double *, Scalars *);   \
   extern template __global__ void flux_kernel<DIR, 1, double, kFluxMB[0], double, 1>(                             \
       Dims, Params, Box, const double *, const double *, const double *, const double *, double *, Scalars *);      \
   extern template __global__ void flux_kernel<DIR, 1, double, kFluxMB[1], double, 1>(                             \
@@ -66,6 +62,8 @@ namespace hg {
 HG_F32_EXTERN(1)
 HG_F32_EXTERN(2)
 HG_F32_EXTERN(3)
+extern template __global__ void fluxes_kernel<0, float>(Dims, Params, FluxJob, const double *, const double *, Scalars *);
+extern template __global__ void fluxes_kernel<2, float>(Dims, Params, FluxJob, const double *, const double *, Scalars *);
 extern template __global__ void w5_state_kernel<float>(Dims, Params, Box, const double *, const double *, float *);
 extern template __global__ void w5_shock_kernel<float>(Dims, Box, const double *, const float *, float *);
 }  // namespace hg
@@ -90,9 +88,32 @@ void set_err(const char *fmt, const char *a = "", int b = 0) {
 // ---------------------------------------------------------------------------
 // corner EMFs (fluxct.c:104-218) on the corners the updated faces read
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) emf_kernel(Dims d, Box box, const double *__restrict__ F1,
+// What reset_stage_kernel clears, for the kernels that do it in passing.
+// step_ch's own loop needs no launch for it: the counters are added to after
+// the EMFs, and the dt minima of a stage that is not the last are not read.
+__device__ __forceinline__ void clear_ndt(const Params &P, Scalars *sc, int thread, int threads) {
+  const unsigned long long big = (unsigned long long)__double_as_longlong(BIGNUM);
+  if (thread >= 1 && thread <= 3) sc->ndtbits[thread] = big;
+  if (P.cell_inst)
+    for (int b = thread; b < P.ninst; b += threads) P.inst[b].ndtbits = big;
+}
+__device__ __forceinline__ void clear_stage_counts(Scalars *sc) {
+  sc->nfail = 0;
+  sc->ncand = 0;
+  sc->ndep = 0;
+  sc->nfixlist = 0;
+}
+
+// stage_clear: 0 nothing (reset_stage_kernel ran before the stage), 1 the
+// counters that the kernels after this one add to, 2 the dt minima too
+__global__ void __launch_bounds__(256) emf_kernel(Dims d, Params P, Box box, const double *__restrict__ F1,
                                                   const double *__restrict__ F2, const double *__restrict__ F3,
-                                                  const double *__restrict__ G, double *__restrict__ E) {
+                                                  const double *__restrict__ G, double *__restrict__ E, Scalars *sc,
+                                                  int stage_clear) {
+  if (stage_clear && blockIdx.x == 0) {
+    if (threadIdx.x == 0) clear_stage_counts(sc);
+    if (stage_clear == 2) clear_ndt(P, sc, threadIdx.x, blockDim.x);
+  }
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= box.size()) return;
   int i, j, k;
@@ -474,6 +495,97 @@ __global__ void __launch_bounds__(128, FV ? 3 : MB) invert_kernel(Dims d, Params
   }
 }
 
+// ndt (advance.c:231) and the dt update of step_ch (step_ch.c:236-247)
+__device__ __forceinline__ void finalize_one(const Params &P, Scalars *sc, int advance_time) {
+  double n1 = __longlong_as_double((long long)sc->ndtbits[1]);
+  double n2 = __longlong_as_double((long long)sc->ndtbits[2]);
+  double n3 = __longlong_as_double((long long)sc->ndtbits[3]);
+  double ndt = P.defcon * 1. / (1. / n1 + 1. / n2 + 1. / n3);
+  if (advance_time && !sc->done) {
+    double dt = sc->dt;
+    sc->t += dt;
+    if (ndt > P.safe * dt) ndt = P.safe * dt;
+    dt = ndt;
+    if (sc->t + dt > P.tf) dt = P.tf - sc->t;
+    sc->dt = dt;
+    // the reference's main loop runs while t < tf (main.c:33)
+    sc->nsteps++;
+    if (!(sc->t < P.tf)) sc->done = 1;
+  }
+  // keep the last ndt where the host can read it
+  sc->ndtbits[0] = (unsigned long long)__double_as_longlong(ndt);
+}
+
+// batch: per-instance ndt combine and dt update (the same formulas per
+// instance; dims of size 1 contribute BIG as in the one-domain case)
+__device__ __forceinline__ void finalize_inst(const Params &P, int b, int advance_time) {
+  Inst &I = P.inst[b];
+  double n1 = __longlong_as_double((long long)I.ndtbits);
+  double ndt = P.defcon * 1. / (1. / n1 + 1. / BIGNUM + 1. / BIGNUM);
+  if (advance_time) {
+    if (I.done) return;
+    double dt = I.dt;
+    I.t += dt;
+    I.nsteps++;
+    if (ndt > P.safe * dt) ndt = P.safe * dt;
+    dt = ndt;
+    if (I.t + dt > I.tf) dt = I.tf - I.t;
+    I.dt = dt;
+    if (!(I.t < I.tf)) I.done = 1;
+  } else {
+    I.dt = ndt;
+  }
+}
+
+__global__ void finalize_kernel(Params P, Scalars *sc, int advance_time) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) finalize_one(P, sc, advance_time);
+}
+
+__global__ void finalize_batch_kernel(Params P, int advance_time) {
+  int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < P.ninst) finalize_inst(P, b, advance_time);
+}
+
+// one block: before a stage (counts), or at the start of a call of steps
+// (call: also what accumulates over a call, as clear_counters)
+__global__ void reset_stage_kernel(Params P, Scalars *sc, int call) {
+  clear_ndt(P, sc, threadIdx.x, blockDim.x);
+  if (threadIdx.x != 0) return;
+  clear_stage_counts(sc);
+  if (call) {
+    sc->iters = 0;
+    sc->err = 0;
+    sc->nfixed = 0;
+    sc->overflow = 0;
+    sc->nfloor = 0;
+  }
+}
+
+// the dt update that closes a step, by the last kernel's last block; the dt
+// minima are left for the next step's first stage
+__device__ __forceinline__ void close_step(const Params &P, Scalars *sc) {
+  if (P.cell_inst)
+    for (int b = threadIdx.x; b < P.ninst; b += blockDim.x) finalize_inst(P, b, 1);
+  else if (threadIdx.x == 0)
+    finalize_one(P, sc, 1);
+  __syncthreads();
+  clear_ndt(P, sc, threadIdx.x, blockDim.x);
+}
+
+// whether this block is the last of the grid to come here: everything that
+// the others read or wrote before is done and visible
+__device__ __forceinline__ bool last_block(Scalars *sc) {
+  __shared__ int last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicInc(&sc->blocks_done, gridDim.x - 1) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  return last;
+}
+
 // ---------------------------------------------------------------------------
 // boundaries: bound_prim_user (bounds.fishmon.c:29-345)
 // ---------------------------------------------------------------------------
@@ -648,30 +760,27 @@ __global__ void bondi_bc_kernel(Dims d, Params P, double *p, const double *__res
   if (err) atomicOr(&sc->err, err);
 }
 
-// Every ghost zone of the full box as the composition of the reference's
+// One ghost zone of the full box as the composition of the reference's
 // sequential fills: x1 (active j,k: copy + inflow check + gamma limit with the
 // ghost's own metric; the Bondi-integral ghosts come from bondi_bc_kernel),
 // then x2 (full i, active k: reflection, and either POLEDEATH zeroing of u~2
 // and B2 (bounds.fishmon.c) or their negation (the generic bounds.c,
-// HGPU_BC_POLARAXIS_FLIP)), then x3 (full i, full j: periodic copy).  Reads
-// only zones this kernel does not write.
-__global__ void __launch_bounds__(128) bound_ghost_kernel(Dims d, Params P, double *p, const double *__restrict__ G,
-                                                          Scalars *sc) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= d.nz) return;
-  int k = (int)(t % d.nt3) - d.g3;
-  long long r = t / d.nt3;
-  int j = (int)(r % d.nt2) - d.g2;
-  int i = (int)(r / d.nt2) - d.g1;
-  bool gi = (i < 0 || i >= d.n1), gj = (j < 0 || j >= d.n2), gk = (k < 0 || k >= d.n3);
-  if (!(gi || gj || gk)) return;
+// HGPU_BC_POLARAXIS_FLIP)), then x3 (full i, full j: periodic copy); pflag
+// (unless null): the failure flags too (bound_pflag_user, boundsint.c:6-266,
+// is the same composition).  Reads only zones that no ghost is.
+__device__ __forceinline__ void bound_ghost(const Dims &d, const Params &P, int i, int j, int k, double *p,
+                                            const double *__restrict__ G, Scalars *sc, int *pflag) {
+  const bool gi = (i < 0 || i >= d.n1), gj = (j < 0 || j >= d.n2), gk = (k < 0 || k >= d.n3);
   // x1 ghosts of active j, k on a Bondi-integral side: bondi_bc_kernel's
   if (gi && !gj && !gk && is_bondi(i < 0 ? P.bc[1] : P.bc[0])) return;
   int si = map_idx(i, d.n1, P.bc[1], P.bc[0]);
   int sj = map_idx(j, d.n2, P.bc[3], P.bc[2]);
   int sk = map_idx(k, d.n3, P.bc[5], P.bc[4]);
+  const long long z = zix(d, i, j, k), zs = zix(d, si, sj, sk);
+  // a finished domain is frozen: its ghost flags keep the values of its last step
+  if (pflag && !sc->done) pflag[z] = pflag[zs];
   double pr[NPR];
-  load_prim(p, d, zix(d, si, sj, sk), pr);
+  load_prim(p, d, zs, pr);
   int err = 0;
   // the generic bounds.c's polar reflection (bounds.c:477-489)
   if (gj && ((j < 0 && P.bc[3] == HGPU_BC_POLARAXIS_FLIP) || (j >= d.n2 && P.bc[2] == HGPU_BC_POLARAXIS_FLIP))) {
@@ -692,71 +801,67 @@ __global__ void __launch_bounds__(128) bound_ghost_kernel(Dims d, Params P, doub
     pr[U2] *= 0;
     pr[B2] *= 0.;
   }
-  store_prim(p, d, t, pr);
+  store_prim(p, d, z, pr);
   if (err) atomicOr(&sc->err, err);
 }
 
-// POLEDEATH on the active first/last x2 rows (after the ghosts have read them)
-__global__ void bound_pole_kernel(Dims d, Params P, double *p) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  long long rows = (long long)d.n1 * d.n3;
-  if (t >= 2 * rows) return;
-  int side = (int)(t / rows);
-  long long r = t % rows;
-  int i = (int)(r / d.n3), k = (int)(r % d.n3);
-  int j;
-  if (side == 0) {
-    if (!(P.bc[3] == HGPU_BC_POLARAXIS)) return;
-    j = 0;
-  } else {
-    if (!(P.bc[2] == HGPU_BC_POLARAXIS)) return;
-    j = d.n2 - 1;
+// bound_prim in one launch over the ghost zones alone (a thread per zone of
+// the box, most of them active and idle, took 60 us on 256x128x128), then
+// POLEDEATH on the active first/last x2 rows.  A ghost zone that reads such a
+// row is in it itself and zeroes what it read, in any order; only the x1
+// ghosts' inflow check looks at u~2 before that, so the rows' first and last
+// zones, which those ghosts read, wait for the last block.
+// close: that block also ends the step.
+struct BoundJob {
+  unsigned n[4];  // threads: x1 ghosts, x2 ghosts (active i), x3 ghosts (active i, j), active pole rows
+  int corners, close;
+};
+__global__ void __launch_bounds__(128) bound_kernel(Dims d, Params P, BoundJob J, double *p,
+                                                    const double *__restrict__ G, Scalars *sc, int *pflag) {
+  unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < J.n[0]) {
+    const int k = (int)(t % d.nt3) - d.g3;
+    const unsigned r = t / d.nt3;
+    const int j = (int)(r % d.nt2) - d.g2, q = (int)(r / d.nt2);
+    bound_ghost(d, P, q < d.g1 ? q - d.g1 : d.n1 + q - d.g1, j, k, p, G, sc, pflag);
+  } else if ((t -= J.n[0]) < J.n[1]) {
+    const int k = (int)(t % d.nt3) - d.g3;
+    const unsigned r = t / d.nt3;
+    const int q = (int)(r % (2 * d.g2)), i = (int)(r / (2 * d.g2));
+    bound_ghost(d, P, i, q < d.g2 ? q - d.g2 : d.n2 + q - d.g2, k, p, G, sc, pflag);
+  } else if ((t -= J.n[1]) < J.n[2]) {
+    const int q = (int)(t % (2 * d.g3));
+    const unsigned r = t / (2 * d.g3);
+    const int j = (int)(r % d.n2), i = (int)(r / d.n2);
+    bound_ghost(d, P, i, j, q < d.g3 ? q - d.g3 : d.n3 + q - d.g3, p, G, sc, pflag);
+  } else if ((t -= J.n[2]) < J.n[3]) {
+    const int k = (int)(t % d.n3);
+    const unsigned r = t / d.n3;
+    const int i = (int)(r >> 1), up = (int)(r & 1);
+    if (i > 0 && i < d.n1 - 1 && P.bc[up ? 2 : 3] == HGPU_BC_POLARAXIS) {
+      const long long z = zix(d, i, up ? d.n2 - 1 : 0, k);
+      p[(long long)U2 * d.nz + z] *= 0;
+      p[(long long)B2 * d.nz + z] *= 0.;
+    }
   }
-  long long z = zix(d, i, j, k);
-  p[(long long)U2 * d.nz + z] *= 0;
-  p[(long long)B2 * d.nz + z] *= 0.;
+  if (!(J.corners || J.close) || !last_block(sc)) return;
+  if (J.corners)
+    for (unsigned c = threadIdx.x; c < (unsigned)d.n3 * 4; c += blockDim.x) {
+      const int k = (int)(c >> 2), up = (int)(c & 1), far = (int)((c >> 1) & 1);
+      if (P.bc[up ? 2 : 3] != HGPU_BC_POLARAXIS || (far && d.n1 == 1)) continue;
+      const long long z = zix(d, far ? d.n1 - 1 : 0, up ? d.n2 - 1 : 0, k);
+      p[(long long)U2 * d.nz + z] *= 0;
+      p[(long long)B2 * d.nz + z] *= 0.;
+    }
+  if (J.close) close_step(P, sc);
+}
+
+__global__ void bsqflags_kernel(Dims d, const double *__restrict__ pv, const double *__restrict__ G,
+                                unsigned char *__restrict__ bf, Scalars *sc) {
+  bsqflags_zone((long long)blockIdx.x * blockDim.x + threadIdx.x, d, pv, G, bf, sc);
 }
 
 // bound_pflag_user (boundsint.c:6-266) as the same composition
-// get_bsqflags (fixup.c:1751-1849), which pre_fixup runs on the stage's
-// input state at the start of every RK stage (step_ch.c:117-120): per zone,
-// with the CENT metric, b^2/rho against BSQORHOLIMIT and b^2/u against
-// BSQOULIMIT (initbase.c:465-466), 2 above the limit, 1 above 0.9 of it,
-// else 0: the FLAGBSQORHO and FLAGBSQOU slots of pflag, packed as
-// FLAGBSQORHO | FLAGBSQOU << 2.  With LIMADJUST = FLUXADJUST = 0 they change
-// no state; the last stage's values are what the reference leaves in pflag.
-// A state whose u^t has no real solution sets ERR_UTCALC_DISCR, as the
-// reference's FAILSTATEMENT ends the step.
-constexpr double BSQORHOLIMIT = 20.0, BSQOULIMIT = 100.0;
-__global__ void bsqflags_kernel(Dims d, const double *__restrict__ pv, const double *__restrict__ G,
-                                unsigned char *__restrict__ bf, Scalars *sc) {
-  const long long z = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (z >= d.nz) return;
-  const int k = (int)(z % d.nt3) - d.g3;
-  const long long r = z / d.nt3;
-  const int j = (int)(r % d.nt2) - d.g2;
-  const int i = (int)(r / d.nt2) - d.g1;
-  double pr[NPR];
-  load_prim(pv, d, z, pr);
-  Metric m;
-  load_metric(G, d, gix(d, i, j), G_CENT, m);
-  State q;
-  if (get_state(pr, m, q)) {
-    atomicOr(&sc->err, ERR_UTCALC_DISCR);
-    bf[z] = 0;
-    return;
-  }
-  const double bsq = dot4(q.bcon, q.bcov);
-  int f0, f3;
-  if (bsq / pr[RHO] > BSQORHOLIMIT) f0 = 2;
-  else if (bsq / pr[RHO] > 0.9 * BSQORHOLIMIT) f0 = 1;
-  else f0 = 0;
-  if (bsq / pr[UU] > BSQOULIMIT) f3 = 2;
-  else if (bsq / pr[UU] > 0.9 * BSQOULIMIT) f3 = 1;
-  else f3 = 0;
-  bf[z] = (unsigned char)(f0 | (f3 << 2));
-}
-
 __global__ void bound_pflag_kernel(Dims d, Params P, int *pflag, const Scalars *sc) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   // a finished domain is frozen: its ghost flags keep the values of its last step
@@ -776,8 +881,8 @@ __global__ void bound_pflag_kernel(Dims d, Params P, int *pflag, const Scalars *
 // Batch of 1D instances: every instance's ghost cells are a plain copy of its
 // first / last active cell (bounds.c OUTFLOW, bounds.c:84-135, 218-292), for
 // the primitives (pv != nullptr) or the failure flags (pflag != nullptr).
-__global__ void bound_batch_kernel(Dims d, Params P, double *pv, int *pflag) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// close: the last block ends the step.
+__device__ __forceinline__ void bound_batch(long long t, const Dims &d, const Params &P, double *pv, int *pflag) {
   if (t >= d.nz) return;
   int i = (int)t - d.g1;  // the batch line is 1D
   const Inst &I = P.inst[P.cell_inst[t]];
@@ -795,6 +900,10 @@ __global__ void bound_batch_kernel(Dims d, Params P, double *pv, int *pflag) {
   }
   if (pflag) pflag[t] = pflag[zs];
 }
+__global__ void bound_batch_kernel(Dims d, Params P, double *pv, int *pflag, Scalars *sc, int close) {
+  bound_batch((long long)blockIdx.x * blockDim.x + threadIdx.x, d, P, pv, pflag);
+  if (close && last_block(sc)) close_step(P, sc);
+}
 
 // ---------------------------------------------------------------------------
 // post_fixup (fixup.c:37-96)
@@ -804,7 +913,7 @@ __global__ void bound_batch_kernel(Dims d, Params P, double *pv, int *pflag) {
 __global__ void checksol_gamma_kernel(Dims d, Params P, Box box, const double *__restrict__ pv,
                                       const double *__restrict__ G,
                                       double *__restrict__ gammacheck, long long *__restrict__ cand, int cap,
-                                      Scalars *sc) {
+                                      Scalars *sc, const int *__restrict__ pflag, long long *__restrict__ fixlist) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= box.size()) return;
   int i, j, k;
@@ -827,6 +936,11 @@ __global__ void checksol_gamma_kernel(Dims d, Params P, Box box, const double *_
     int slot = atomicAdd(&sc->ncand, 1);
     if (slot < cap) cand[slot] = z;
     else atomicOr(&sc->overflow, 1);
+  } else if (fixlist && activez && !sc->done && pflag[z] != 0) {
+    // fixup_small_kernel's list: failed zones that checksolution leaves alone
+    int slot = atomicAdd(&sc->nfixlist, 1);
+    if (slot < cap) fixlist[slot] = z;
+    else atomicOr(&sc->overflow, 2);
   }
 }
 
@@ -888,15 +1002,34 @@ __device__ __forceinline__ int checksol_vote(unsigned int b, unsigned int ok) {
   return v;
 }
 
-__global__ void checksol_map_kernel(const long long *__restrict__ cand, const int *__restrict__ pflag, int *candmap,
-                                    int *orig, int cap, const Scalars *sc) {
-  int n = sc->ncand;
-  if (n > cap) n = cap;
-  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-    const long long z = cand[a];
-    candmap[z] = a;
-    orig[a] = pflag[z];
+// the arrays and settings of post_fixup's kernels (no restrict: one kernel
+// writes what it reads later)
+struct FixJob {
+  Dims d;
+  double *pv;
+  const double *G, *gammacheck;
+  int *pflag;
+  const long long *cand;
+  int *candmap, *orig, *dec;
+  unsigned int *bits;
+  int *deplist;
+  long long *list;
+  double *outv;
+  double *ufv;
+  int cap, finalstep;
+  Scalars *sc;
+};
+__device__ __forceinline__ int listed(int n, int cap) { return n > cap ? cap : n; }
+
+__device__ __forceinline__ void checksol_map(const FixJob &J, int n, int a0, int step) {
+  for (int a = a0; a < n; a += step) {
+    const long long z = J.cand[a];
+    J.candmap[z] = a;
+    J.orig[a] = J.pflag[z];
   }
+}
+__global__ void checksol_map_kernel(FixJob J) {
+  checksol_map(J, listed(J.sc->ncand, J.cap), blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // packed per candidate: bits 0-7 gamma vote, 8-15 u vote, 16-23 fixed
@@ -906,15 +1039,11 @@ __global__ void checksol_map_kernel(const long long *__restrict__ cand, const in
 // all of them not (the votes only grow with more neighbours not failed):
 // those candidates go to deplist with their original flag as the first
 // guess; every other candidate's decision is final here.
-__global__ void checksol_prep_kernel(Dims d, const double *__restrict__ pv, const double *__restrict__ gammacheck,
-                                     const int *__restrict__ pflag, const long long *__restrict__ cand,
-                                     const int *__restrict__ candmap, const int *__restrict__ orig,
-                                     int *__restrict__ dec, unsigned int *__restrict__ bits,
-                                     int *__restrict__ deplist, int cap, Scalars *sc) {
-  int n = sc->ncand;
-  if (n > cap) n = cap;
-  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-    const long long z = cand[a];
+__device__ __forceinline__ void checksol_prep(const FixJob &J, int n, int a0, int step) {
+  const Dims &d = J.d;
+  const double *pv = J.pv, *gammacheck = J.gammacheck;
+  for (int a = a0; a < n; a += step) {
+    const long long z = J.cand[a];
     const double gc = gammacheck[z], uc = pv[(long long)UU * d.nz + z];
     long long nb[8];
     checksol_neighbours(d, z, nb);
@@ -927,55 +1056,52 @@ __global__ void checksol_prep_kernel(Dims d, const double *__restrict__ pv, cons
       if (q == 0) gate = pd >= 0.0;
       if ((fabs(pd) > 2.0) || (fabs(pd) < 1.0 / 2.0)) v0 |= 1u << q;
       if ((fabs(pd2) > 10.0) || (fabs(pd2) < 1.0 / 10.0)) v1 |= 1u << q;
-      if (nb[q] < z && candmap[nb[q]] >= 0) earlier |= 1u << q;
-      else if (pflag[nb[q]] <= UTOPRIMNOFAIL) okfix |= 1u << q;
+      if (nb[q] < z && J.candmap[nb[q]] >= 0) earlier |= 1u << q;
+      else if (J.pflag[nb[q]] <= UTOPRIMNOFAIL) okfix |= 1u << q;
     }
     // a not-failed neighbour 0 with a negative (or NaN) ratio gates all votes
     if (!gate) v0 = v1 = 0;
     const unsigned int bw = v0 | (v1 << 8) | (okfix << 16) | (earlier << 24);
-    bits[a] = bw;
+    J.bits[a] = bw;
     const int vlo = checksol_vote(bw, okfix);
     if (earlier != 0 && ((earlier & 1u) || vlo != checksol_vote(bw, okfix | earlier))) {
-      dec[a] = orig[a];
-      deplist[atomicAdd(&sc->ndep, 1)] = a;
+      J.dec[a] = J.orig[a];
+      J.deplist[atomicAdd(&J.sc->ndep, 1)] = a;
     } else {
-      dec[a] = vlo ? kChecksolCodes[vlo] : orig[a];
+      J.dec[a] = vlo ? kChecksolCodes[vlo] : J.orig[a];
     }
   }
 }
+__global__ void checksol_prep_kernel(FixJob J) {
+  checksol_prep(J, listed(J.sc->ncand, J.cap), blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
 
 // one block: sweeps over the dependent candidates until no decision changes
-__global__ void __launch_bounds__(1024) checksol_resolve_kernel(Dims d, const long long *__restrict__ cand,
-                                                                const int *__restrict__ candmap,
-                                                                const int *__restrict__ orig, int *dec,
-                                                                const unsigned int *__restrict__ bits,
-                                                                const int *__restrict__ deplist, int cap, Scalars *sc) {
-  int m = sc->ndep;
-  if (m > cap) m = cap;
-  if (m == 0) return;
+__device__ __forceinline__ void checksol_resolve(const FixJob &J, int m) {
+  const Dims &d = J.d;
   __shared__ int changed;
   // a chain can be at most m long; the sweep count is also capped so that a
   // pathological input ends with an error bit instead of a long kernel
   const int max_sweeps = m + 1 < 4096 ? m + 1 : 4096;
   for (int sweep = 0; sweep < max_sweeps; sweep++) {
-    if (sweep == max_sweeps - 1 && threadIdx.x == 0 && max_sweeps < m + 1) atomicOr(&sc->overflow, 4);
+    if (sweep == max_sweeps - 1 && threadIdx.x == 0 && max_sweeps < m + 1) atomicOr(&J.sc->overflow, 4);
     if (threadIdx.x == 0) changed = 0;
     __syncthreads();
     for (int e = threadIdx.x; e < m; e += blockDim.x) {
-      const int a = deplist[e];
-      const unsigned int b = bits[a];
+      const int a = J.deplist[e];
+      const unsigned int b = J.bits[a];
       unsigned int ok = (b >> 16) & 0xffu;
       const unsigned int earlier = b >> 24;
       long long nb[8];
-      checksol_neighbours(d, cand[a], nb);
+      checksol_neighbours(d, J.cand[a], nb);
 #pragma unroll
       for (int q = 0; q < 8; q++)
         if ((earlier >> q) & 1u)
-          if (dec[candmap[nb[q]]] <= UTOPRIMNOFAIL) ok |= 1u << q;
+          if (J.dec[J.candmap[nb[q]]] <= UTOPRIMNOFAIL) ok |= 1u << q;
       const int v = checksol_vote(b, ok);
-      const int nd = v ? kChecksolCodes[v] : orig[a];
-      if (nd != dec[a]) {
-        dec[a] = nd;
+      const int nd = v ? kChecksolCodes[v] : J.orig[a];
+      if (nd != J.dec[a]) {
+        J.dec[a] = nd;
         changed = 1;
       }
     }
@@ -985,16 +1111,28 @@ __global__ void __launch_bounds__(1024) checksol_resolve_kernel(Dims d, const lo
   }
 }
 
-// the decisions into pflag; candmap back to -1
-__global__ void checksol_apply_kernel(const long long *__restrict__ cand, const int *__restrict__ dec, int *pflag,
-                                      int *candmap, int cap, const Scalars *sc) {
-  int n = sc->ncand;
-  if (n > cap) n = cap;
-  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-    const long long z = cand[a];
-    pflag[z] = dec[a];
-    candmap[z] = -1;
+__global__ void __launch_bounds__(1024) checksol_resolve_kernel(FixJob J) {
+  const int m = listed(J.sc->ndep, J.cap);
+  if (m) checksol_resolve(J, m);
+}
+
+// the decisions into pflag; candmap back to -1; collect: the candidates that
+// are failed now onto the fixup list
+__device__ __forceinline__ void checksol_apply(const FixJob &J, int n, int a0, int step, bool collect) {
+  for (int a = a0; a < n; a += step) {
+    const long long z = J.cand[a];
+    const int f = J.dec[a];
+    J.pflag[z] = f;
+    J.candmap[z] = -1;
+    if (collect && f != 0) {
+      int slot = atomicAdd(&J.sc->nfixlist, 1);
+      if (slot < J.cap) J.list[slot] = z;
+      else atomicOr(&J.sc->overflow, 2);
+    }
   }
+}
+__global__ void checksol_apply_kernel(FixJob J) {
+  checksol_apply(J, listed(J.sc->ncand, J.cap), blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, false);
 }
 
 // fixup_utoprim (fixup.c:669-1470), part 1: list the active failed zones
@@ -1043,13 +1181,14 @@ __device__ __forceinline__ bool becomes_fixed(int f, int finalstep) {
 // tests neighbour pflags that earlier visits may already have reset to -1; a
 // neighbour's reset depends only on its own code, so "earlier active failed
 // neighbour that becomes fixed" counts as good here.
-__global__ void fixup_compute_kernel(Dims d, Params P, const double *__restrict__ pv, const int *__restrict__ pflag,
-                                     const double *__restrict__ G, const long long *__restrict__ list,
-                                     double *__restrict__ outv, int cap, int finalstep, Scalars *sc) {
-  int n = sc->nfixlist;
-  if (n > cap) n = cap;
-  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-  long long z = list[a];
+__device__ __forceinline__ void fixup_compute(const FixJob &J, const Params &P, int n, int a0, int step) {
+  const Dims &d = J.d;
+  const double *pv = J.pv, *__restrict__ G = J.G;
+  const int *pflag = J.pflag;
+  const int finalstep = J.finalstep;
+  Scalars *sc = J.sc;
+  for (int a = a0; a < n; a += step) {
+  long long z = J.list[a];
   int k = (int)(z % d.nt3) - d.g3;
   long long r = z / d.nt3;
   int j = (int)(r % d.nt2) - d.g2;
@@ -1135,18 +1274,23 @@ __global__ void fixup_compute_kernel(Dims d, Params P, const double *__restrict_
     if (limit_gamma(gamma, pr, m, &err) == -1) ffc_count(P, d.nz, z, CNT_LIMITGAMMAACT);
   }
 #pragma unroll
-  for (int v = 0; v < 5; v++) outv[(long long)a * 5 + v] = pr[v];
+  for (int v = 0; v < 5; v++) J.outv[(long long)a * 5 + v] = pr[v];
   if (err) atomicOr(&sc->err, err);
   }
 }
+__global__ void fixup_compute_kernel(FixJob J, Params P) {
+  fixup_compute(J, P, listed(J.sc->nfixlist, J.cap), blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
 
-__global__ void fixup_scatter_kernel(Dims d, Params P, double *pv, int *pflag, const long long *__restrict__ list,
-                                     const double *__restrict__ outv, int cap, int finalstep, Scalars *sc,
-                                     const double *__restrict__ G, double *__restrict__ ufv) {
-  int n = sc->nfixlist;
-  if (n > cap) n = cap;
-  for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-    long long z = list[a];
+__device__ __forceinline__ void fixup_scatter(const FixJob &J, const Params &P, int n, int a0, int step) {
+  const Dims &d = J.d;
+  double *pv = J.pv, *ufv = J.ufv;
+  const double *__restrict__ G = J.G, *outv = J.outv;
+  int *pflag = J.pflag;
+  const int finalstep = J.finalstep;
+  Scalars *sc = J.sc;
+  for (int a = a0; a < n; a += step) {
+    long long z = J.list[a];
     double pr0[NPR], pr[NPR];
     if (ufv && finalstep) load_prim(pv, d, z, pr0);
 #pragma unroll
@@ -1178,6 +1322,45 @@ __global__ void fixup_scatter_kernel(Dims d, Params P, double *pv, int *pflag, c
   }
 }
 
+__global__ void fixup_scatter_kernel(FixJob J, Params P) {
+  fixup_scatter(J, P, listed(J.sc->nfixlist, J.cap), blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+// checksolution from the candidates on and fixup_utoprim in one launch of one
+// cluster, whose hardware barrier stands where the kernels above end: seven
+// launches less a stage (with bound_kernel and the resets 246 -> 168 us a step
+// on 64x64).  Its 4096 threads do for the short lists of a flow; a larger
+// domain takes the kernels, which fill the GPU, and there seven launches are
+// under 1% of the step.  In a batch of strong 1D problems a good part of the
+// zones are candidates (128 problems, 77k zones: 88 ms to t = 0.2 with the
+// cluster, 79 with the kernels), so it has to be smaller by far.
+constexpr int FIX_CLUSTER = 8, FIX_THREADS = 512;
+constexpr long long kSmallDomain = 1LL << 18, kSmallBatch = 1LL << 13;
+__global__ void __cluster_dims__(FIX_CLUSTER, 1, 1) __launch_bounds__(FIX_THREADS)
+    fixup_small_kernel(FixJob J, Params P) {
+  auto cluster = cooperative_groups::this_cluster();
+  const int a0 = blockIdx.x * FIX_THREADS + threadIdx.x, step = FIX_CLUSTER * FIX_THREADS;
+  const int n = listed(*(volatile int *)&J.sc->ncand, J.cap);
+  if (n > 0) {
+    checksol_map(J, n, a0, step);
+    cluster.sync();
+    checksol_prep(J, n, a0, step);
+    cluster.sync();
+    const int m = listed(*(volatile int *)&J.sc->ndep, J.cap);
+    if (m > 0) {
+      if (blockIdx.x == 0) checksol_resolve(J, m);
+      cluster.sync();
+    }
+    checksol_apply(J, n, a0, step, true);
+    cluster.sync();
+  }
+  const int nf = listed(*(volatile int *)&J.sc->nfixlist, J.cap);
+  if (nf == 0) return;
+  fixup_compute(J, P, nf, a0, step);
+  cluster.sync();
+  fixup_scatter(J, P, nf, a0, step);
+}
+
 // B components of the fluxes after flux_ct (fluxct.c:724-781) on the faces
 // the update reads; used only to hand fluxes back through hgpu_fluxcalc (the
 // update kernel rebuilds them from the EMFs on the fly)
@@ -1202,69 +1385,6 @@ __global__ void bflux_kernel(Dims d, int dir, Box box, const double *__restrict_
     F[B2 * nz + z] = -0.5 * (e1[z] + e1[z + d.s2 * o2]);
     F[B3 * nz + z] = 0.;
   }
-}
-
-// ndt (advance.c:231) and the dt update of step_ch (step_ch.c:236-247)
-__global__ void finalize_kernel(Params P, Scalars *sc, int advance_time) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double n1 = __longlong_as_double((long long)sc->ndtbits[1]);
-  double n2 = __longlong_as_double((long long)sc->ndtbits[2]);
-  double n3 = __longlong_as_double((long long)sc->ndtbits[3]);
-  double ndt = P.defcon * 1. / (1. / n1 + 1. / n2 + 1. / n3);
-  if (advance_time && !sc->done) {
-    double dt = sc->dt;
-    sc->t += dt;
-    if (ndt > P.safe * dt) ndt = P.safe * dt;
-    dt = ndt;
-    if (sc->t + dt > P.tf) dt = P.tf - sc->t;
-    sc->dt = dt;
-    // the reference's main loop runs while t < tf (main.c:33)
-    sc->nsteps++;
-    if (!(sc->t < P.tf)) sc->done = 1;
-  }
-  // keep the last ndt where the host can read it
-  sc->ndtbits[0] = (unsigned long long)__double_as_longlong(ndt);
-}
-
-// batch: per-instance ndt combine and dt update (the same formulas per
-// instance; dims of size 1 contribute BIG as in the one-domain case)
-__global__ void finalize_batch_kernel(Params P, int advance_time) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= P.ninst) return;
-  Inst &I = P.inst[b];
-  double n1 = __longlong_as_double((long long)I.ndtbits);
-  double ndt = P.defcon * 1. / (1. / n1 + 1. / BIGNUM + 1. / BIGNUM);
-  if (advance_time) {
-    if (I.done) return;
-    double dt = I.dt;
-    I.t += dt;
-    I.nsteps++;
-    if (ndt > P.safe * dt) ndt = P.safe * dt;
-    dt = ndt;
-    if (I.t + dt > I.tf) dt = I.tf - I.t;
-    I.dt = dt;
-    if (!(I.t < I.tf)) I.done = 1;
-  } else {
-    I.dt = ndt;
-  }
-}
-
-__global__ void reset_batch_kernel(Params P) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= P.ninst) return;
-  P.inst[b].ndtbits = (unsigned long long)__double_as_longlong(BIGNUM);
-}
-
-__global__ void reset_stage_kernel(Scalars *sc) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  unsigned long long big = (unsigned long long)__double_as_longlong(BIGNUM);
-  sc->ndtbits[1] = big;
-  sc->ndtbits[2] = big;
-  sc->ndtbits[3] = big;
-  sc->nfail = 0;
-  sc->ncand = 0;
-  sc->ndep = 0;
-  sc->nfixlist = 0;
 }
 
 // reference AoS [zone][8] <-> device SoA [8][zone]
@@ -1340,11 +1460,14 @@ __global__ void pack_geometry_kernel(const double *__restrict__ raw, long long n
     for (int q = 0; q < 4; q++) m.gcon[q] = rcon[(ij * 8 + L) * 16 + q];
     m.g = rgdet[ij * 8 + L];
     derive_metric(m);
-    G[(long long)(s * GLOC + 34) * nij + ij] = m.alpha;
-    G[(long long)(s * GLOC + 35) * nij + ij] = m.ralpha;
+    if (s == G_CENT) {
+      G[(long long)G_LAPSE * nij + ij] = m.alpha;
+      G[(long long)(G_LAPSE + 1) * nij + ij] = m.ralpha;
+    } else {
+      const double v[6] = {m.alpha, m.ralpha, m.beta[0], m.beta[1], m.beta[2], m.rg};
 #pragma unroll
-    for (int q = 0; q < 3; q++) G[(long long)(s * GLOC + 36 + q) * nij + ij] = m.beta[q];
-    G[(long long)(s * GLOC + 39) * nij + ij] = m.rg;
+      for (int q = 0; q < 6; q++) G[(long long)(s * GLOC + g_derived(q)) * nij + ij] = v[q];
+    }
   }
   G[(long long)(G_CORN + 0) * nij + ij] = rgdet[ij * 8 + R_CORN1];
   G[(long long)(G_CORN + 1) * nij + ij] = rgdet[ij * 8 + R_CORN2];
@@ -1463,12 +1586,12 @@ bool w5_tile_accepted(int lb, int w) {
 // host context
 // ---------------------------------------------------------------------------
 enum KernelId {
-  K_RESET, K_FLUX1, K_FLUX2, K_FLUX3, K_EMF, K_UPDATE, K_BOUND_GHOST, K_BOUND_POLE, K_BOUND_PFLAG, K_CHECK_GAMMA,
+  K_RESET, K_FLUX, K_FLUX1, K_FLUX2, K_FLUX3, K_EMF, K_UPDATE, K_BOUND_GHOST, K_BOUND_PFLAG, K_CHECK_GAMMA,
   K_CHECK_RESOLVE, K_FIX_COLLECT, K_FIX_COMPUTE, K_FIX_SCATTER, K_FINALIZE, K_WENO5, K_W5STATE, K_INVERT, K_OTHER, K_NKERNELS
 };
 static const char *kKernelNames[K_NKERNELS] = {
-    "reset_stage",  "flux_x1",         "flux_x2",       "flux_x3",       "emf",           "update",
-    "bound_ghost",  "bound_pole",      "bound_pflag",   "checksol_gamma", "checksol_resolve", "fixup_collect",
+    "reset_stage",  "flux",           "flux_x1",         "flux_x2",       "flux_x3",       "emf",           "update",
+    "bound_ghost",  "bound_pflag",   "checksol_gamma", "checksol_resolve", "fixup_collect",
     "fixup_compute", "fixup_scatter",  "finalize",      "weno5",         "w5_state",      "invert",        "other"};
 
 struct ProfEvent {
@@ -1508,7 +1631,6 @@ struct hgpu_ctx {
   double *staging = nullptr;  // AoS staging for uploads/downloads
   double *pL = nullptr, *pR = nullptr;  // WENO5 face values
   double *w5pu = nullptr;               // WENO5: per-zone dP/P state pieces (2 planes)
-  double *w5ss = nullptr;               // WENO5: shock factor per direction (3 planes)
   unsigned char *bsqf = nullptr;        // FLAGBSQORHO | FLAGBSQOU << 2 per zone
   unsigned int *ffc = nullptr;          // failure/floor counters, NFFC planes
   double *bondi_tab = nullptr;          // Bondi-integral boundaries' coordinate data
@@ -1633,9 +1755,9 @@ void hgpu_destroy(hgpu_ctx *x) {
   if (x->graph) cudaGraphDestroy(x->graph);
   collect_profile(x);
   for (cudaEvent_t e : x->freelist) cudaEventDestroy(e);
-  void *ptrs[] = {x->p, x->pk, x->uf, x->ucum, x->F[1], x->F[2], x->F[3], x->E, x->G, x->pflag, x->gammacheck,
-                  x->cand, x->fixlist, x->cand_orig, x->cand_dec, x->cand_bits, x->cand_deplist, x->candmap, x->fixvals, x->sc, x->staging, x->istaging,
-                  x->pL, x->pR, x->w5pu, x->w5ss, x->bsqf, x->ffc, x->bondi_tab, x->cell_inst, x->inst, x->progress, x->pk1, x->ui};
+  void *ptrs[] = {x->p, x->pk, x->uf, x->ucum, x->F[1], x->F[2], x->F[3], x->E, x->G, x->pflag,
+                  x->candmap, x->sc, x->staging, x->istaging,
+                  x->pL, x->pR, x->w5pu, x->bsqf, x->ffc, x->bondi_tab, x->cell_inst, x->inst, x->progress, x->pk1, x->ui};
   for (void *q : ptrs)
     if (q) cudaFree(q);
   cudaStreamDestroy(x->stream);
@@ -1770,15 +1892,7 @@ int hgpu_create(const hgpu_config *cfg, hgpu_ctx **out) {
             cudaMalloc(&x->E, sizeof(double) * 3 * nz) == cudaSuccess &&
             cudaMalloc(&x->G, sizeof(double) * G_NCOMP * d.nij) == cudaSuccess &&
             cudaMalloc(&x->pflag, sizeof(int) * nz) == cudaSuccess &&
-            cudaMalloc(&x->gammacheck, sizeof(double) * nz) == cudaSuccess &&
-            cudaMalloc(&x->cand, sizeof(long long) * x->cap) == cudaSuccess &&
-            cudaMalloc(&x->fixlist, sizeof(long long) * x->cap) == cudaSuccess &&
-            cudaMalloc(&x->cand_orig, sizeof(int) * x->cap) == cudaSuccess &&
-            cudaMalloc(&x->cand_dec, sizeof(int) * x->cap) == cudaSuccess &&
-            cudaMalloc(&x->cand_bits, sizeof(unsigned int) * x->cap) == cudaSuccess &&
-            cudaMalloc(&x->cand_deplist, sizeof(int) * x->cap) == cudaSuccess &&
             cudaMalloc(&x->candmap, sizeof(int) * nz) == cudaSuccess &&
-            cudaMalloc(&x->fixvals, sizeof(double) * 5 * x->cap) == cudaSuccess &&
             cudaMalloc(&x->sc, sizeof(Scalars)) == cudaSuccess &&
             cudaMalloc(&x->bsqf, nz) == cudaSuccess && cudaMemset(x->bsqf, 0, nz) == cudaSuccess &&
             cudaMalloc(&x->ffc, sizeof(unsigned int) * NFFC * nz) == cudaSuccess &&
@@ -1790,14 +1904,24 @@ int hgpu_create(const hgpu_config *cfg, hgpu_ctx **out) {
          cudaMemset(x->ucum, 0, pb) == cudaSuccess;
   if (ok && cfg->lim == HGPU_LIM_WENO5)
     ok = cudaMalloc(&x->pL, pb) == cudaSuccess && cudaMalloc(&x->pR, pb) == cudaSuccess &&
-         cudaMalloc(&x->w5pu, sizeof(double) * 2 * nz) == cudaSuccess &&
-         cudaMalloc(&x->w5ss, sizeof(double) * 3 * nz) == cudaSuccess;
+         cudaMalloc(&x->w5pu, sizeof(double) * 2 * nz) == cudaSuccess;
   if (!ok) {
     hgpu_destroy(x);
     set_err("device allocation failed");
     return HGPU_E_NOMEM;
   }
   x->P.ffc = x->ffc;
+  // post_fixup's lists and scratch live in the flux planes, which are read
+  // for the last time by the conserved update before it and written by the
+  // next stage's fluxes (cap <= nz)
+  x->gammacheck = x->F[1];
+  x->fixvals = x->F[2];
+  x->cand = (long long *)(x->F[2] + 5 * nz);
+  x->fixlist = (long long *)(x->F[2] + 6 * nz);
+  x->cand_orig = (int *)(x->F[2] + 7 * nz);
+  x->cand_dec = x->cand_orig + nz;
+  x->cand_bits = (unsigned int *)(x->F[3]);
+  x->cand_deplist = (int *)(x->F[3]) + nz;
   cudaMemsetAsync(x->p, 0, pb, x->stream);
   cudaMemsetAsync(x->pk, 0, pb, x->stream);
   cudaMemsetAsync(x->uf, 0, pb, x->stream);
@@ -2009,7 +2133,7 @@ template <int DIR, typename TW, int BMB>
 static void launch_w5(hgpu_ctx *x, const double *pb) {
   const Dims &d = x->d;
   const W5Tile &tl = x->w5[DIR];
-  const TW *SS = (const TW *)x->w5ss;
+  const TW *SS = (const TW *)x->E;
   double *pL = x->pL, *pR = x->pR;
   ProfScope ps__(x, K_WENO5);
   const unsigned grid = grid_for((long long)tl.nlines * tl.nseg * NPR, W5_THREADS);
@@ -2023,13 +2147,14 @@ static void launch_w5(hgpu_ctx *x, const double *pb) {
   }
 }
 
-// the WENO5 state pieces and shock factors, for every direction
+// the WENO5 state pieces and shock factors, for every direction (the factors
+// in the EMFs' planes, which are formed after the last direction's fluxes)
 template <typename TW>
 static void launch_w5_state(hgpu_ctx *x, const double *pb) {
   LAUNCH(x, K_W5STATE, w5_state_kernel<TW>, grid_for(x->w5_state_box.size(), 128), 128, x->d, x->P, x->w5_state_box,
          pb, x->G, (TW *)x->w5pu);
   LAUNCH(x, K_W5STATE, w5_shock_kernel<TW>, grid_for(x->w5_shock_box.size(), 256), 256, x->d, x->w5_shock_box, pb,
-         (const TW *)x->w5pu, (TW *)x->w5ss);
+         (const TW *)x->w5pu, (TW *)x->E);
 }
 
 template <int DIR, typename TW, typename TF, int FMB, int BMB, int MIX = 0>
@@ -2038,26 +2163,44 @@ static void launch_dir(hgpu_ctx *x, const double *pb) {
   const Params &P = x->P;
   const int kid = (DIR == 1) ? K_FLUX1 : ((DIR == 2) ? K_FLUX2 : K_FLUX3);
   unsigned gf = grid_for(x->face_box[DIR].size(), 128);
-  if (P.lim == HGPU_LIM_WENO5) {
-    launch_w5<DIR, TW, BMB>(x, pb);
-    LAUNCH(x, kid, (flux_kernel<DIR, 1, TF, FMB, double, MIX>), gf, 128, d, P, x->face_box[DIR], pb, x->pL, x->pR, x->G,
-           x->F[DIR], x->sc);
-  } else if (P.lim == HGPU_LIM_PARA) {
-    LAUNCH(x, kid, (flux_kernel<DIR, 2, TF, FMB, TF>), gf, 128, d, P, x->face_box[DIR], pb, nullptr, nullptr, x->G,
-           x->F[DIR], x->sc);
-  } else {
-    LAUNCH(x, kid, (flux_kernel<DIR, 0, TF, FMB, TF>), gf, 128, d, P, x->face_box[DIR], pb, nullptr, nullptr, x->G,
-           x->F[DIR], x->sc);
-  }
+  launch_w5<DIR, TW, BMB>(x, pb);
+  LAUNCH(x, kid, (flux_kernel<DIR, 1, TF, FMB, double, MIX>), gf, 128, d, P, x->face_box[DIR], pb, x->pL, x->pR, x->G,
+         x->F[DIR], x->sc);
 }
 
+// bsq: also the b^2 flags of the step's state (pre_fixup of the last stage)
 template <typename TW, typename TF, int FMB, int BMB, int MIX = 0>
-static void launch_fluxes_t(hgpu_ctx *x, const double *pb) {
+static void launch_fluxes_t(hgpu_ctx *x, const double *pb, bool bsq) {
   const Dims &d = x->d;
-  if (x->P.lim == HGPU_LIM_WENO5) launch_w5_state<TW>(x, pb);
-  if (d.n1 > 1) launch_dir<1, TW, TF, FMB, BMB, MIX>(x, pb);
-  if (d.n2 > 1) launch_dir<2, TW, TF, FMB, BMB, MIX>(x, pb);
-  if (d.n3 > 1) launch_dir<3, TW, TF, FMB, BMB, MIX>(x, pb);
+  // (the FP32 Riemann kernels are those of the point reconstructions)
+  if constexpr (sizeof(TF) == 8) {
+    if (x->P.lim == HGPU_LIM_WENO5) {
+      if (bsq) LAUNCH(x, K_OTHER, bsqflags_kernel, grid_for(d.nz, 256), 256, d, x->p, x->G, x->bsqf, x->sc);
+      launch_w5_state<TW>(x, pb);
+      if (d.n1 > 1) launch_dir<1, TW, TF, FMB, BMB, MIX>(x, pb);
+      if (d.n2 > 1) launch_dir<2, TW, TF, FMB, BMB, MIX>(x, pb);
+      if (d.n3 > 1) launch_dir<3, TW, TF, FMB, BMB, MIX>(x, pb);
+      return;
+    }
+  }
+  FluxJob J;
+  const int n[4] = {0, d.n1, d.n2, d.n3};
+  J.first[0] = 0;
+  for (int q = 1; q <= 3; q++) {
+    J.box[q] = x->face_box[q];
+    J.F[q] = x->F[q];
+    J.first[q] = J.first[q - 1] + (n[q] > 1 ? grid_for(x->face_box[q].size(), 128) : 0);
+  }
+  J.first[4] = J.first[3] + (bsq ? grid_for(d.nz, 128) : 0);
+  J.pi = x->p;
+  J.bsqf = x->bsqf;
+  if (J.first[4] == 0) return;
+  if constexpr (MIX == 0) {
+    if (x->P.lim == HGPU_LIM_PARA)
+      LAUNCH(x, K_FLUX, (fluxes_kernel<2, TF, FMB>), J.first[4], 128, d, x->P, J, pb, x->G, x->sc);
+    else
+      LAUNCH(x, K_FLUX, (fluxes_kernel<0, TF, FMB>), J.first[4], 128, d, x->P, J, pb, x->G, x->sc);
+  }
 }
 // the WENO5 state pieces and one direction's reconstruction with the
 // context's precision and WENO5 variant (for timing tilings)
@@ -2082,41 +2225,49 @@ static void launch_w5_any(hgpu_ctx *x, const double *pb, bool state) {
 // whose reconstruction runs inside the Riemann kernel, that kernel runs in
 // FP32.  The fluxes are stored in FP64 and everything after them (flux-CT,
 // update, inversion) stays FP64.
-static void launch_fluxes(hgpu_ctx *x, const double *pb) {
+static void launch_fluxes(hgpu_ctx *x, const double *pb, bool bsq = false, int stage_clear = 0) {
   const Dims &d = x->d;
   const int fv = x->tune.flux, bv = x->tune.weno;
   if (x->cfg.precision == HGPU_PREC_MIXED) {
     constexpr int WMB = MinBlocks<float>::weno;
-    if (x->P.lim != HGPU_LIM_WENO5) launch_fluxes_t<float, float, MinBlocks<float>::flux, WMB>(x, pb);
-    else if (fv == 0) launch_fluxes_t<float, double, kFluxMB[0], WMB, 1>(x, pb);
-    else launch_fluxes_t<float, double, kFluxMB[1], WMB, 1>(x, pb);
+    if (x->P.lim != HGPU_LIM_WENO5) launch_fluxes_t<float, float, MinBlocks<float>::flux, WMB>(x, pb, bsq);
+    else if (fv == 0) launch_fluxes_t<float, double, kFluxMB[0], WMB, 1>(x, pb, bsq);
+    else launch_fluxes_t<float, double, kFluxMB[1], WMB, 1>(x, pb, bsq);
   } else {
-    if (fv == 0 && bv == 0) launch_fluxes_t<double, double, kFluxMB[0], kWenoMB[0]>(x, pb);
-    else if (fv == 0) launch_fluxes_t<double, double, kFluxMB[0], kWenoMB[1]>(x, pb);
-    else if (bv == 0) launch_fluxes_t<double, double, kFluxMB[1], kWenoMB[0]>(x, pb);
-    else launch_fluxes_t<double, double, kFluxMB[1], kWenoMB[1]>(x, pb);
+    if (fv == 0 && bv == 0) launch_fluxes_t<double, double, kFluxMB[0], kWenoMB[0]>(x, pb, bsq);
+    else if (fv == 0) launch_fluxes_t<double, double, kFluxMB[0], kWenoMB[1]>(x, pb, bsq);
+    else if (bv == 0) launch_fluxes_t<double, double, kFluxMB[1], kWenoMB[0]>(x, pb, bsq);
+    else launch_fluxes_t<double, double, kFluxMB[1], kWenoMB[1]>(x, pb, bsq);
   }
-  LAUNCH(x, K_EMF, emf_kernel, grid_for(x->emf_box.size(), 256), 256, d, x->emf_box, x->F[1], x->F[2], x->F[3], x->G,
-         x->E);
+  LAUNCH(x, K_EMF, emf_kernel, grid_for(x->emf_box.size(), 256), 256, d, x->P, x->emf_box, x->F[1], x->F[2], x->F[3],
+         x->G, x->E, x->sc, stage_clear);
 }
 
-static void launch_bound(hgpu_ctx *x, double *pv) {
+// flags: the failure flags' ghosts too; close: the kernel also ends the step
+static void launch_bound(hgpu_ctx *x, double *pv, bool flags = false, bool close = false) {
   const Dims &d = x->d;
+  int *pf = flags ? x->pflag : nullptr;
   if (x->P.cell_inst) {
-    LAUNCH(x, K_BOUND_GHOST, bound_batch_kernel, grid_for(d.nz, 128), 128, d, x->P, pv, (int *)nullptr);
+    LAUNCH(x, K_BOUND_GHOST, bound_batch_kernel, grid_for(d.nz, 128), 128, d, x->P, pv, pf, x->sc, (int)close);
     return;
   }
   if (x->P.bondi) {
     const long long nb = 2LL * d.g1 * d.n2 * d.n3;
     LAUNCH(x, K_BOUND_GHOST, bondi_bc_kernel, grid_for(nb, 128), 128, d, x->P, pv, x->G, x->sc);
   }
-  LAUNCH(x, K_BOUND_GHOST, bound_ghost_kernel, grid_for(d.nz, 128), 128, d, x->P, pv, x->G, x->sc);
-  if (d.n2 > 1) LAUNCH(x, K_BOUND_POLE, bound_pole_kernel, grid_for(2LL * d.n1 * d.n3, 128), 128, d, x->P, pv);
+  BoundJob J;
+  J.n[0] = (unsigned)(2 * d.g1) * d.nt2 * d.nt3;
+  J.n[1] = (unsigned)d.n1 * 2 * d.g2 * d.nt3;
+  J.n[2] = (unsigned)d.n1 * d.n2 * 2 * d.g3;
+  J.corners = d.n2 > 1 && (x->P.bc[2] == HGPU_BC_POLARAXIS || x->P.bc[3] == HGPU_BC_POLARAXIS);
+  J.n[3] = J.corners ? (unsigned)d.n1 * 2 * d.n3 : 0;
+  J.close = close;
+  const unsigned blocks = grid_for((long long)J.n[0] + J.n[1] + J.n[2] + J.n[3], 128);
+  LAUNCH(x, K_BOUND_GHOST, bound_kernel, blocks ? blocks : 1, 128, d, x->P, J, pv, x->G, x->sc, pf);
 }
 
-static void launch_reset(hgpu_ctx *x) {
-  LAUNCH(x, K_RESET, reset_stage_kernel, 1, 32, x->sc);
-  if (x->P.cell_inst) LAUNCH(x, K_RESET, reset_batch_kernel, grid_for(x->P.ninst, 128), 128, x->P);
+static void launch_reset(hgpu_ctx *x, bool call = false) {
+  LAUNCH(x, K_RESET, reset_stage_kernel, 1, 128, x->P, x->sc, (int)call);
 }
 
 static void launch_finalize(hgpu_ctx *x, int advance_time) {
@@ -2163,7 +2314,8 @@ static double *stage_output(hgpu_ctx *x, int timeorder) {
 // closing bound_prim.  A domain split along x3 exchanges the x3 ghost planes
 // of pf and pflag after the first half and of pf after the second, where the
 // reference's bound_prim and bound_pflag call bound_mpi / bound_mpi_int.
-static void launch_stage_advance(hgpu_ctx *x, int timeorder) {
+// folded: within a run of whole steps, where other kernels do the resets
+static void launch_stage_advance(hgpu_ctx *x, int timeorder, bool folded = false) {
   const Dims &d = x->d;
   const int norders = num_orders(x);
   const RKStage &S = rk_stage(x, timeorder);
@@ -2174,11 +2326,9 @@ static void launch_stage_advance(hgpu_ctx *x, int timeorder) {
   int finalstep = (timeorder == norders - 1);
   double CUf0 = S.cuf[0], CUf1 = S.cuf[1], CUf2 = S.cuf[2];
   double Cn0 = S.cun[0], Cn1 = S.cun[1], Cn2 = S.cun[2];
-  launch_reset(x);
+  if (!folded) launch_reset(x);
   // pre_fixup: only the last stage's flags survive the step
-  if (finalstep && !x->P.cell_inst)
-    LAUNCH(x, K_OTHER, bsqflags_kernel, grid_for(d.nz, 256), 256, d, pi, x->G, x->bsqf, x->sc);
-  launch_fluxes(x, pb);
+  launch_fluxes(x, pb, finalstep && !x->P.cell_inst, folded ? (finalstep ? 1 : 2) : 0);
   const int fv = (x->cfg.doenoflux == HGPU_ENOFINITEVOLUME);
   double *ufv = (fv && finalstep) ? x->ucum : nullptr;
   // ulast and ucum enter a stage only where an earlier one left them other
@@ -2206,51 +2356,74 @@ static void launch_stage_advance(hgpu_ctx *x, int timeorder) {
     LAUNCH(x, K_INVERT, invert, gi, 128, d, x->P, x->active_box, pb, pf, x->uf, x->ucum, x->G, x->pflag, x->sc, finalstep,
            ufv);
   }
-  launch_bound(x, pf);
-  // post_fixup (fixup.c:37-96)
-  if (x->P.cell_inst)
-    LAUNCH(x, K_BOUND_PFLAG, bound_batch_kernel, grid_for(d.nz, 256), 256, d, x->P, (double *)nullptr, x->pflag);
-  else
-    LAUNCH(x, K_BOUND_PFLAG, bound_pflag_kernel, grid_for(d.nz, 256), 256, d, x->P, x->pflag, x->sc);
+  // bound_prim, and bound_pflag, which opens post_fixup (fixup.c:37-96)
+  launch_bound(x, pf, true);
 }
 
 // fixup_checksolution and fixup_utoprim on pf with the context's flags
 static void launch_checksol_fixup(hgpu_ctx *x, double *pf, int finalstep) {
   const Dims &d = x->d;
-  double *ufv = (x->cfg.doenoflux == HGPU_ENOFINITEVOLUME && finalstep) ? x->ucum : nullptr;
+  FixJob J;
+  J.d = d;
+  J.pv = pf;
+  J.G = x->G;
+  J.gammacheck = x->gammacheck;
+  J.pflag = x->pflag;
+  J.cand = x->cand;
+  J.candmap = x->candmap;
+  J.orig = x->cand_orig;
+  J.dec = x->cand_dec;
+  J.bits = x->cand_bits;
+  J.deplist = x->cand_deplist;
+  J.list = x->fixlist;
+  J.outv = x->fixvals;
+  J.ufv = (x->cfg.doenoflux == HGPU_ENOFINITEVOLUME && finalstep) ? x->ucum : nullptr;
+  J.cap = x->cap;
+  J.finalstep = finalstep;
+  J.sc = x->sc;
+  const bool small = (long long)d.n1 * d.n2 * d.n3 <= (x->P.cell_inst ? kSmallBatch : kSmallDomain);
   LAUNCH(x, K_CHECK_GAMMA, checksol_gamma_kernel, grid_for(x->dq_box.size(), 128), 128, d, x->P, x->dq_box, pf, x->G,
-         x->gammacheck, x->cand, x->cap, x->sc);
+         x->gammacheck, x->cand, x->cap, x->sc, x->pflag, small ? x->fixlist : nullptr);
+  if (small) {
+    LAUNCH(x, K_CHECK_RESOLVE, fixup_small_kernel, FIX_CLUSTER, FIX_THREADS, J, x->P);
+    return;
+  }
   // grid-stride over the device-side candidate count; idle blocks exit at once
   int cgrid = (int)grid_for(x->cap, 256);
   if (cgrid > 592) cgrid = 592;
-  LAUNCH(x, K_CHECK_RESOLVE, checksol_map_kernel, cgrid, 256, x->cand, x->pflag, x->candmap, x->cand_orig, x->cap,
-         x->sc);
-  LAUNCH(x, K_CHECK_RESOLVE, checksol_prep_kernel, cgrid, 256, d, pf, x->gammacheck, x->pflag, x->cand, x->candmap,
-         x->cand_orig, x->cand_dec, x->cand_bits, x->cand_deplist, x->cap, x->sc);
-  LAUNCH(x, K_CHECK_RESOLVE, checksol_resolve_kernel, 1, 1024, d, x->cand, x->candmap, x->cand_orig, x->cand_dec,
-         x->cand_bits, x->cand_deplist, x->cap, x->sc);
-  LAUNCH(x, K_CHECK_RESOLVE, checksol_apply_kernel, cgrid, 256, x->cand, x->cand_dec, x->pflag, x->candmap, x->cap,
-         x->sc);
+  LAUNCH(x, K_CHECK_RESOLVE, checksol_map_kernel, cgrid, 256, J);
+  LAUNCH(x, K_CHECK_RESOLVE, checksol_prep_kernel, cgrid, 256, J);
+  LAUNCH(x, K_CHECK_RESOLVE, checksol_resolve_kernel, 1, 1024, J);
+  LAUNCH(x, K_CHECK_RESOLVE, checksol_apply_kernel, cgrid, 256, J);
   LAUNCH(x, K_FIX_COLLECT, fixup_collect_kernel, grid_for(x->active_box.size(), 256), 256, d, x->P, x->active_box, x->pflag,
          x->fixlist, x->cap, x->sc);
   // grid-stride over the device-side list length; idle blocks exit at once
   int fixgrid = (int)grid_for(x->cap, 128);
   if (fixgrid > 296) fixgrid = 296;
-  LAUNCH(x, K_FIX_COMPUTE, fixup_compute_kernel, fixgrid, 128, d, x->P, pf, x->pflag, x->G, x->fixlist, x->fixvals,
-         x->cap, finalstep, x->sc);
-  LAUNCH(x, K_FIX_SCATTER, fixup_scatter_kernel, fixgrid, 128, d, x->P, pf, x->pflag, x->fixlist, x->fixvals, x->cap,
-         finalstep, x->sc, x->G, ufv);
+  LAUNCH(x, K_FIX_COMPUTE, fixup_compute_kernel, fixgrid, 128, J, x->P);
+  LAUNCH(x, K_FIX_SCATTER, fixup_scatter_kernel, fixgrid, 128, J, x->P);
 }
 
-static void launch_stage_fixup(hgpu_ctx *x, int timeorder) {
+static void launch_stage_fixup(hgpu_ctx *x, int timeorder, bool close = false) {
   double *pf = stage_output(x, timeorder);
   launch_checksol_fixup(x, pf, timeorder == num_orders(x) - 1);
-  launch_bound(x, pf);
+  launch_bound(x, pf, false, close);
 }
 
 static void launch_stage(hgpu_ctx *x, int timeorder) {
   launch_stage_advance(x, timeorder);
   launch_stage_fixup(x, timeorder);
+}
+
+// One time step within a run of steps: the resets and the dt update ride on
+// kernels that are there anyway (before the first step of a run,
+// launch_reset(x, true); after the last the dt minima are cleared).
+static void launch_step(hgpu_ctx *x) {
+  const int norders = num_orders(x);
+  for (int o = 0; o < norders; o++) {
+    launch_stage_advance(x, o, true);
+    launch_stage_fixup(x, o, o == norders - 1);
+  }
 }
 
 static int read_stats(hgpu_ctx *x, hgpu_stats *st) {
@@ -2301,11 +2474,8 @@ static int boundaries_ready(const hgpu_ctx *x) {
 int hgpu_step_ch(hgpu_ctx *x, int nsteps, hgpu_stats *stats) {
   if (!x || nsteps < 0) return HGPU_E_INVALID;
   if (boundaries_ready(x)) return HGPU_E_INVALID;
-  clear_counters(x);
-  for (int n = 0; n < nsteps; n++) {
-    for (int o = 0; o < num_orders(x); o++) launch_stage(x, o);
-    launch_finalize(x, 1);
-  }
+  launch_reset(x, true);
+  for (int n = 0; n < nsteps; n++) launch_step(x);
   CUDA_TRY(cudaGetLastError());
   if (stats) return read_stats(x, stats);
   return HGPU_OK;
@@ -2374,8 +2544,7 @@ int hgpu_step_graph(hgpu_ctx *x, int nsteps, hgpu_stats *stats) {
     CUDA_TRY(cudaStreamSynchronize(x->stream));
     CUDA_TRY(cudaStreamBeginCapture(x->stream, cudaStreamCaptureModeThreadLocal));
     long long l0 = x->launches;
-    for (int o = 0; o < num_orders(x); o++) launch_stage(x, o);
-    launch_finalize(x, 1);
+    launch_step(x);
     x->launches_per_step = x->launches - l0;
     x->launches = l0;
     cudaGraph_t g = nullptr;
@@ -2392,7 +2561,7 @@ int hgpu_step_graph(hgpu_ctx *x, int nsteps, hgpu_stats *stats) {
     }
     x->graph = g;
   }
-  clear_counters(x);
+  launch_reset(x, true);
   for (int n = 0; n < nsteps; n++) {
     CUDA_TRY(cudaGraphLaunch(x->graph_exec, x->stream));
     x->launches += x->launches_per_step;
@@ -2422,6 +2591,8 @@ int hgpu_advance_stage(hgpu_ctx *x, int timeorder, double *ndt, hgpu_stats *stat
 int hgpu_fluxcalc(hgpu_ctx *x, int which, double *F1, double *F2, double *F3, double *ndt1, double *ndt2,
                   double *ndt3) {
   if (!x || (which != 0 && which != 1)) return HGPU_E_INVALID;
+  // zero wherever no face flux is written (post_fixup's lists pass through these planes)
+  for (int q = 1; q <= 3; q++) CUDA_TRY(cudaMemsetAsync(x->F[q], 0, sizeof(double) * NPR * x->d.nz, x->stream));
   launch_reset(x);
   launch_fluxes(x, which ? x->pk : x->p);
   CUDA_TRY(cudaGetLastError());
@@ -2694,12 +2865,9 @@ int hgpu_step_ch_timed(hgpu_ctx *x, int nsteps, float *ms, hgpu_stats *stats) {
   cudaEvent_t a, b;
   CUDA_TRY(cudaEventCreate(&a));
   CUDA_TRY(cudaEventCreate(&b));
-  clear_counters(x);
+  launch_reset(x, true);
   CUDA_TRY(cudaEventRecord(a, x->stream));
-  for (int n = 0; n < nsteps; n++) {
-    for (int o = 0; o < num_orders(x); o++) launch_stage(x, o);
-    launch_finalize(x, 1);
-  }
+  for (int n = 0; n < nsteps; n++) launch_step(x);
   CUDA_TRY(cudaEventRecord(b, x->stream));
   CUDA_TRY(cudaEventSynchronize(b));
   float t = 0.f;
@@ -2751,16 +2919,16 @@ int hgpu_autotune(hgpu_ctx *x, hgpu_tuning *out) {
     if (ib) cudaMemcpyAsync(x->inst, si, ib, cudaMemcpyDeviceToDevice, x->stream);
   };
   auto one_step = [&]() {
-    clear_counters(x);
-    for (int o = 0; o < num_orders(x); o++) launch_stage(x, o);
-    launch_finalize(x, 1);
+    launch_reset(x, true);
+    launch_step(x);
   };
   const bool fp64 = x->cfg.precision == HGPU_PREC_FP64;
   int *knob[4] = {&x->tune.flux, &x->tune.weno, &x->tune.conserve, &x->tune.invert};
   // the mixed-precision path runs the FP64 Riemann kernel after a WENO5
   // reconstruction (its FP32 kernels have fixed variants)
   const bool applies[4] = {fp64 || x->P.lim == HGPU_LIM_WENO5, fp64 && x->P.lim == HGPU_LIM_WENO5, true, true};
-  const int kids[4][3] = {{K_FLUX1, K_FLUX2, K_FLUX3}, {K_WENO5, -1, -1}, {K_UPDATE, -1, -1}, {K_INVERT, -1, -1}};
+  const int kids[4][4] = {{K_FLUX, K_FLUX1, K_FLUX2, K_FLUX3}, {K_WENO5, -1, -1, -1}, {K_UPDATE, -1, -1, -1},
+                          {K_INVERT, -1, -1, -1}};
   float ms[4][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
   int rc = HGPU_OK;
   x->profiling = true;
@@ -2777,7 +2945,7 @@ int hgpu_autotune(hgpu_ctx *x, hgpu_tuning *out) {
         }
         collect_profile(x);
         double t = 0.0;
-        for (int q = 0; q < 3; q++)
+        for (int q = 0; q < 4; q++)
           if (kids[f][q] >= 0) t += x->kms[kids[f][q]];
         if (rep == 1) ms[f][v] = (float)t;
         for (int k = 0; k < K_NKERNELS; k++) {
@@ -3151,8 +3319,6 @@ extern "C" size_t hgpu_context_bytes(const hgpu_config *c) {
   size_t nt1 = tot(c->n1), nt2 = tot(c->n2), nt3 = tot(c->n3);
   size_t nz = nt1 * nt2 * nt3;
   size_t nij = (nt1 + (c->n1 > 1)) * (nt2 + (c->n2 > 1));
-  size_t zones = (size_t)c->n1 * c->n2 * c->n3;
-  size_t cap = zones < (1u << 22) ? zones : (1u << 22);
   size_t plane = sizeof(double) * NPR * nz;
   size_t b = 7 * plane                       // p, pk, uf, ucum, F1..F3
              + sizeof(double) * 3 * nz        // corner EMFs
@@ -3160,10 +3326,8 @@ extern "C" size_t hgpu_context_bytes(const hgpu_config *c) {
              + sizeof(int) * 2 * nz           // pflag, candidate map
              + (size_t)nz                     // b^2 flags
              + sizeof(unsigned int) * NFFC * nz  // failure/floor counters
-             + sizeof(double) * nz            // gamma check
-             + cap * (2 * sizeof(long long) + 4 * sizeof(int) + 5 * sizeof(double))
              + plane;                         // staging for uploads and downloads
-  if (c->lim == HGPU_LIM_WENO5) b += 2 * plane + sizeof(double) * 5 * nz;  // pL, pR, dP/P state pieces, shock factors
+  if (c->lim == HGPU_LIM_WENO5) b += 2 * plane + sizeof(double) * 2 * nz;  // pL, pR, dP/P state pieces
   if (c->timeorder >= 3) b += plane;                     // pk1
   if (c->doenoflux == HGPU_ENOFINITEVOLUME) b += plane;  // ui
   if (c->bc[0] == HGPU_BC_BONDIMDOTOUTFLOW || c->bc[1] == HGPU_BC_BONDIINTOUTFLOW)
