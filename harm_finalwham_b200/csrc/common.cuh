@@ -282,6 +282,7 @@ template <> struct MinBlocks<float> {
 constexpr int kFluxMB[2] = {HG_MINB_FLUX, HG_MINB_FLUX - 1};
 constexpr int kWenoMB[2] = {HG_MINB_WENO, HG_MINB_WENO - 1};
 constexpr int kConserveMB[2] = {HG_MINB_UPDATE, HG_MINB_UPDATE + 1};
+// (1 and 2 name the inversion's variants for hgpu_tuning; they ask for 4 and 3 blocks)
 constexpr int kInvertMB[2] = {HG_MINB_INVERT, 2};
 
 template <int DIR>
@@ -315,14 +316,17 @@ __device__ __forceinline__ long long dir_stride(const Dims &d) {
 // from each cell's own value and writes FP64 face values (the cell's value
 // plus the FP32 offset), which the FP64 Riemann kernel reads.
 //
-// Bound by instruction issue, FP64 first (FP64 pipe 51-59% active, 250 FP64
+// Bound by instruction issue, FP64 first (FP64 pipe 65-67% active, 240 FP64
 // instructions a cell and primitive).  The form before this one staged tiles
 // of a line in shared memory, one stage at a time between barriers, and held
 // 1.7 other instructions (addresses, shared memory, selects, the branches of
-// its divisions) to an FP64 one: 2.63 -> 1.49 ms a launch on 256x128x128.
+// its divisions) to an FP64 one: 2.63 -> 1.12 ms a launch on 256x128x128.
+// The loop stays rolled: unrolled by 2 or 4, to spare the moves of its windows
+// (a fifth of its instructions), it ran 15% and 52% longer.
 // ---------------------------------------------------------------------------
 constexpr int W5_THREADS = 128;
 constexpr int W5_CHUNK = 8;               // FS: line cells staged per warp and turn
+constexpr int W5_RING = 4;                // not FS: cells of a thread's ring
 constexpr int W5_PITCH = W5_CHUNK + 1;    // odd, so that lanes on different rows meet different banks
 
 struct W5Tile {
@@ -402,16 +406,33 @@ __device__ __forceinline__ long long w5_line(const Dims &d, const Box &b, int li
   return zix(d, i, j, k);
 }
 
-// FS (a line's cells are contiguous): a warp's 32 rows (segments of lines) lie
-// far apart, so it brings W5_CHUNK cells of each at a time through shared
-// memory, a row's cells by neighbouring lanes, and the face values back the
-// same way; otherwise neighbouring lanes are neighbouring lines and read and
-// write the planes directly.
+// one value from global to shared memory, asynchronously
+template <typename V>
+__device__ __forceinline__ void copy_async(double *to, const V *from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from),
+               "n"(sizeof(V)));
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;"); }
+template <int PENDING>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
+// Lines next to one another in memory (not FS): neighbouring lanes are
+// neighbouring lines; each thread keeps the next three cells of its line and
+// of the shock factor on their way into a ring of its own in shared memory
+// (loaded into registers a step ahead, they were waited for: 2 of 6.6 stall
+// cycles an instruction).  FS (a line's cells are contiguous): a warp's 32
+// rows (segments of lines) lie far apart, so it brings W5_CHUNK cells of each
+// at a time, a row's cells by neighbouring lanes, the next chunk while one is
+// worked on, and the face values go back the same way through the slots of
+// the cells they came from.
 template <int DIR, bool FS, typename T, int MB = MinBlocks<T>::weno>
 __global__ void __launch_bounds__(W5_THREADS, MB) weno5_kernel(Dims d, W5Tile tl, const double *__restrict__ pb,
                                                                const T *__restrict__ SS, double *__restrict__ pL,
                                                                double *__restrict__ pR) {
-  __shared__ double stage[FS ? W5_THREADS / 32 : 1][FS ? 4 : 1][FS ? 32 * W5_PITCH : 1];
+  // FS: [warp][buffer][Y, S][row][cell]; otherwise [slot][Y, S][thread]
+  __shared__ double stage[FS ? W5_THREADS / 32 * 4 * 32 * W5_PITCH : W5_RING * 2 * W5_THREADS];
   const unsigned lane = threadIdx.x & 31;
   const unsigned rows = (unsigned)tl.nlines * tl.nseg;
   unsigned t = blockIdx.x * W5_THREADS + threadIdx.x;
@@ -430,10 +451,28 @@ __global__ void __launch_bounds__(W5_THREADS, MB) weno5_kernel(Dims d, W5Tile tl
   const double *src = pb + zv;
   const T *ssrc = SS + (long long)(DIR - 1) * d.nz + zc;
   const int slast = nv + 4;  // the last cell this thread's output reads
-  double *Ys = stage[FS ? threadIdx.x >> 5 : 0][0];
-  double *Ss = stage[FS ? threadIdx.x >> 5 : 0][FS ? 1 : 0];
-  double *Ls = stage[FS ? threadIdx.x >> 5 : 0][FS ? 2 : 0];
-  double *Rs = stage[FS ? threadIdx.x >> 5 : 0][FS ? 3 : 0];
+  double *buf = FS ? stage + (threadIdx.x >> 5) * 4 * 32 * W5_PITCH : stage + threadIdx.x;
+  // FS: cells s .. s+CHUNK-1 of the warp's rows, and of the shock factor s-5 ..
+  auto bring_chunk = [&](int s, int which) {
+    double *Yb = buf + which * 2 * 32 * W5_PITCH, *Sb = Yb + 32 * W5_PITCH;
+#pragma unroll
+    for (int it = 0; it < W5_CHUNK; it++) {
+      const int row = it * (32 / W5_CHUNK) + (int)(lane / W5_CHUNK), c = (int)(lane % W5_CHUNK);
+      const double *rs = (const double *)__shfl_sync(0xffffffffu, (unsigned long long)src, row);
+      const T *rss = (const T *)__shfl_sync(0xffffffffu, (unsigned long long)ssrc, row);
+      const int last = __shfl_sync(0xffffffffu, slast, row);
+      copy_async(Yb + row * W5_PITCH + c, rs + min(s + c, last));
+      copy_async(Sb + row * W5_PITCH + c, rss + max(min(s + c - 5, last - 5), 0));
+    }
+    copy_commit();
+  };
+  // otherwise: cell s of this thread's line
+  auto bring = [&](int s) {
+    double *slot = buf + ((s + 5) % W5_RING) * 2 * W5_THREADS;
+    copy_async(slot, src + (long long)min(s, slast) * o);
+    copy_async(slot + W5_THREADS, ssrc + (long long)max(min(s - 5, nv - 1), 0) * o);
+    copy_commit();
+  };
 
   double y[8];  // the line at cells s-7 .. s
   T w0[5], w1[4], w2[4];  // weights of cells s-6 .. s-2 (w0), s-5 .. s-2
@@ -445,36 +484,35 @@ __global__ void __launch_bounds__(W5_THREADS, MB) weno5_kernel(Dims d, W5Tile tl
   for (int q = 0; q < 5; q++) w0[q] = T(0.);
 #pragma unroll
   for (int q = 0; q < 4; q++) w1[q] = w2[q] = T(0.);
-  double ynext = 0.;
-  if (!FS) ynext = __ldg(src + (long long)min(-5, slast) * o);
-
-  for (int s = -5; s < tl.lb + 5; s++) {
-    const int slot = (s + 5) % W5_CHUNK;
-    if (FS && slot == 0) {
-      // cells s .. s+CHUNK-1 of the line and s-5 .. of the shock factor
-      __syncwarp();
+  if (FS) {
+    bring_chunk(-5, 0);
+  } else {
 #pragma unroll
-      for (int it = 0; it < W5_CHUNK; it++) {
-        const int row = it * (32 / W5_CHUNK) + (int)(lane / W5_CHUNK), c = (int)(lane % W5_CHUNK);
-        const double *rs = (const double *)__shfl_sync(0xffffffffu, (unsigned long long)src, row);
-        const T *rss = (const T *)__shfl_sync(0xffffffffu, (unsigned long long)ssrc, row);
-        const int last = __shfl_sync(0xffffffffu, slast, row);
-        Ys[row * W5_PITCH + c] = __ldg(rs + min(s + c, last));
-        if (s + c >= 5) Ss[row * W5_PITCH + c] = (double)__ldg(rss + min(s + c - 5, max(last - 5, 0)));
+    for (int s = 0; s < W5_RING - 1; s++) bring(s - 5);
+  }
+  // (FS: whole chunks, whose face values leave with their last step)
+  const int send = FS ? (tl.lb + 10 + W5_CHUNK - 1) / W5_CHUNK * W5_CHUNK - 5 : tl.lb + 5;
+  for (int s = -5; s < send; s++) {
+    const int slot = (s + 5) % W5_CHUNK, half = ((s + 5) / W5_CHUNK) & 1;
+    double *ys = FS ? buf + half * 2 * 32 * W5_PITCH + lane * W5_PITCH + slot
+                    : buf + ((s + 5) % W5_RING) * 2 * W5_THREADS;
+    double *sst = ys + (FS ? 32 * W5_PITCH : W5_THREADS);
+    if (FS) {
+      if (slot == 0) {
+        // this chunk has come; the other buffer's face values are out
+        copy_wait<0>();
+        __syncwarp();
+        if (s + W5_CHUNK < send) bring_chunk(s + W5_CHUNK, half ^ 1);
       }
-      __syncwarp();
+    } else {
+      copy_wait<W5_RING - 2>();
     }
 #pragma unroll
     for (int q = 0; q < 7; q++) y[q] = y[q + 1];
-    T ss = T(0.);
-    if (FS) {
-      y[7] = Ys[lane * W5_PITCH + slot];
-      if (s >= 5) ss = (T)Ss[lane * W5_PITCH + slot];
-    } else {
-      y[7] = ynext;
-      ynext = __ldg(src + (long long)min(s + 1, slast) * o);
-      if (s >= 5) ss = __ldg(ssrc + (long long)min(s - 5, max(nv - 1, 0)) * o);
-    }
+    y[7] = *ys;
+    const T ss = *(const T *)sst;
+    // (into the slot read a step ago)
+    if (!FS) bring(s + W5_RING - 1);
     // the stencil of the cell at y[q]: values for FP64; in FP32 offsets from
     // the cell's own value, and the values for magnitudes
     auto stencil = [&](int q, T *yd, T *yn) {
@@ -488,7 +526,9 @@ __global__ void __launch_bounds__(W5_THREADS, MB) weno5_kernel(Dims d, W5Tile tl
         }
       }
     };
-    if (s >= -1) {
+    // (the steps that only fill the last chunk compute nothing)
+    const bool live = !FS || s < tl.lb + 5;
+    if (s >= -1 && live) {
       T ya[5], yb[5], w[3];
       stencil(5, ya, yb);
       const int code = w5::code_of(ya + 2, yb + 2);
@@ -505,12 +545,12 @@ __global__ void __launch_bounds__(W5_THREADS, MB) weno5_kernel(Dims d, W5Tile tl
       w1[3] = w[1];
       w2[3] = w[2];
     }
-    if (s >= 3) {
+    if (s >= 3 && live) {
       Rm = Rc;
       Rc = Rp;
       Rp = w5::lower_fraction((int)(codes >> 4) & 3, w0[2], w2[1], w0[0], w2[3]);
     }
-    if (s >= 5) {
+    if (s >= 5 && live) {
       T lof = Rc;
       lof = w5::wmax(lof, ss * Rp);
       lof = w5::wmax(lof, ss * Rm);
@@ -521,29 +561,31 @@ __global__ void __launch_bounds__(W5_THREADS, MB) weno5_kernel(Dims d, W5Tile tl
       const double fl = sizeof(T) == 4 ? y[2] + (double)yl : (double)yl;
       const double fr = sizeof(T) == 4 ? y[2] + (double)yr : (double)yr;
       if (FS) {
-        Ls[lane * W5_PITCH + slot] = fl;
-        Rs[lane * W5_PITCH + slot] = fr;
+        *ys = fl;
+        *sst = fr;
       } else if (s - 5 < nv) {
         pL[zv + (long long)(s - 5) * o] = fl;
         pR[zv + (long long)(s - 5) * o] = fr;
       }
     }
-    if (FS && (slot == W5_CHUNK - 1 || s == tl.lb + 4)) {
-      // the face values of this turn's output cells, s-5-slot ..
+    if (FS && slot == W5_CHUNK - 1) {
+      // the face values of this chunk's output cells, s-5-slot ..
       __syncwarp();
+      const double *Lb = buf + half * 2 * 32 * W5_PITCH, *Rb = Lb + 32 * W5_PITCH;
 #pragma unroll
       for (int it = 0; it < W5_CHUNK; it++) {
         const int row = it * (32 / W5_CHUNK) + (int)(lane / W5_CHUNK), c = (int)(lane % W5_CHUNK);
         const long long rz = __shfl_sync(0xffffffffu, zv, row);
         const int rnv = __shfl_sync(0xffffffffu, nv, row);
         const int cell = s - 5 - slot + c;
-        if (c <= slot && cell >= 0 && cell < rnv) {
-          pL[rz + cell] = Ls[row * W5_PITCH + c];
-          pR[rz + cell] = Rs[row * W5_PITCH + c];
+        if (cell >= 0 && cell < rnv) {
+          pL[rz + cell] = Lb[row * W5_PITCH + c];
+          pR[rz + cell] = Rb[row * W5_PITCH + c];
         }
       }
     }
   }
+  copy_wait<0>();
 }
 
 // ---------------------------------------------------------------------------

@@ -30,6 +30,7 @@
 //   finalize_kernel   ndt combine (advance.c:231) and dt update (step_ch.c:236-247)
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -421,7 +422,7 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
 // ms a launch on 256x128x128.  With it, 3 blocks spill 140 B in the branch
 // of the floored zones: 83 -> 58 us a launch on 128x64x32 (RK4, Jon).
 template <int UV, int MB, bool FV>
-__global__ void __launch_bounds__(128, FV ? 3 : MB) invert_kernel(Dims d, Params P, Box box, const double *pb,
+__global__ void __launch_bounds__(128, FV || UV == 8 || MB == 2 ? 3 : 4) invert_kernel(Dims d, Params P, Box box, const double *pb,
                                                                      double *pf, const double *__restrict__ uf,
                                                                      const double *__restrict__ ucum,
                                                                      const double *__restrict__ G,
@@ -1516,17 +1517,22 @@ __global__ void utoprim_batch_kernel(const double *__restrict__ U, const double 
 
 inline unsigned grid_for(long long n, int block) { return (unsigned)((n + block - 1) / block); }
 
-// Time of a WENO5 pass with segments of lb cells, in steps of one thread
-// along its line.  A thread takes lb + 10 steps, of which lb do the whole
-// work and the first ten about as much as five.  While an SM holds one block
-// its four schedulers wait on the results of a warp each; further blocks fill
-// them and cost about 0.6 of a block's time apiece (up to four resident, the
-// rest in turn).
-double w5_cost(int nout, long long nlines, int lb) {
+// Time of a WENO5 pass with segments of lb cells, in steps of one thread along
+// its line.  A thread takes lb + 10 steps (staged lines: whole chunks), of
+// which the first ten cost about five.  Up to four blocks an SM, all resident,
+// a step takes the latency of its arithmetic however many there are; beyond
+// that blocks come in turn, at 0.71 of that time per four.  Measured on the
+// B200, us a step of two stages, x1 of 128x64x32 in 1, 2, 4, 6, 10, 24 segments:
+// 1040, 856, 777, 758, 748, 772 (modelled 135, 70, 38, 35, 36, 44); x1 of
+// 256x128x64 in 1, 3, 6, 16: 3958, 3727, 3688, 3799 (263, 202, 199, 214).
+// Near ties go to the longer segments, which repeat fewer cells.
+double w5_cost(int nout, long long nlines, int lb, bool staged) {
   const long long nseg = (nout + lb - 1) / lb;
   const long long blocks = (nlines * nseg * NPR + W5_THREADS - 1) / W5_THREADS;
-  const double per_sm = (double)((blocks + 147) / 148);
-  return (lb + 5.0) * (per_sm <= 1.0 ? 1.0 : 0.4 + 0.6 * per_sm);
+  const double per_sm = (double)blocks / 148.0;
+  const int steps = staged ? (lb + 10 + W5_CHUNK - 1) / W5_CHUNK * W5_CHUNK - 5 : lb + 5;
+  const double turns = per_sm <= 4.0 ? 1.0 : 0.71 * per_sm / 4.0 + 0.29;
+  return steps * turns * (1.0 + 0.03 * log2((double)nseg));
 }
 
 // WENO5 segmentings of the output box b along direction dir, best first (at
@@ -1544,9 +1550,9 @@ int w5_candidates(const Dims &d, const Box &b, int dir, W5Tile *out, int max) {
     const int lb = (nout + nseg - 1) / nseg;
     if (lb == last) continue;
     last = lb;
-    if (lb < 4 && nseg > 1) break;
+    if (lb < 3 && nseg > 1) break;
     // the best four so far, in order
-    const double c = w5_cost(nout, nlines, lb);
+    const double c = w5_cost(nout, nlines, lb, stride == 1);
     int at = n < 4 ? n++ : 4;
     cost[at] = c;
     lbs[at] = lb;

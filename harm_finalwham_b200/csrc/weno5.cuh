@@ -413,6 +413,32 @@ __device__ __forceinline__ void faces(const T *u, const T *un, T m0, bool is_cus
 
 enum { kZero = 0, kOne = 1, kBlend = 2, kCusp = 3 };  // monoindicator 0, 1, in between; cusp (indicator 0)
 
+// The plain FP64 routines out of line, for the few cells that need them: the
+// marching loop has to stay within the instruction cache.
+struct Pair { double a, b; };
+struct Triple { double a, b, c; };
+static __device__ __noinline__ double mono_cold(double ym2, double ym1, double y0, double yp1, double yp2) {
+  const double y[5] = {ym2, ym1, y0, yp1, yp2};
+  return mono(y + 2, y + 2);
+}
+static __device__ __noinline__ Triple unopt3_cold(int code, double ym2, double ym1, double y0, double yp1, double yp2) {
+  const double y[5] = {ym2, ym1, y0, yp1, yp2};
+  double w[3];
+  unopt3(code == kBlend ? mono(y + 2, y + 2) : 0.0, y + 2, y + 2, w);
+  return Triple{w[0], w[1], w[2]};
+}
+static __device__ __noinline__ Pair faces_cold(int code, double ym2, double ym1, double y0, double yp1, double yp2,
+                                               double w0, double w1, double w2, double lof) {
+  const double y[5] = {ym2, ym1, y0, yp1, yp2}, w[3] = {w0, w1, w2};
+  double l, r;
+  faces(y + 2, y + 2, code == kBlend ? mono(y + 2, y + 2) : 0.0, code == kCusp, w, lof, &l, &r);
+  return Pair{l, r};
+}
+static __device__ __noinline__ double ratio_cold(double wc0, double wc2, double wl0, double wr2) {
+  const double wc[3] = {wc0, 0.0, wc2};
+  return ratio_lof(wc, wl0, wr2, 0.0);
+}
+
 template <typename T>
 __device__ __forceinline__ int code_of(const T *y, const T *yn) {
   if (cusp(y, yn)) return kCusp;
@@ -430,14 +456,14 @@ __device__ __forceinline__ double times_sign(double x, uint32_t hs) {
 //   0 where a pair of estimates differs in sign or the outer difference of
 //     either side is 0 (minmod gives 0);
 //   1 where every estimate is above the cut (they are compared by exponent
-//     word; x/12 > x/16, and the cusp test's norm is not below mono's cut but
-//     for rounding, which the word after the next covers);
+//     word; x/12 > x/16);
 //   otherwise mono decides.
 template <>
 __device__ __forceinline__ int code_of<double>(const double *y, const double *) {
   const double df_m1 = y[-1] - y[-2], df0 = y[0] - y[-1], df1 = y[1] - y[0], df2 = y[2] - y[1];
   const double ddf_m1 = df0 - df_m1, ddf0 = df1 - df0, ddf1 = df2 - df1;
-  const double norm = (fabs(y[-2]) + fabs(y[-1]) + fabs(y[0]) + fabs(y[1]) + fabs(y[2]) + K<double>::small) * K<double>::smono;
+  const double sum = fabs(y[-2]) + fabs(y[-1]) + fabs(y[0]) + fabs(y[1]) + fabs(y[2]);
+  const double norm = (sum + K<double>::small) * K<double>::smono;
   const uint32_t h0 = hi_word(df0), h1 = hi_word(df1);
   if (fabs(df0) > norm && times_sign(ddf_m1, h0) > norm && -times_sign(ddf0, h0) > norm &&
       ((-times_sign(df2, h0) > norm && fabs(df2 + df0) > 0.25 * (fabs(df2) + fabs(df0))) ||
@@ -447,6 +473,10 @@ __device__ __forceinline__ int code_of<double>(const double *y, const double *) 
       ((-times_sign(df_m1, h1) > norm && fabs(df_m1 + df1) > 0.25 * (fabs(df_m1) + fabs(df1))) ||
        (-times_sign(df0, h1) > norm && fabs(df0 + df1) > 0.25 * (fabs(df0) + fabs(df1)))))
     return kCusp;
+  // (estimates that both outer differences must agree with cannot agree with
+  // two of opposite sign)
+  const uint32_t dl = hi_word(df_m1), dr = hi_word(df2);
+  if ((int)(dl ^ dr) < 0 || df_m1 == 0.0 || df2 == 0.0) return kZero;
   // the numerators of mono's estimates
   const uint32_t l1 = hi_word(((-3 * y[-2] + y[2]) + (-10 * y[-1] - 6 * y[1])) + 18 * y[0]);
   const uint32_t l2 = hi_word(((11 * y[-2] - y[2]) + (-20 * y[-1] + 4 * y[1])) + 6 * y[0]);
@@ -454,15 +484,16 @@ __device__ __forceinline__ int code_of<double>(const double *y, const double *) 
   const uint32_t r1 = hi_word(((-y[-2] + 3 * y[2]) + (6 * y[-1] + 10 * y[1])) - 18 * y[0]);
   const uint32_t r2 = hi_word(((-y[-2] + 11 * y[2]) + (4 * y[-1] - 20 * y[1])) + 6 * y[0]);
   const uint32_t r3 = hi_word(((y[-2] + 3 * y[2]) - (6 * y[-1] + 10 * y[1])) + 12 * y[0]);
-  const uint32_t dl = hi_word(df_m1), dr = hi_word(df2);
-  const uint32_t diff = (l1 ^ dl) | (l1 ^ r1) | (l1 ^ dr) | (l2 ^ r2) | (l3 ^ r3);
-  if ((int)diff < 0 || df_m1 == 0.0 || df2 == 0.0) return kZero;
+  if ((int)((l1 ^ dl) | (l1 ^ r1) | (l2 ^ r2) | (l3 ^ r3)) < 0) return kZero;
   const uint32_t m = 0x7fffffffu;
   const int e12 = (int)min(min(l1 & m, r1 & m), min(l2 & m, r2 & m)) - (4 << 20);
   const int e2 = (int)min(l3 & m, r3 & m) - (1 << 20);
   const int e1 = (int)min(dl & m, dr & m);
-  if (min(min(e12, e2), e1) > (int)hi_word(norm) + 2) return kOne;
-  const double m0 = mono(y, y);
+  // (2^-43 of the sum is above mono's cut; where the cut is near the square
+  // root of the smallest number, its products underflow and it decides)
+  const int cut = max((int)hi_word(sum) - (43 << 20), (1023 - 500) << 20);
+  if (min(min(e12, e2), e1) > cut + 2) return kOne;
+  const double m0 = mono_cold(y[-2], y[-1], y[0], y[1], y[2]);
   return m0 == 0.0 ? kZero : (m0 == 1.0 ? kOne : kBlend);
 }
 
@@ -472,11 +503,26 @@ __device__ __forceinline__ void weights3(int code, const T *u, const T *un, T w[
   unopt3(m0, u, un, w);
 }
 
-// whether a divisor of the smoothness terms, or the square of a normalised
-// one, has a reciprocal by rcp_rn: each numerator is at least 1e-28 of it, so
-// [2^-700, 2^700] leaves the remainders exact
-__device__ __forceinline__ bool w_rcp_ok(double s) {
-  return (hi_word(s) << 1) - exp_word2(-700) < exp_word2(700) - exp_word2(-700) && lo_word(s) != 0xffffffffu;
+// The smoothness terms over their sum (+ DBL_MIN).  A small sum, down to 0, is
+// brought up with its terms by a power of two, which leaves the quotients as
+// they are: at the edge of a field that spreads into a region without one, a
+// line falls by hundreds of orders of magnitude within a few cells, and those
+// cells held their warps for most of a pass.  Each term is at least 1e-28 of
+// the sum unless it has underflowed, so the remainders (2^-104 of a term) are
+// exact.  False: a sum near the largest number, or a significand that rcp_rn
+// excludes.
+constexpr double kLift = 0x1p600;
+template <int N>
+__device__ __forceinline__ bool smooth_quotients(double (&si)[N], double s, double (&t)[N]) {
+  if (hi_word(s) < (uint32_t)(1023 - 400) << 20) {
+    s = (s + K<double>::tiny) * kLift;
+#pragma unroll
+    for (int q = 0; q < N; q++) si[q] *= kLift;
+  }
+  const double y = rcp_rn(s);
+#pragma unroll
+  for (int q = 0; q < N; q++) t[q] = quot(si[q], s, y);
+  return hi_word(s) < (uint32_t)(1023 + 860) << 20 && lo_word(s) != 0xffffffffu;
 }
 
 template <>
@@ -495,16 +541,12 @@ __device__ __forceinline__ void weights3<double>(int code, const double *u, cons
     const double sd1 = (u[-1] + u[1]) - t0;
     const double sd2 = (u[0] + u[-2]) - 2 * u[-1];
     const double e = (((u[-2] * u[-2] + u[2] * u[2]) + (u[-1] * u[-1] + u[1] * u[1])) + u[0] * u[0]) * K<double>::eps;
-    const double si0 = (13. / 12. * sd0 * sd0 + 1. / 4. * fd0 * fd0) + e;
-    const double si1 = (13. / 12. * sd1 * sd1 + 1. / 4. * fd1 * fd1) + e;
-    const double si2 = (13. / 12. * sd2 * sd2 + 1. / 4. * fd2 * fd2) + e;
-    const double s = (si0 + si2) + si1;
-    // a line of zeros: 0 / DBL_MIN = 0, as 0 times 0 gives
-    const bool z = s == 0.0;
-    ok = ok && (z || w_rcp_ok(s));
-    const double y = z ? 0.0 : rcp_rn(s);
-    double t0q = quot(si0, s, y) + K<double>::eps, t1q = quot(si1, s, y) + K<double>::eps,
-           t2q = quot(si2, s, y) + K<double>::eps;
+    double si[3] = {(13. / 12. * sd0 * sd0 + 1. / 4. * fd0 * fd0) + e,
+                    (13. / 12. * sd1 * sd1 + 1. / 4. * fd1 * fd1) + e,
+                    (13. / 12. * sd2 * sd2 + 1. / 4. * fd2 * fd2) + e};
+    double t[3];
+    ok = smooth_quotients(si, (si[0] + si[2]) + si[1], t) && ok;
+    double t0q = t[0] + K<double>::eps, t1q = t[1] + K<double>::eps, t2q = t[2] + K<double>::eps;
     t0q *= t0q;
     t1q *= t1q;
     t2q *= t2q;
@@ -517,7 +559,12 @@ __device__ __forceinline__ void weights3<double>(int code, const double *u, cons
     w[1] = quot(w1, sw, yw);
     w[2] = quot(w2, sw, yw);
   }
-  if (!ok) unopt3(code == kBlend ? mono(u, un) : 0.0, u, un, w);
+  if (!ok) {
+    const Triple r = unopt3_cold(code, u[-2], u[-1], u[0], u[1], u[2]);
+    w[0] = r.a;
+    w[1] = r.b;
+    w[2] = r.c;
+  }
 }
 
 // lower-order fraction of a cell from its weights, weights[0] of cell-2 and
@@ -539,8 +586,7 @@ __device__ __forceinline__ double lower_fraction<double>(int code, double wc0, d
   const double lo2 = 1.2999 * mb;
   if (ma < lo2 || (na < 1.2999 * nb && ma >= lo2)) return 0.0;
   if (na > 1.6001 * nb && ma > 1.6001 * mb) return 1.0;
-  const double wc[3] = {wc0, 0.0, wc2};
-  return ratio_lof(wc, wl0, wr2, 0.0);
+  return ratio_cold(wc0, wc2, wl0, wr2);
 }
 
 template <typename T>
@@ -582,12 +628,9 @@ __device__ __forceinline__ void face_values<double>(int code, const double *u, c
     // unopt2 and its optimised weights
     const double fd0 = dp - d0, fd1 = d0 - dm;
     const double e = ((dm * dm + dp * dp) + d0 * d0) * K<double>::eps;
-    const double si0 = fd0 * fd0 + e, si1 = fd1 * fd1 + e;
-    const double s = si0 + si1;
-    const bool z = s == 0.0;
-    ok = ok && (z || w_rcp_ok(s));
-    const double y = z ? 0.0 : rcp_rn(s);
-    double t0 = quot(si0, s, y) + K<double>::eps, t1 = quot(si1, s, y) + K<double>::eps;
+    double si[2] = {fd0 * fd0 + e, fd1 * fd1 + e}, t[2];
+    ok = smooth_quotients(si, si[0] + si[1], t) && ok;
+    double t0 = t[0] + K<double>::eps, t1 = t[1] + K<double>::eps;
     t0 *= t0;
     t1 *= t1;
     ok = ok && lo_word(t0) != 0xffffffffu && lo_word(t1) != 0xffffffffu;
@@ -618,8 +661,11 @@ __device__ __forceinline__ void face_values<double>(int code, const double *u, c
                     r1 * ((s18 + q38) + p34);
   *yl = vl + vl2;
   *yr = vr + vr2;
-  if (!ok)
-    faces(u, un, code == kBlend ? mono(u, un) : 0.0, code == kCusp, w, lof, yl, yr);
+  if (!ok) {
+    const Pair f = faces_cold(code, u[-2], u[-1], u[0], u[1], u[2], w[0], w[1], w[2], lof);
+    *yl = f.a;
+    *yr = f.b;
+  }
 }
 
 }  // namespace w5
