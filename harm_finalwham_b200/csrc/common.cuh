@@ -156,11 +156,14 @@ struct Box {
   int i0, j0, k0, ni, nj, nk;
   __host__ __device__ long long size() const { return (long long)ni * nj * nk; }
 };
+// (a context's zones number below 2^32 -- each takes over 600 bytes of device
+// memory -- so the index is divided in 32 bits, not by 64-bit routines)
 __device__ __forceinline__ void box_ijk(const Box &b, long long t, int &i, int &j, int &k) {
-  k = (int)(t % b.nk);
-  long long r = t / b.nk;
-  j = (int)(r % b.nj);
-  i = (int)(r / b.nj);
+  const unsigned u = (unsigned)t;
+  const unsigned r = u / (unsigned)b.nk;
+  k = (int)(u - r * b.nk);
+  i = (int)(r / (unsigned)b.nj);
+  j = (int)(r - (unsigned)i * b.nj);
   i += b.i0;
   j += b.j0;
   k += b.k0;
@@ -176,6 +179,18 @@ __device__ __forceinline__ void warp_min_atomic(unsigned long long *dst, double 
     bits = ob < bits ? ob : bits;
   }
   if ((threadIdx.x & 31) == 0 && bits != 0xFFFFFFFFFFFFFFFFull) atomicMin(dst, bits);
+}
+
+// one value from global to shared memory, asynchronously
+template <typename V>
+__device__ __forceinline__ void copy_async(double *to, const V *from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from),
+               "n"(sizeof(V)));
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;"); }
+template <int PENDING>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
 }
 
 // MC / VANL / MINM / DONOR slopes (interppoint.c:387-443)
@@ -247,8 +262,9 @@ __device__ __forceinline__ void para4(const T *y, T *lout, T *rout) {
 // the 256x128x128 WENO5 torus, 237 / 259 on 97x51x33 MC, 58 / 54 on 64x64
 // (there the few warps gain nothing from the fourth block and pay its
 // spills); WENO5 4 against 3 blocks 8921 / 9716 on 256x128x128, 1008 / 1100 on
-// 128x64x32; update 4 against 3 blocks 2240 / 1505, 154 / 85, 36 / 27: its
-// spills sit in the contraction with the connection, so 3.
+// 128x64x32; update 4 against 3 blocks 154 / 85 on 97x51x33,
+// 36 / 27 on 64x64 (its spills sit in the contraction with the connection), but
+// for the staged form (conserve_kernel), which takes 4.
 #ifndef HG_MINB_FLUX
 #define HG_MINB_FLUX 4
 #endif
@@ -404,18 +420,6 @@ __device__ __forceinline__ long long w5_line(const Dims &d, const Box &b, int li
     j = b.j0 + line % b.nj;
   }
   return zix(d, i, j, k);
-}
-
-// one value from global to shared memory, asynchronously
-template <typename V>
-__device__ __forceinline__ void copy_async(double *to, const V *from) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from),
-               "n"(sizeof(V)));
-}
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;"); }
-template <int PENDING>
-__device__ __forceinline__ void copy_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
 }
 
 // Lines next to one another in memory (not FS): neighbouring lanes are

@@ -30,7 +30,6 @@
 //   finalize_kernel   ndt combine (advance.c:231) and dt update (step_ch.c:236-247)
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
-#include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -259,12 +258,12 @@ __global__ void pi2u_kernel(Dims d, Params P, const double *__restrict__ p, cons
 }
 
 // source() -> source_conn() (phys.c:578-752): the connection contraction of
-// T^mu_nu for the state pbz (q, e formed from it), times gdet
-__device__ __forceinline__ void source_conn(const Dims &d, const double *__restrict__ G, long long ij,
-                                            const double *pbz, const State &q, const EM &e, const Metric &m,
+// T^mu_nu for the state pbz (q, e formed from it), times gdet; conn(jj, l, kk)
+// is the reference's conn[kk][l][jj]
+template <typename C>
+__device__ __forceinline__ void source_conn(C conn, const double *pbz, const State &q, const EM &e, const Metric &m,
                                             double gam, double *dUg) {
   double dUconn[4] = {0., 0., 0., 0.};
-  const double *conn = G + (long long)G_CONN * d.nij + ij;
   // each T^jj_kk row is contracted as soon as it is formed; every
   // dUconn[l] still adds its terms in the order jj, then kk
 #pragma unroll
@@ -275,7 +274,7 @@ __device__ __forceinline__ void source_conn(const Dims &d, const double *__restr
     for (int l = 0; l < 4; l++) {
       double s = dUconn[l];
 #pragma unroll
-      for (int kk = 0; kk < 4; kk++) s += row[kk] * __ldg(conn + (long long)((kk * 4 + l) * 4 + jj) * d.nij);
+      for (int kk = 0; kk < 4; kk++) s += row[kk] * conn(jj, l, kk);
       dUconn[l] = s;
     }
   }
@@ -283,7 +282,7 @@ __device__ __forceinline__ void source_conn(const Dims &d, const double *__restr
   for (int l = 0; l < 4; l++) {
     double s = dUconn[l];
 #pragma unroll
-    for (int jj = 0; jj < 4; jj++) s += -pbz[RHO] * q.ucon[jj] * __ldg(conn + (long long)((0 * 4 + l) * 4 + jj) * d.nij);
+    for (int jj = 0; jj < 4; jj++) s += -pbz[RHO] * q.ucon[jj] * conn(jj, l, 0);
     dUconn[l] = s;
   }
   // dU = sum of the NUMSOURCES components; only GEOMSOURCE is nonzero
@@ -292,26 +291,74 @@ __device__ __forceinline__ void source_conn(const Dims &d, const double *__restr
   for (int pl = 0; pl < NPR; pl++) dUg[pl] = (pl >= UU && pl <= U3) ? 0. + m.g * full[pl] : 0.;
 }
 
-// Bound by FP64 issue and registers: 0.75 ms a launch on 256x128x128 (RK2),
-// 1.37 ms with the tensors' zero diagonals multiplied out, every quotient a
-// division, 4 blocks per SM and both accumulators moved in each stage.
-template <int MB>
+// What the update reads of one (i, j), in the order in which STAGE keeps it in
+// shared memory: gcov 16, g^t1..3, alpha, 1/alpha, 1+g_tt, gdet, one unused,
+// then conn as [jj][l][kk].
+constexpr int GEO_WORDS = 88, GEO_CONN = 24;
+__device__ __forceinline__ long long geo_plane(int c) {
+  constexpr int cent = G_CENT * GLOC;
+  if (c < 16) return cent + c;
+  if (c < 19) return cent + 16 + (c - 15);
+  if (c < 21) return G_LAPSE + (c - 19);
+  if (c < 23) return cent + 32 + (c - 21);
+  if (c < GEO_CONN) return cent;  // unused
+  const int q = c - GEO_CONN;     // (jj, l, kk)
+  return G_CONN + (((q & 3) * 4 + ((q >> 2) & 3)) * 4 + (q >> 4));
+}
+constexpr int GEO_SLOTS = 5;       // (i, j) that 128 zones can touch when x3 has at least 32
+constexpr int STAGE_MIN_NK = 32;
+
+// Bound by FP64 issue, registers and the latency of its loads: 0.57 ms a launch
+// on 256x128x128 (RK2), 1.37 ms with the tensors' zero diagonals multiplied
+// out, every quotient a division and both accumulators moved in each stage.
+// STAGE: the block's few (i, j) and each thread's primitives (and ucum) come
+// into shared memory by asynchronous copies while the flux differences are
+// loaded and formed.  Read from global memory where they are used, they were
+// waited for in batches as wide as the free registers: 5.8 of 9 stall cycles
+// an instruction.  With fewer than STAGE_MIN_NK zones along x3 a block meets
+// up to 128 (i, j), each read by one lane, and the direct loads are coalesced.
+// Two launches on 256x128x128, 3 / 4 blocks per SM: 1505 / 2240 us direct, 1271
+// / 1131 staged; on 128x64x32 (RK4, four launches) 314 -> 210 us.
+template <int MB, bool STAGE>
 __global__ void __launch_bounds__(128, MB) conserve_kernel(
     Dims d, Params P, Box box, const double *pi, const double *pb, double *__restrict__ uf,
     double *__restrict__ ucum, const double *__restrict__ F1, const double *__restrict__ F2,
     const double *__restrict__ F3, const double *__restrict__ E, const double *__restrict__ G, Scalars *sc,
     double CUf0, double CUf1, double CUf2, double Cunew0, double Cunew1, double Cunew2, int timeorder,
     double *__restrict__ ui, int fv, int read_uf, int read_ucum, int write_uf) {
+  __shared__ __align__(16) double geo[STAGE ? GEO_SLOTS * GEO_WORDS : 1];
+  __shared__ double own[STAGE ? 3 * NPR * 128 : 1];
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= box.size()) return;
-  int i, j, k;
-  box_ijk(box, t, i, j, k);
-  const long long z = zix(d, i, j, k);
+  const bool in = t < box.size();
+  if (!STAGE && !in) return;
   const long long nz = d.nz;
+  int i, j, k;
+  box_ijk(box, in ? t : box.size() - 1, i, j, k);
+  const long long z = zix(d, i, j, k);
   const long long o1 = (long long)d.nt2 * d.nt3, o2 = d.nt3, o3 = 1;
   const long long ij = gix(d, i, j);
+  const double *mine = geo;
+  if constexpr (STAGE) {
+    // (i, j) rows of the box from the block's first zone to its last
+    const unsigned first = blockIdx.x * 128u / (unsigned)box.nk;
+    const unsigned rows = (unsigned)box.ni * box.nj;
+    mine = geo + ((unsigned)t / (unsigned)box.nk - first) * GEO_WORDS;
+    for (int c = threadIdx.x; c < GEO_SLOTS * GEO_WORDS; c += 128) {
+      const unsigned r = min(first + c / GEO_WORDS, rows - 1);
+      const unsigned ri = r / (unsigned)box.nj;
+      copy_async(geo + c, G + geo_plane(c % GEO_WORDS) * d.nij + gix(d, box.i0 + ri, box.j0 + (r - ri * box.nj)));
+    }
+#pragma unroll
+    for (int v = 0; v < NPR; v++) {
+      copy_async(own + v * 128 + threadIdx.x, pb + v * nz + z);
+      if (!fv && pi != pb) copy_async(own + (NPR + v) * 128 + threadIdx.x, pi + v * nz + z);
+      if (read_ucum || (fv && timeorder == 0)) copy_async(own + (2 * NPR + v) * 128 + threadIdx.x, ucum + v * nz + z);
+    }
+    copy_commit();
+  }
   double dt, gam, dx1;
-  if (!zone_step(P, sc, z, i, dt, gam, dx1)) return;
+  const bool live = zone_step(P, sc, z, i, dt, gam, dx1) && in;
+  if (!STAGE && !live) return;
     double Ui[NPR], dUg[NPR], dUr[NPR];
     // the flux differences first: their ~50 independent loads are in flight
     // together before the arithmetic of U(pi) and the source term
@@ -349,8 +396,38 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
         dUr[pl] = a1 + a2 + a3;
       }
     }
+    if constexpr (STAGE) {
+      copy_wait<0>();
+      __syncthreads();
+      if (!live) return;
+    }
     Metric m;
-    load_metric(G, d, ij, G_CENT, m);
+    if constexpr (STAGE) {
+#pragma unroll
+      for (int q = 0; q < 16; q++) m.gcov[q] = mine[q];
+#pragma unroll
+      for (int q = 1; q < 4; q++) m.gcon[q] = mine[15 + q];
+      m.alpha = mine[19];
+      m.ralpha = mine[20];
+      m.gcovpert_tt = mine[21];
+      m.g = mine[22];
+      derive_shift(m);
+    } else {
+      load_metric(G, d, ij, G_CENT, m);
+    }
+    auto conn = [&](int jj, int l, int kk) {
+      if constexpr (STAGE) return mine[GEO_CONN + (jj * 4 + l) * 4 + kk];
+      else return __ldg(G + (long long)(G_CONN + (kk * 4 + l) * 4 + jj) * d.nij + ij);
+    };
+    // a primitive vector (or ucum: 2) of this zone
+    auto load_own = [&](int which, const double *from, double *to) {
+      if constexpr (STAGE) {
+#pragma unroll
+        for (int v = 0; v < NPR; v++) to[v] = own[(which * NPR + v) * 128 + threadIdx.x];
+      } else {
+        load_prim(from, d, z, to);
+      }
+    };
     int err = 0;
     if (fv) {
       // advance_finitevolume (advance.c:245-501): Ui is the stored conserved
@@ -359,7 +436,7 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
       if (timeorder == 0) {
 #pragma unroll
         for (int pl = 0; pl < NPR; pl++) {
-          Ui[pl] = ucum[pl * nz + z];
+          Ui[pl] = STAGE ? own[(2 * NPR + pl) * 128 + threadIdx.x] : ucum[pl * nz + z];
           ui[pl * nz + z] = Ui[pl];
         }
       } else {
@@ -367,27 +444,27 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
         for (int pl = 0; pl < NPR; pl++) Ui[pl] = ui[pl * nz + z];
       }
       double pbz[NPR];
-      load_prim(pb, d, z, pbz);
+      load_own(0, pb, pbz);
       State q;
       EM e;
       if (get_state(pbz, m, q)) err |= ERR_UTCALC_DISCR;
       em_prepare<0>(pbz, m, q, e);
-      source_conn(d, G, ij, pbz, q, e, m, gam, dUg);
+      source_conn(conn, pbz, q, e, m, gam, dUg);
     } else if (pi == pb) {
       // a first substep: U(pi) and the source read the same state, whose
       // get_state and field terms are formed once
       double pbz[NPR];
-      load_prim(pb, d, z, pbz);
+      load_own(0, pb, pbz);
       State q;
       EM e;
       if (get_state(pbz, m, q)) err |= ERR_UTCALC_DISCR;
       em_prepare<0>(pbz, m, q, e);
       primtoflux<0>(pbz, q, e, m, gam, Ui);
-      source_conn(d, G, ij, pbz, q, e, m, gam, dUg);
+      source_conn(conn, pbz, q, e, m, gam, dUg);
     } else {
       {
         double pr[NPR];
-        load_prim(pi, d, z, pr);
+        load_own(1, pi, pr);
         State qi;
         EM ei;
         if (get_state(pr, m, qi)) err |= ERR_UTCALC_DISCR;
@@ -395,19 +472,19 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
         primtoflux<0>(pr, qi, ei, m, gam, Ui);
       }
       double pbz[NPR];
-      load_prim(pb, d, z, pbz);
+      load_own(0, pb, pbz);
       State q;
       EM e;
       if (get_state(pbz, m, q)) err |= ERR_UTCALC_DISCR;
       em_prepare<0>(pbz, m, q, e);
-      source_conn(d, G, ij, pbz, q, e, m, gam, dUg);
+      source_conn(conn, pbz, q, e, m, gam, dUg);
     }
     // dUtoU (advance.c:922-949)
     double Uf[NPR], Ucum[NPR];
 #pragma unroll
     for (int pl = 0; pl < NPR; pl++) {
       const double ufo = read_uf ? uf[pl * nz + z] : 0.0;
-      const double uco = read_ucum ? ucum[pl * nz + z] : 0.0;
+      const double uco = read_ucum ? (STAGE ? own[(2 * NPR + pl) * 128 + threadIdx.x] : ucum[pl * nz + z]) : 0.0;
       Uf[pl] = CUf0 * Ui[pl] + CUf1 * ufo + CUf2 * dt * (dUr[pl] + dUg[pl]);
       Ucum[pl] = uco + (Cunew0 * Ui[pl] + Cunew1 * dt * (dUr[pl] + dUg[pl]) + Cunew2 * Uf[pl]);
       if (write_uf) uf[pl * nz + z] = Uf[pl];
@@ -1521,18 +1598,19 @@ inline unsigned grid_for(long long n, int block) { return (unsigned)((n + block 
 // its line.  A thread takes lb + 10 steps (staged lines: whole chunks), of
 // which the first ten cost about five.  Up to four blocks an SM, all resident,
 // a step takes the latency of its arithmetic however many there are; beyond
-// that blocks come in turn, at 0.71 of that time per four.  Measured on the
-// B200, us a step of two stages, x1 of 128x64x32 in 1, 2, 4, 6, 10, 24 segments:
-// 1040, 856, 777, 758, 748, 772 (modelled 135, 70, 38, 35, 36, 44); x1 of
-// 256x128x64 in 1, 3, 6, 16: 3958, 3727, 3688, 3799 (263, 202, 199, 214).
-// Near ties go to the longer segments, which repeat fewer cells.
+// that blocks come in turn, at 0.71 of that time per four, and the last ones
+// leave half a turn idle.  Measured on the B200, us a step of two stages, x1 of
+// 128x64x32 in 1, 2, 4, 6, 10, 24 segments: 1040, 856, 777, 758, 748, 772
+// (modelled 135, 70, 38, 41, 39, 47); x1 of 256x128x64 in 1, 3, 6, 16: 3958,
+// 3727, 3688, 3799 (263, 221, 210, 217); x3 of 256x128x128 in 1, 2, 4: 8267,
+// 7994, 8062 (420, 415, 452).
 double w5_cost(int nout, long long nlines, int lb, bool staged) {
   const long long nseg = (nout + lb - 1) / lb;
   const long long blocks = (nlines * nseg * NPR + W5_THREADS - 1) / W5_THREADS;
   const double per_sm = (double)blocks / 148.0;
   const int steps = staged ? (lb + 10 + W5_CHUNK - 1) / W5_CHUNK * W5_CHUNK - 5 : lb + 5;
-  const double turns = per_sm <= 4.0 ? 1.0 : 0.71 * per_sm / 4.0 + 0.29;
-  return steps * turns * (1.0 + 0.03 * log2((double)nseg));
+  const double turns = 0.71 * per_sm / 4.0 + 0.5;
+  return steps * (per_sm <= 4.0 ? 1.0 : turns);
 }
 
 // WENO5 segmentings of the output box b along direction dir, best first (at
@@ -1962,6 +2040,8 @@ int hgpu_create_batch(const hgpu_config *cfg, int ninst, const int *n1, const do
     set_err("a batch runs the standard (NOENOFLUX) scheme");
     return HGPU_E_INVALID;
   }
+  // the staged update hides its spills: 4 blocks, where the direct one takes 3
+  x->tune.conserve = x->active_box.nk >= STAGE_MIN_NK ? 1 : 0;
   long long total = 0;
   for (int b = 0; b < ninst; b++) {
     if (n1[b] < cfg->ng || !(dx1[b] > 0.0) || !(gam[b] > 1.0)) {
@@ -2346,7 +2426,9 @@ static void launch_stage_advance(hgpu_ctx *x, int timeorder, bool folded = false
     read_ucum |= E.cun[0] != 0.0 || E.cun[1] != 0.0 || E.cun[2] != 0.0;
   }
   const int read_uf = timeorder > 0 && CUf1 != 0.0, write_uf = !finalstep;
-  auto update = x->tune.conserve ? conserve_kernel<kConserveMB[1]> : conserve_kernel<kConserveMB[0]>;
+  const bool stage = x->active_box.nk >= STAGE_MIN_NK;
+  auto update = x->tune.conserve ? (stage ? conserve_kernel<kConserveMB[1], true> : conserve_kernel<kConserveMB[1], false>)
+                                 : (stage ? conserve_kernel<kConserveMB[0], true> : conserve_kernel<kConserveMB[0], false>);
   LAUNCH(x, K_UPDATE, update, grid_for(x->active_box.size(), 128), 128, d, x->P, x->active_box, pi, pb, x->uf, x->ucum,
          x->F[1], x->F[2], x->F[3], x->E, x->G, x->sc, CUf0, CUf1, CUf2, Cn0, Cn1, Cn2, timeorder, x->ui, fv, read_uf,
          (int)read_ucum, write_uf);
