@@ -883,43 +883,109 @@ __device__ __forceinline__ void bound_ghost(const Dims &d, const Params &P, int 
   if (err) atomicOr(&sc->err, err);
 }
 
+// fixup_checksolution (fixup.c:460-560), part 1: gamma on i,j,k = -1..N and the
+// list of active candidate zones (gamma >= 2); fixlist (unless null): the
+// failed zones that checksolution leaves alone, for fixup_small_kernel
+struct GammaJob {
+  double *gammacheck;  // null: no gamma pass
+  long long *cand, *fixlist;
+  int cap;
+};
+__device__ __forceinline__ void checksol_gamma(const Dims &d, const Params &P, const GammaJob &J, int i, int j, int k,
+                                               long long z, double u1, double u2, double u3,
+                                               const double *__restrict__ G, Scalars *sc, const int *pflag) {
+  if (i < -d.s1 || i > d.n1 - 1 + d.s1 || j < -d.s2 || j > d.n2 - 1 + d.s2 || k < -d.s3 || k > d.n3 - 1 + d.s3) return;
+  Metric m;
+  load_metric(G, d, gix(d, i, j), G_CENT, m);
+  const double pr[NPR] = {0., 0., u1, u2, u3, 0., 0., 0.};
+  double gamma = 0.0;
+  if (gamma_calc(pr, m, &gamma)) atomicOr(&sc->err, ERR_UTCALC_DISCR);
+  J.gammacheck[z] = gamma;
+  bool activez = (i >= 0 && i < d.n1 && j >= 0 && j < d.n2 && k >= 0 && k < d.n3);
+  if (P.cell_inst) {
+    const Inst &I = P.inst[P.cell_inst[z]];
+    int loc = i - I.i0;
+    activez = (loc >= 0 && loc < I.n && !I.done);
+  }
+  if (!activez || sc->done) return;
+  if (gamma >= 2.0) {
+    int slot = atomicAdd(&sc->ncand, 1);
+    if (slot < J.cap) J.cand[slot] = z;
+    else atomicOr(&sc->overflow, 1);
+  } else if (J.fixlist && pflag[z] != 0) {
+    int slot = atomicAdd(&sc->nfixlist, 1);
+    if (slot < J.cap) J.fixlist[slot] = z;
+    else atomicOr(&sc->overflow, 2);
+  }
+}
+
 // bound_prim in one launch over the ghost zones alone (a thread per zone of
 // the box, most of them active and idle, took 60 us on 256x128x128), then
 // POLEDEATH on the active first/last x2 rows.  A ghost zone that reads such a
 // row is in it itself and zeroes what it read, in any order; only the x1
 // ghosts' inflow check looks at u~2 before that, so the rows' first and last
 // zones, which those ghosts read, wait for the last block.
-// close: that block also ends the step.
+// close: that block also ends the step.  gamma: every zone's Lorentz factor for
+// checksolution follows from what its thread has just written or left, and
+// the threads of the pole rows become threads of all active zones.
 struct BoundJob {
-  unsigned n[4];  // threads: x1 ghosts, x2 ghosts (active i), x3 ghosts (active i, j), active pole rows
+  unsigned n[4];  // threads: x1 ghosts, x2 ghosts (active i), x3 ghosts (active i, j), active pole rows or zones
   int corners, close;
+  GammaJob gamma;
 };
 __global__ void __launch_bounds__(128) bound_kernel(Dims d, Params P, BoundJob J, double *p,
                                                     const double *__restrict__ G, Scalars *sc, int *pflag) {
   unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  int i, j, k;
+  bool ghost = true, any = true;
   if (t < J.n[0]) {
-    const int k = (int)(t % d.nt3) - d.g3;
+    k = (int)(t % d.nt3) - d.g3;
     const unsigned r = t / d.nt3;
-    const int j = (int)(r % d.nt2) - d.g2, q = (int)(r / d.nt2);
-    bound_ghost(d, P, q < d.g1 ? q - d.g1 : d.n1 + q - d.g1, j, k, p, G, sc, pflag);
+    j = (int)(r % d.nt2) - d.g2;
+    const int q = (int)(r / d.nt2);
+    i = q < d.g1 ? q - d.g1 : d.n1 + q - d.g1;
   } else if ((t -= J.n[0]) < J.n[1]) {
-    const int k = (int)(t % d.nt3) - d.g3;
+    k = (int)(t % d.nt3) - d.g3;
     const unsigned r = t / d.nt3;
-    const int q = (int)(r % (2 * d.g2)), i = (int)(r / (2 * d.g2));
-    bound_ghost(d, P, i, q < d.g2 ? q - d.g2 : d.n2 + q - d.g2, k, p, G, sc, pflag);
+    const int q = (int)(r % (2 * d.g2));
+    j = q < d.g2 ? q - d.g2 : d.n2 + q - d.g2;
+    i = (int)(r / (2 * d.g2));
   } else if ((t -= J.n[1]) < J.n[2]) {
     const int q = (int)(t % (2 * d.g3));
+    k = q < d.g3 ? q - d.g3 : d.n3 + q - d.g3;
     const unsigned r = t / (2 * d.g3);
-    const int j = (int)(r % d.n2), i = (int)(r / d.n2);
-    bound_ghost(d, P, i, j, q < d.g3 ? q - d.g3 : d.n3 + q - d.g3, p, G, sc, pflag);
-  } else if ((t -= J.n[2]) < J.n[3]) {
-    const int k = (int)(t % d.n3);
+    j = (int)(r % d.n2);
+    i = (int)(r / d.n2);
+  } else {
+    ghost = false;
+    any = (t -= J.n[2]) < J.n[3];
+    k = (int)(t % d.n3);
     const unsigned r = t / d.n3;
-    const int i = (int)(r >> 1), up = (int)(r & 1);
-    if (i > 0 && i < d.n1 - 1 && P.bc[up ? 2 : 3] == HGPU_BC_POLARAXIS) {
-      const long long z = zix(d, i, up ? d.n2 - 1 : 0, k);
-      p[(long long)U2 * d.nz + z] *= 0;
-      p[(long long)B2 * d.nz + z] *= 0.;
+    if (J.gamma.gammacheck) {
+      j = (int)(r % d.n2);
+      i = (int)(r / d.n2);
+    } else {
+      j = (r & 1) ? d.n2 - 1 : 0;
+      i = (int)(r >> 1);
+    }
+  }
+  if (any) {
+    const long long z = zix(d, i, j, k);
+    bool pole = false;
+    if (ghost) {
+      bound_ghost(d, P, i, j, k, p, G, sc, pflag);
+    } else {
+      pole = J.corners && ((j == 0 && P.bc[3] == HGPU_BC_POLARAXIS) || (j == d.n2 - 1 && P.bc[2] == HGPU_BC_POLARAXIS));
+      if (pole && i > 0 && i < d.n1 - 1) {
+        p[(long long)U2 * d.nz + z] *= 0;
+        p[(long long)B2 * d.nz + z] *= 0.;
+      }
+    }
+    if (J.gamma.gammacheck) {
+      // (the corner zones' u~2 goes to zero below)
+      double u2 = p[(long long)U2 * d.nz + z];
+      if (pole) u2 *= 0;
+      checksol_gamma(d, P, J.gamma, i, j, k, z, p[(long long)U1 * d.nz + z], u2, p[(long long)U3 * d.nz + z], G, sc, pflag);
     }
   }
   if (!(J.corners || J.close) || !last_block(sc)) return;
@@ -978,48 +1044,28 @@ __device__ __forceinline__ void bound_batch(long long t, const Dims &d, const Pa
   }
   if (pflag) pflag[t] = pflag[zs];
 }
-__global__ void bound_batch_kernel(Dims d, Params P, double *pv, int *pflag, Scalars *sc, int close) {
-  bound_batch((long long)blockIdx.x * blockDim.x + threadIdx.x, d, P, pv, pflag);
+__global__ void bound_batch_kernel(Dims d, Params P, double *pv, int *pflag, const double *__restrict__ G,
+                                   GammaJob gamma, Scalars *sc, int close) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  bound_batch(t, d, P, pv, pflag);
+  if (gamma.gammacheck && t < d.nz)
+    checksol_gamma(d, P, gamma, (int)t - d.g1, 0, 0, t, pv[U1 * d.nz + t], pv[U2 * d.nz + t], pv[U3 * d.nz + t], G, sc,
+                   pflag);
   if (close && last_block(sc)) close_step(P, sc);
 }
 
 // ---------------------------------------------------------------------------
 // post_fixup (fixup.c:37-96)
 // ---------------------------------------------------------------------------
-// fixup_checksolution (fixup.c:460-560), part 1: gamma on i,j,k = -1..N and
-// the list of active candidate zones (gamma >= 2)
-__global__ void checksol_gamma_kernel(Dims d, Params P, Box box, const double *__restrict__ pv,
-                                      const double *__restrict__ G,
-                                      double *__restrict__ gammacheck, long long *__restrict__ cand, int cap,
-                                      Scalars *sc, const int *__restrict__ pflag, long long *__restrict__ fixlist) {
+// fixup_checksolution (fixup.c:460-560), part 1, as a kernel of its own
+__global__ void checksol_gamma_kernel(Dims d, Params P, Box box, GammaJob J, const double *__restrict__ pv,
+                                      const double *__restrict__ G, Scalars *sc, const int *__restrict__ pflag) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= box.size()) return;
   int i, j, k;
   box_ijk(box, t, i, j, k);
-  long long z = zix(d, i, j, k);
-  Metric m;
-  load_metric(G, d, gix(d, i, j), G_CENT, m);
-  double pr[NPR];
-  load_prim(pv, d, z, pr);
-  double gamma = 0.0;
-  if (gamma_calc(pr, m, &gamma)) atomicOr(&sc->err, ERR_UTCALC_DISCR);
-  gammacheck[z] = gamma;
-  bool activez = (i >= 0 && i < d.n1 && j >= 0 && j < d.n2 && k >= 0 && k < d.n3);
-  if (P.cell_inst) {
-    const Inst &I = P.inst[P.cell_inst[z]];
-    int loc = i - I.i0;
-    activez = (loc >= 0 && loc < I.n && !I.done);
-  }
-  if (activez && gamma >= 2.0 && !sc->done) {
-    int slot = atomicAdd(&sc->ncand, 1);
-    if (slot < cap) cand[slot] = z;
-    else atomicOr(&sc->overflow, 1);
-  } else if (fixlist && activez && !sc->done && pflag[z] != 0) {
-    // fixup_small_kernel's list: failed zones that checksolution leaves alone
-    int slot = atomicAdd(&sc->nfixlist, 1);
-    if (slot < cap) fixlist[slot] = z;
-    else atomicOr(&sc->overflow, 2);
-  }
+  const long long z = zix(d, i, j, k);
+  checksol_gamma(d, P, J, i, j, k, z, pv[U1 * d.nz + z], pv[U2 * d.nz + z], pv[U3 * d.nz + z], G, sc, pflag);
 }
 
 // In the reference the candidates are visited in loop order (i, then j, then
@@ -1994,6 +2040,8 @@ int hgpu_create(const hgpu_config *cfg, hgpu_ctx **out) {
     set_err("device allocation failed");
     return HGPU_E_NOMEM;
   }
+  // the staged update hides its spills: 4 blocks, where the direct one takes 3
+  x->tune.conserve = x->active_box.nk >= STAGE_MIN_NK ? 1 : 0;
   x->P.ffc = x->ffc;
   // post_fixup's lists and scratch live in the flux planes, which are read
   // for the last time by the conserved update before it and written by the
@@ -2040,8 +2088,6 @@ int hgpu_create_batch(const hgpu_config *cfg, int ninst, const int *n1, const do
     set_err("a batch runs the standard (NOENOFLUX) scheme");
     return HGPU_E_INVALID;
   }
-  // the staged update hides its spills: 4 blocks, where the direct one takes 3
-  x->tune.conserve = x->active_box.nk >= STAGE_MIN_NK ? 1 : 0;
   long long total = 0;
   for (int b = 0; b < ninst; b++) {
     if (n1[b] < cfg->ng || !(dx1[b] > 0.0) || !(gam[b] > 1.0)) {
@@ -2329,12 +2375,29 @@ static void launch_fluxes(hgpu_ctx *x, const double *pb, bool bsq = false, int s
          x->G, x->E, x->sc, stage_clear);
 }
 
-// flags: the failure flags' ghosts too; close: the kernel also ends the step
-static void launch_bound(hgpu_ctx *x, double *pv, bool flags = false, bool close = false) {
+// whether post_fixup runs in one cluster (fixup_small_kernel)
+static bool small_fixup(const hgpu_ctx *x) {
+  return (long long)x->d.n1 * x->d.n2 * x->d.n3 <= (x->P.cell_inst ? kSmallBatch : kSmallDomain);
+}
+// Whether the bound kernel of a step also forms checksolution's Lorentz factors.
+// It saves a launch, and costs the active zones the heavier kernel: us a step
+// with / without, 64x64 155 / 168, 97x51x33 450 / 456, 128x64x32 (RK4) 2182 /
+// 2157, 256x128x128 13233 / 12980; a batch's kernel is light (72 / 77 ms).
+static bool fused_gamma(const hgpu_ctx *x) {
+  return x->P.cell_inst || (long long)x->d.n1 * x->d.n2 * x->d.n3 <= 200000;
+}
+static GammaJob gamma_job(const hgpu_ctx *x) {
+  return GammaJob{x->gammacheck, x->cand, small_fixup(x) ? x->fixlist : nullptr, x->cap};
+}
+
+// flags: the failure flags' ghosts too; gamma: checksolution's Lorentz factors
+// and lists; close: the kernel also ends the step
+static void launch_bound(hgpu_ctx *x, double *pv, bool flags = false, bool close = false, bool gamma = false) {
   const Dims &d = x->d;
+  const GammaJob gj = gamma ? gamma_job(x) : GammaJob{nullptr, nullptr, nullptr, 0};
   int *pf = flags ? x->pflag : nullptr;
   if (x->P.cell_inst) {
-    LAUNCH(x, K_BOUND_GHOST, bound_batch_kernel, grid_for(d.nz, 128), 128, d, x->P, pv, pf, x->sc, (int)close);
+    LAUNCH(x, K_BOUND_GHOST, bound_batch_kernel, grid_for(d.nz, 128), 128, d, x->P, pv, pf, x->G, gj, x->sc, (int)close);
     return;
   }
   if (x->P.bondi) {
@@ -2346,8 +2409,9 @@ static void launch_bound(hgpu_ctx *x, double *pv, bool flags = false, bool close
   J.n[1] = (unsigned)d.n1 * 2 * d.g2 * d.nt3;
   J.n[2] = (unsigned)d.n1 * d.n2 * 2 * d.g3;
   J.corners = d.n2 > 1 && (x->P.bc[2] == HGPU_BC_POLARAXIS || x->P.bc[3] == HGPU_BC_POLARAXIS);
-  J.n[3] = J.corners ? (unsigned)d.n1 * 2 * d.n3 : 0;
+  J.n[3] = gamma ? (unsigned)d.n1 * d.n2 * d.n3 : (J.corners ? (unsigned)d.n1 * 2 * d.n3 : 0);
   J.close = close;
+  J.gamma = gj;
   const unsigned blocks = grid_for((long long)J.n[0] + J.n[1] + J.n[2] + J.n[3], 128);
   LAUNCH(x, K_BOUND_GHOST, bound_kernel, blocks ? blocks : 1, 128, d, x->P, J, pv, x->G, x->sc, pf);
 }
@@ -2444,12 +2508,13 @@ static void launch_stage_advance(hgpu_ctx *x, int timeorder, bool folded = false
     LAUNCH(x, K_INVERT, invert, gi, 128, d, x->P, x->active_box, pb, pf, x->uf, x->ucum, x->G, x->pflag, x->sc, finalstep,
            ufv);
   }
-  // bound_prim, and bound_pflag, which opens post_fixup (fixup.c:37-96)
-  launch_bound(x, pf, true);
+  // bound_prim, and bound_pflag, which opens post_fixup (fixup.c:37-96); the
+  // Lorentz factors wait for the ghost planes where others may bring them
+  launch_bound(x, pf, true, false, folded && fused_gamma(x));
 }
 
 // fixup_checksolution and fixup_utoprim on pf with the context's flags
-static void launch_checksol_fixup(hgpu_ctx *x, double *pf, int finalstep) {
+static void launch_checksol_fixup(hgpu_ctx *x, double *pf, int finalstep, bool gamma_done = false) {
   const Dims &d = x->d;
   FixJob J;
   J.d = d;
@@ -2469,10 +2534,10 @@ static void launch_checksol_fixup(hgpu_ctx *x, double *pf, int finalstep) {
   J.cap = x->cap;
   J.finalstep = finalstep;
   J.sc = x->sc;
-  const bool small = (long long)d.n1 * d.n2 * d.n3 <= (x->P.cell_inst ? kSmallBatch : kSmallDomain);
-  LAUNCH(x, K_CHECK_GAMMA, checksol_gamma_kernel, grid_for(x->dq_box.size(), 128), 128, d, x->P, x->dq_box, pf, x->G,
-         x->gammacheck, x->cand, x->cap, x->sc, x->pflag, small ? x->fixlist : nullptr);
-  if (small) {
+  if (!gamma_done)
+    LAUNCH(x, K_CHECK_GAMMA, checksol_gamma_kernel, grid_for(x->dq_box.size(), 128), 128, d, x->P, x->dq_box, gamma_job(x),
+           pf, x->G, x->sc, x->pflag);
+  if (small_fixup(x)) {
     LAUNCH(x, K_CHECK_RESOLVE, fixup_small_kernel, FIX_CLUSTER, FIX_THREADS, J, x->P);
     return;
   }
@@ -2492,9 +2557,10 @@ static void launch_checksol_fixup(hgpu_ctx *x, double *pf, int finalstep) {
   LAUNCH(x, K_FIX_SCATTER, fixup_scatter_kernel, fixgrid, 128, J, x->P);
 }
 
-static void launch_stage_fixup(hgpu_ctx *x, int timeorder, bool close = false) {
+static void launch_stage_fixup(hgpu_ctx *x, int timeorder, bool folded = false) {
   double *pf = stage_output(x, timeorder);
-  launch_checksol_fixup(x, pf, timeorder == num_orders(x) - 1);
+  const bool close = folded && timeorder == num_orders(x) - 1;
+  launch_checksol_fixup(x, pf, timeorder == num_orders(x) - 1, folded && fused_gamma(x));
   launch_bound(x, pf, false, close);
 }
 
@@ -2510,7 +2576,7 @@ static void launch_step(hgpu_ctx *x) {
   const int norders = num_orders(x);
   for (int o = 0; o < norders; o++) {
     launch_stage_advance(x, o, true);
-    launch_stage_fixup(x, o, o == norders - 1);
+    launch_stage_fixup(x, o, true);
   }
 }
 
@@ -2752,6 +2818,9 @@ static int utoprim_batch_impl(const double *U, const double *gcov, const double 
   if (e != cudaSuccess) {
     rc = HGPU_E_NOMEM;
   } else {
+    double *dU = base, *dgcov = dU + 8 * n, *dgcon = dgcov + 16 * n, *dg = dgcon + 16 * n, *dpr = dg + n;
+    unsigned long long *dit = (unsigned long long *)(dpr + 8 * n);
+    int *dpf = (int *)(dit + 1);
     cudaMemcpy(dU, U, sizeof(double) * 8 * n, cudaMemcpyHostToDevice);
     cudaMemcpy(dgcov, gcov, sizeof(double) * 16 * n, cudaMemcpyHostToDevice);
     cudaMemcpy(dgcon, gcon, sizeof(double) * 16 * n, cudaMemcpyHostToDevice);
@@ -2812,9 +2881,6 @@ __device__ double divb_fluxct(const Dims &d, const Params &P, const double *__re
   auto avg2 = [&](int ii, int jj, int kk, int pl) { return 0.5 * (Fg(ii, jj, kk, pl) + Fg(ii, jj - s2, kk, pl)); };
   auto for1 = [&](int ii, int jj, int kk) { return 0.5 * (avg2(ii, jj, kk, B1) + avg2(ii, jj, kk - s3, B1)); };
   auto for2 = [&](int ii, int jj, int kk) { return 0.5 * (avg1(ii, jj, kk, B2) + avg1(ii, jj, kk - s3, B2)); };
-    double *dU = base, *dgcov = dU + 8 * n, *dgcon = dgcov + 16 * n, *dg = dgcon + 16 * n, *dpr = dg + n;
-    unsigned long long *dit = (unsigned long long *)(dpr + 8 * n);
-    int *dpf = (int *)(dit + 1);
   auto for3 = [&](int ii, int jj, int kk) { return 0.5 * (avg2(ii, jj, kk, B3) + avg2(ii - s1, jj, kk, B3)); };
   double dfx = for1(i, j, k) - for1(i - s1, j, k);
   double dfy = for2(i, j, k) - for2(i, j - s2, k);
