@@ -624,13 +624,14 @@ __global__ void finalize_batch_kernel(Params P, int advance_time) {
   if (b < P.ninst) finalize_inst(P, b, advance_time);
 }
 
-// one block: before a stage (counts), or at the start of a call of steps
-// (call: also what accumulates over a call, as clear_counters)
+// one block: before a stage, or at the start of a call of steps (call: what
+// accumulates over a call, as clear_counters; each stage clears its counts)
 __global__ void reset_stage_kernel(Params P, Scalars *sc, int call) {
   clear_ndt(P, sc, threadIdx.x, blockDim.x);
   if (threadIdx.x != 0) return;
-  clear_stage_counts(sc);
-  if (call) {
+  if (!call) {
+    clear_stage_counts(sc);
+  } else {
     sc->iters = 0;
     sc->err = 0;
     sc->nfixed = 0;
@@ -1659,6 +1660,12 @@ double w5_cost(int nout, long long nlines, int lb, bool staged) {
   return steps * (per_sm <= 4.0 ? 1.0 : turns);
 }
 
+// What hgpu_set_tuning accepts as a tile of lb cells on w lines: the shared
+// memory that the tiled form of the kernel took for it, up to 72 KB.
+bool w5_tile_accepted(int lb, int w) {
+  return (long long)w * (8LL * (lb + 10) + 8 * (6LL * lb + 26)) <= 72 * 1024;
+}
+
 // WENO5 segmentings of the output box b along direction dir, best first (at
 // most `max`, at most 4): every segment count whose last segment is not
 // mostly empty, by the cost above.  Lines whose cells are contiguous in
@@ -1675,6 +1682,7 @@ int w5_candidates(const Dims &d, const Box &b, int dir, W5Tile *out, int max) {
     if (lb == last) continue;
     last = lb;
     if (lb < 3 && nseg > 1) break;
+    if (!w5_tile_accepted(lb, 1)) continue;
     // the best four so far, in order
     const double c = w5_cost(nout, nlines, lb, stride == 1);
     int at = n < 4 ? n++ : 4;
@@ -1692,7 +1700,8 @@ int w5_candidates(const Dims &d, const Box &b, int dir, W5Tile *out, int max) {
     t.nlines = (int)nlines;
     t.fast_s = stride == 1;
     t.lb = lbs[i];
-    t.w = 32;
+    t.w = 32;  // as many as hgpu_set_tuning would take with lb
+    while (t.w > 1 && !w5_tile_accepted(t.lb, t.w)) t.w >>= 1;
     t.nseg = (nout + t.lb - 1) / t.lb;
   }
   return n;
@@ -1702,12 +1711,6 @@ W5Tile w5_tiling(const Dims &d, const Box &b, int dir) {
   W5Tile t[1];
   w5_candidates(d, b, dir, t, 1);
   return t[0];
-}
-
-// What hgpu_set_tuning accepts as a tile of lb cells on w lines: the shared
-// memory that the tiled form of the kernel took for it, up to 72 KB.
-bool w5_tile_accepted(int lb, int w) {
-  return (long long)w * (8LL * (lb + 10) + 8 * (6LL * lb + 26)) <= 72 * 1024;
 }
 
 }  // namespace

@@ -400,7 +400,7 @@ class HarmGPU:
 
     def autotune(self):
         """hgpu_autotune: pick the resident-block variant of each heavy FP64
-        kernel and the WENO5 tile shape per direction on this state; returns
+        kernel and the WENO5 segment length per direction on this state; returns
         {family: {"minb": chosen, "ms": {candidate: ms}}, "weno_tiles": {dir:
         {"lb": cells, "lines": lines, "ms": per launch}}}."""
         tu = hgpu_tuning()
@@ -416,7 +416,7 @@ class HarmGPU:
 
     def set_tuning(self, minb):
         """hgpu_set_tuning: {"flux": 4, "weno": 3, "update": 3, "invert": 1} (blocks per SM), optionally
-        "weno_tiles": {dir: (cells per tile, lines per tile)}."""
+        "weno_tiles": {dir: (cells per segment, lines)}."""
         tu = hgpu_tuning()
         tu.flux_minb, tu.weno_minb = int(minb["flux"]), int(minb["weno"])
         tu.update_minb, tu.invert_minb = int(minb["update"]), int(minb["invert"])

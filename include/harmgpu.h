@@ -283,11 +283,12 @@ typedef struct {
   int flux_minb, weno_minb, update_minb, invert_minb;
   int flux_cand[2], weno_cand[2], update_cand[2], invert_cand[2];
   float flux_ms[2], weno_ms[2], update_ms[2], invert_ms[2];
-  /* WENO5 tile shape per direction d = 1..3 (index 0 unused): output cells
-     per tile along the direction and lines per tile (a power of two); the
-     autotuner times up to four candidate shapes of its cost model per
-     direction (weno_tile_ms: the chosen one's time per launch).  In
-     hgpu_set_tuning, 0 keeps the current shape. */
+  /* WENO5 segments per direction d = 1..3 (index 0 unused): output cells per
+     segment of a line; the autotuner times up to four candidates of its cost
+     model per direction (weno_tile_ms: the chosen one's time per launch).  In
+     hgpu_set_tuning, weno_lb 0 keeps the current length.  weno_lines: a power
+     of two with weno_lb x weno_lines within the bounds of a tile of lines; it
+     no longer changes the work (segments fill the warps by themselves). */
   int weno_lb[4], weno_lines[4];
   float weno_tile_ms[4];
 } hgpu_tuning;
