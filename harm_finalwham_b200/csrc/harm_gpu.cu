@@ -13,21 +13,24 @@
 //   weno5_kernel<dir> WENO5 line reconstruction (interpline.c:517-678), one
 //                     kernel per direction, a thread per segment of a line
 //                     and primitive (lim = WENO5 only; weno5.cuh, common.cuh)
-//   flux_kernel<dir>  fluxcalc_standard (flux.c:469-680) fused with the
-//                     MC/PARA reconstruction (or reading the WENO5 face
-//                     values), both Riemann states, vchar, HLL/LaxF, the gdet
-//                     strip of flux_ct and the dt-min (common.cuh; the FP32
+//   fluxes_kernel     fluxcalc_standard (flux.c:469-680) of every direction,
+//                     fused with the MC/PARA reconstruction, both Riemann
+//                     states, vchar, HLL/LaxF, the gdet strip of flux_ct and
+//                     the dt-min; flux_kernel<dir> the same per direction
+//                     from the WENO5 face values (common.cuh; the FP32
 //                     instances of the mixed path are built in flux_f32.cu)
 //   emf_kernel        corner EMFs of flux_ct (fluxct.c:148-218)
 //   conserve_kernel   advance_standard zone loop (advance.c:143-213): U(pi),
 //                     source_conn, flux divergence (B fluxes rebuilt from the
 //                     EMFs, fluxct.c:724-781), dUtoU
 //   invert_kernel     Utoprimgen and, on the final substep, fixup1zone
-//   bound kernels     bound_prim (bounds.fishmon.c:29-345)
+//   bound_kernel      bound_prim (bounds.fishmon.c:29-345) and bound_pflag; at
+//                     the end of a step also the ndt combine (advance.c:231)
+//                     and the dt update (step_ch.c:236-247)
 //   fixup kernels     post_fixup (fixup.c:37-96) in an order-independent
 //                     formulation that reproduces the reference's sequential
-//                     sweep exactly (see checksol_resolve / fixup_compute)
-//   finalize_kernel   ndt combine (advance.c:231) and dt update (step_ch.c:236-247)
+//                     sweep exactly (see checksol_resolve / fixup_compute),
+//                     for small domains in one cluster (fixup_small_kernel)
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdio.h>
@@ -738,7 +741,7 @@ __device__ __forceinline__ void inflow_check_x1(const Dims &d, const Params &P, 
 // u^mu, metptomet to Kerr-Schild u^r, transforms.c:51-84, 310-328), carried
 // unchanged to the ghost (interpn of order 1), then the ghost's primitives
 // (bondi_generate_solution, bounds.c:839-888).  Runs before
-// bound_ghost_kernel, which takes these zones as the sources of the x2/x3
+// bound_kernel, which takes these zones as the sources of the x2/x3
 // ghost corners.
 __device__ __forceinline__ void mat4_vec(const double *M, const double *u, double *out) {
 #pragma unroll

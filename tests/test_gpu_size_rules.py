@@ -64,6 +64,7 @@ def test_an_autotuned_choice_can_be_set_again(n):
         dom = riemann.domain(riemann.RiemannProblem(n[0], 4.0 / 3.0, np.array([1.0, 1, 0, 0, 0, 0.5, 1, 0]),
                                                     np.array([0.1, 0.1, 0, 0, 0, 0.5, -1, 0])), ng=6)
         dom.lim = "WENO5"
+        dom.pflag = np.zeros(dom.p.shape[:3], dtype=np.int32)
     with HarmGPU.from_problem(problem_of(dom)) as g:
         tu = g.autotune()
         g.set_tuning({**{f: tu[f]["minb"] for f in ("flux", "weno", "update", "invert")},
