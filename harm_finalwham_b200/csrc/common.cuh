@@ -789,23 +789,41 @@ __device__ __forceinline__ void bsqflags_zone(long long z, const Dims &d, const 
 // on one another: on a 64x64 grid one direction's 33 blocks take 11 us on 148
 // SMs, all of it latency, so that two directions at once cost the time of
 // one; on large grids the last wave of one direction fills with the next.
+//
+// The finite-volume scheme's faces beyond one zone across the grid feed only
+// the dt minimum and stop after the wave speeds.  They come as boxes of their
+// own: in rows of 34 full and 20 such faces (11 ghosts on 32 zones along x3) a
+// third of every warp waited on the others.
+constexpr int FACE_BOXES = 5;  // the faces with fluxes, and the ring on four sides
+struct FaceBoxes {
+  Box box[FACE_BOXES];
+  unsigned first[FACE_BOXES + 1];  // first block of each box, and the number of blocks
+};
 struct FluxJob {
-  Box box[4];             // faces per direction
+  FaceBoxes faces[4];     // per direction
   unsigned first[5];      // first block of direction 1, 2, 3, of the flags, and the number of blocks
   double *F[4];
   const double *pi;
   unsigned char *bsqf;
 };
+template <int DIR, int RECON, typename T>
+__device__ __forceinline__ void flux_boxes(unsigned block, const Dims &d, const Params &P, const FaceBoxes &B,
+                                           const double *__restrict__ pb, const double *__restrict__ G,
+                                           double *__restrict__ F, Scalars *sc) {
+  int s = 0;
+  while (s < FACE_BOXES - 1 && block >= B.first[s + 1]) s++;
+  flux_block<DIR, RECON, T, T, 0>(block - B.first[s], d, P, B.box[s], pb, nullptr, nullptr, G, F, sc);
+}
 template <int RECON, typename T, int MB = MinBlocks<T>::flux>
 __global__ void __launch_bounds__(128, MB) fluxes_kernel(Dims d, Params P, FluxJob J, const double *__restrict__ pb,
                                                          const double *__restrict__ G, Scalars *sc) {
   const unsigned b = blockIdx.x;
   if (b < J.first[1])
-    flux_block<1, RECON, T, T, 0>(b, d, P, J.box[1], pb, nullptr, nullptr, G, J.F[1], sc);
+    flux_boxes<1, RECON, T>(b, d, P, J.faces[1], pb, G, J.F[1], sc);
   else if (b < J.first[2])
-    flux_block<2, RECON, T, T, 0>(b - J.first[1], d, P, J.box[2], pb, nullptr, nullptr, G, J.F[2], sc);
+    flux_boxes<2, RECON, T>(b - J.first[1], d, P, J.faces[2], pb, G, J.F[2], sc);
   else if (b < J.first[3])
-    flux_block<3, RECON, T, T, 0>(b - J.first[2], d, P, J.box[3], pb, nullptr, nullptr, G, J.F[3], sc);
+    flux_boxes<3, RECON, T>(b - J.first[2], d, P, J.faces[3], pb, G, J.F[3], sc);
   else
     bsqflags_zone((long long)(b - J.first[3]) * blockDim.x + threadIdx.x, d, J.pi, G, J.bsqf, sc);
 }

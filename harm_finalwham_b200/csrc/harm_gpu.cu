@@ -2306,6 +2306,37 @@ static void launch_dir(hgpu_ctx *x, const double *pb) {
          x->F[DIR], x->sc);
 }
 
+// The faces of direction q as boxes: with a ring (the finite-volume scheme's
+// faces beyond one zone across the grid), the inner faces and the ring's four
+// sides, each face in one of them.
+static FaceBoxes face_boxes(const Dims &d, const Box &full, int q, bool ring) {
+  FaceBoxes B;
+  for (Box &b : B.box) b = Box{0, 0, 0, 0, 0, 0};
+  int lo[3] = {full.i0, full.j0, full.k0}, num[3] = {full.ni, full.nj, full.nk};
+  const int n[3] = {d.n1, d.n2, d.n3}, s[3] = {d.s1, d.s2, d.s3};
+  auto box = [&]() { return Box{lo[0], lo[1], lo[2], num[0], num[1], num[2]}; };
+  int at = 1;
+  if (ring)
+    for (int a = 0; a < 3; a++) {
+      if (a == q - 1) continue;
+      // below and above the inner range of direction a, over what the
+      // directions before it have left of the others
+      const int in0 = -s[a], inn = n[a] + 2 * s[a], lo0 = lo[a], num0 = num[a];
+      num[a] = in0 - lo0;
+      B.box[at++] = box();
+      lo[a] = in0 + inn;
+      num[a] = lo0 + num0 - lo[a];
+      B.box[at++] = box();
+      lo[a] = in0;
+      num[a] = inn;
+    }
+  B.box[0] = box();
+  B.first[0] = 0;
+  for (int c = 0; c < FACE_BOXES; c++)
+    B.first[c + 1] = B.first[c] + (B.box[c].size() > 0 ? grid_for(B.box[c].size(), 128) : 0);
+  return B;
+}
+
 // bsq: also the b^2 flags of the step's state (pre_fixup of the last stage)
 template <typename TW, typename TF, int FMB, int BMB, int MIX = 0>
 static void launch_fluxes_t(hgpu_ctx *x, const double *pb, bool bsq) {
@@ -2325,9 +2356,9 @@ static void launch_fluxes_t(hgpu_ctx *x, const double *pb, bool bsq) {
   const int n[4] = {0, d.n1, d.n2, d.n3};
   J.first[0] = 0;
   for (int q = 1; q <= 3; q++) {
-    J.box[q] = x->face_box[q];
+    J.faces[q] = face_boxes(d, x->face_box[q], q, x->P.fvring != 0);
     J.F[q] = x->F[q];
-    J.first[q] = J.first[q - 1] + (n[q] > 1 ? grid_for(x->face_box[q].size(), 128) : 0);
+    J.first[q] = J.first[q - 1] + (n[q] > 1 ? J.faces[q].first[FACE_BOXES] : 0);
   }
   J.first[4] = J.first[3] + (bsq ? grid_for(d.nz, 128) : 0);
   J.pi = x->p;
