@@ -473,6 +473,10 @@ __device__ __forceinline__ int code_of<double>(const double *y, const double *) 
       ((-times_sign(df_m1, h1) > norm && fabs(df_m1 + df1) > 0.25 * (fabs(df_m1) + fabs(df1))) ||
        (-times_sign(df0, h1) > norm && fabs(df0 + df1) > 0.25 * (fabs(df0) + fabs(df1)))))
     return kCusp;
+  // (mono's estimates are capped at 1e50 against 1e-13 of the sum, and its
+  // products overflow from 2^508 on: lines above 2^200, infinities and NaN
+  // among them, stay with its plain form)
+  if (hi_word(sum) >= (uint32_t)(1023 + 200) << 20) return kBlend;
   // (estimates that both outer differences must agree with cannot agree with
   // two of opposite sign)
   const uint32_t dl = hi_word(df_m1), dr = hi_word(df2);
@@ -661,6 +665,10 @@ __device__ __forceinline__ void face_values<double>(int code, const double *u, c
                     r1 * ((s18 + q38) + p34);
   *yl = vl + vl2;
   *yr = vr + vr2;
+  // (the reference leaves out a stencil whose weight is 0, which a product
+  // with an infinity or NaN does not)
+  const uint32_t m = 0x7fffffffu;
+  ok = ok && max(hi_word(*yl) & m, hi_word(*yr) & m) < 0x7ff00000u;
   if (!ok) {
     const Pair f = faces_cold(code, u[-2], u[-1], u[0], u[1], u[2], w[0], w[1], w[2], lof);
     *yl = f.a;
