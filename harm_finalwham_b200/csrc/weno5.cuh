@@ -623,6 +623,11 @@ __device__ __forceinline__ void face_values<double>(int code, const double *u, c
   double vl2 = 0.0, vr2 = 0.0;
   if (0.0 < lof) {
     const double f = 1. - lof;
+    // (the plain routine leaves out a stencil of weight 0, which a product
+    // with an infinity, a NaN or a sum that overflows does not)
+    const uint32_t m = 0x7fffffffu;
+    ok = ok && max(max(max(hi_word(u[-2]) & m, hi_word(u[2]) & m), max(hi_word(dm) & m, hi_word(dp) & m)),
+                   hi_word(d0) & m) < (uint32_t)(1023 + 1000) << 20;
     l0 *= f;
     l1 *= f;
     l2 *= f;
@@ -665,10 +670,6 @@ __device__ __forceinline__ void face_values<double>(int code, const double *u, c
                     r1 * ((s18 + q38) + p34);
   *yl = vl + vl2;
   *yr = vr + vr2;
-  // (the reference leaves out a stencil whose weight is 0, which a product
-  // with an infinity or NaN does not)
-  const uint32_t m = 0x7fffffffu;
-  ok = ok && max(hi_word(*yl) & m, hi_word(*yr) & m) < 0x7ff00000u;
   if (!ok) {
     const Pair f = faces_cold(code, u[-2], u[-1], u[0], u[1], u[2], w[0], w[1], w[2], lof);
     *yl = f.a;
