@@ -142,6 +142,20 @@ __device__ __forceinline__ void load_metric(const double *__restrict__ G, const 
   load_metric_t(G, d, ij, slot, m);
 }
 
+// poison() of a state at a location
+template <typename T>
+__device__ __forceinline__ unsigned poison_at(const T *pr, const double *G, long long nij, long long ij, int slot) {
+  Dims d;
+  d.nij = nij;
+  MetricT<T> m;
+  load_metric_t(G, d, ij, slot, m);
+  StateT<T> q;
+  EMT<T> e;
+  get_state(pr, m, q);
+  em_prepare<0>(pr, m, q, e);
+  return poison(pr, q, e);
+}
+
 __device__ __forceinline__ void load_prim(const double *__restrict__ P, const Dims &d, long long z, double *pr) {
 #pragma unroll
   for (int v = 0; v < NPR; v++) pr[v] = P[(long long)v * d.nz + z];
@@ -592,6 +606,65 @@ __global__ void __launch_bounds__(W5_THREADS, MB) weno5_kernel(Dims d, W5Tile tl
   copy_wait<0>();
 }
 
+// the two states of face z of direction DIR
+template <int DIR, int RECON, typename T, typename TR>
+__device__ __forceinline__ void face_states(int lim, long long nz, long long z, long long o, const double *__restrict__ pb,
+                                            const TR *__restrict__ pL, const TR *__restrict__ pR, T *p_l, T *p_r) {
+  if (RECON == 1) {
+    // getp2interplr (flux.c:788-808), line-type branch
+#pragma unroll
+    for (int v = 0; v < NPR; v++) {
+      p_l[v] = (T)__ldg(pR + (long long)v * nz + z - o);
+      p_r[v] = (T)__ldg(pL + (long long)v * nz + z);
+    }
+  } else if (RECON == 2) {
+    // PARA: pright of the cell on the left, pleft of the cell on the right
+#pragma unroll
+    for (int v = 0; v < NPR; v++) {
+      const double *q = pb + (long long)v * nz + z;
+      T y[6];
+#pragma unroll
+      for (int l = 0; l < 6; l++) y[l] = (T)__ldg(q + (l - 3) * o);
+      T dummy;
+      para4(y + 2, &dummy, &p_l[v]);
+      para4(y + 3, &p_r[v], &dummy);
+    }
+  } else {
+#pragma unroll
+    for (int v = 0; v < NPR; v++) {
+      const double *q = pb + (long long)v * nz + z;
+      T ym2 = (T)__ldg(q - 2 * o), ym1 = (T)__ldg(q - o), y0 = (T)__ldg(q), yp1 = (T)__ldg(q + o);
+      T dqm = slope3(lim, ym2, ym1, y0);
+      T dq0 = slope3(lim, ym1, y0, yp1);
+      // getp2interplr (flux.c:788-808)
+      p_l[v] = ym1 + T(0.5) * dqm;
+      p_r[v] = y0 - T(0.5) * dq0;
+    }
+  }
+  // BDIRCONT (flux.c:629-633)
+  p_l[B1 + DIR - 1] = p_r[B1 + DIR - 1] = T(0.5) * (p_l[B1 + DIR - 1] + p_r[B1 + DIR - 1]);
+}
+
+// A stored flux that is not finite: the components that a NaN product of
+// either state reaches.  Out of line and from the states' sources: few faces
+// come here, and what the products need, kept beside two states, cost the
+// Riemann kernels 400 B of spills a thread.
+template <int DIR, int RECON, typename T, typename TR>
+static __device__ __noinline__ void poison_face(int lim, long long nz, long long z, long long o, const double *pb,
+                                                const TR *pL, const TR *pR, const double *G, long long nij, long long ij,
+                                                double *F) {
+  T p_l[NPR], p_r[NPR], nans[NPR] = {};
+  face_states<DIR, RECON>(lim, nz, z, o, pb, pL, pR, p_l, p_r);
+  const unsigned l = poison_at(p_l, G, nij, ij, DIR - 1), r = poison_at(p_r, G, nij, ij, DIR - 1);
+  put_poison(l, DIR, nans);
+  put_poison(l, 0, nans);
+  put_poison(r, DIR, nans);
+  put_poison(r, 0, nans);
+#pragma unroll
+  for (int v = UU; v <= U3; v++)
+    if (nans[v] != T(0.)) F[(long long)v * nz + z] = NAN;
+}
+
 // ---------------------------------------------------------------------------
 // face flux kernel (one per direction); RECON 0: MC-type slopes in the
 // kernel, RECON 1: Riemann states from the WENO5 face values pL/pR (stored
@@ -612,45 +685,14 @@ __device__ __forceinline__ void flux_block(unsigned block, const Dims &d, const 
   long long t = (long long)block * blockDim.x + threadIdx.x;
   bool active = t < box.size();
   double dtij = 0.0;
+  bool bad = false;
   if (active) {
     int i, j, k;
     box_ijk(box, t, i, j, k);
     long long z = zix(d, i, j, k);
     const long long o = dir_stride<DIR>(d);
     T p_l[NPR], p_r[NPR];
-    if (RECON == 1) {
-      // getp2interplr (flux.c:788-808), line-type branch
-#pragma unroll
-      for (int v = 0; v < NPR; v++) {
-        p_l[v] = (T)__ldg(pR + (long long)v * d.nz + z - o);
-        p_r[v] = (T)__ldg(pL + (long long)v * d.nz + z);
-      }
-    } else if (RECON == 2) {
-      // PARA: pright of the cell on the left, pleft of the cell on the right
-#pragma unroll
-      for (int v = 0; v < NPR; v++) {
-        const double *q = pb + (long long)v * d.nz + z;
-        T y[6];
-#pragma unroll
-        for (int l = 0; l < 6; l++) y[l] = (T)__ldg(q + (l - 3) * o);
-        T dummy;
-        para4(y + 2, &dummy, &p_l[v]);
-        para4(y + 3, &p_r[v], &dummy);
-      }
-    } else {
-#pragma unroll
-      for (int v = 0; v < NPR; v++) {
-        const double *q = pb + (long long)v * d.nz + z;
-        T ym2 = (T)__ldg(q - 2 * o), ym1 = (T)__ldg(q - o), y0 = (T)__ldg(q), yp1 = (T)__ldg(q + o);
-        T dqm = slope3(P.lim, ym2, ym1, y0);
-        T dq0 = slope3(P.lim, ym1, y0, yp1);
-        // getp2interplr (flux.c:788-808)
-        p_l[v] = ym1 + T(0.5) * dqm;
-        p_r[v] = y0 - T(0.5) * dq0;
-      }
-    }
-    // BDIRCONT (flux.c:629-633)
-    p_l[B1 + DIR - 1] = p_r[B1 + DIR - 1] = T(0.5) * (p_l[B1 + DIR - 1] + p_r[B1 + DIR - 1]);
+    face_states<DIR, RECON>(P.lim, d.nz, z, o, pb, pL, pR, p_l, p_r);
     MetricT<T> m;
     load_metric_t(G, d, gix(d, i, j), DIR - 1, m);
     int b = P.cell_inst ? P.cell_inst[z] : -1;
@@ -716,6 +758,7 @@ __device__ __forceinline__ void flux_block(unsigned block, const Dims &d, const 
       Fo[B2] = Fs[1];
       Fo[B3] = Fs[2];
       store_prim(F, d, z, Fo);
+      bad = not_finite(Fo[UU + DIR]);
     }
     double dxd = (DIR == 1) ? P.dx1 : ((DIR == 2) ? P.dx2 : P.dx3);
     if (b >= 0) {
@@ -734,6 +777,11 @@ __device__ __forceinline__ void flux_block(unsigned block, const Dims &d, const 
     }
   }
   warp_min_atomic(&sc->ndtbits[DIR], dtij, active);
+  if (bad) {
+    int i, j, k;
+    box_ijk(box, t, i, j, k);
+    poison_face<DIR, RECON, T>(P.lim, d.nz, zix(d, i, j, k), dir_stride<DIR>(d), pb, pL, pR, G, d.nij, gix(d, i, j), F);
+  }
 }
 
 template <int DIR, int RECON, typename T, int MB = MinBlocks<T>::flux, typename TR = T, int MIX = 0>

@@ -118,6 +118,10 @@ __device__ __forceinline__ void derive_metric(Metric &m) {
   m.rg = kept_rcp(m.g);
 }
 
+// whether x is an infinity or NaN
+__device__ __forceinline__ bool not_finite(double x) { return (hi_word(x) & 0x7fffffffu) >= 0x7ff00000u; }
+__device__ __forceinline__ bool not_finite(float x) { return !(fabs(x) <= 3.402823466e38f); }
+
 template <typename T>
 __device__ __forceinline__ T dot4(const T *a, const T *b) {
   return a[0] * b[0] + a[1] * b[1] + a[2] * b[2] + a[3] * b[3];
@@ -294,6 +298,35 @@ __device__ __forceinline__ void mhd_row(const T *pr, int dir, T gam, const State
   TEM[dir] -= T(0.25) * e.Msq;
 #pragma unroll
   for (int j = 0; j < 4; j++) mhd[j] += TEM[j];
+}
+
+// In the reference the products left out above are 0 times a pressure or a
+// tensor component, which is NaN where that is not finite; such a state has to
+// fail as it does there.  Then Msq or the pressure is not finite either, and
+// with it every T^mu_mu, which is where callers look.  poison: which products
+// are NaN, bits 0-5 by Mcov and 6-11 by Mcon (the pairs as em_prepare's sums
+// list them), 12 the pressure, 13 a diagonal B^j u^j - B^j u^j, which every
+// component takes in.  put_poison: into row dir of a flux.  (The induction
+// flux's own component is left 0: flux-CT replaces it unread.)
+__device__ constexpr int em_pair(int j, int k) { return j * k == 0 ? j + k - 1 : (j * k == 2 ? 3 : (j * k == 6 ? 4 : 5)); }
+template <typename T>
+__device__ __forceinline__ unsigned poison(const T *pr, const StateT<T> &q, const EMT<T> &e) {
+  unsigned n = (unsigned)not_finite(pr[UU]) << 12;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    if (j > 0) n |= (unsigned)not_finite(pr[B1 + j - 1] * q.ucon[j]) << 13;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (j != k)
+        n |= (unsigned)not_finite(e.Mcov[j][k]) << em_pair(j, k) | (unsigned)not_finite(e.Mcon[j][k]) << (6 + em_pair(j, k));
+  }
+  return n;
+}
+template <typename T>
+__device__ __forceinline__ void put_poison(unsigned n, int dir, T *flux) {
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+    if (n >> 13 || (j != dir && (n >> 12 || n >> em_pair(j, dir) & 0x41u))) flux[UU + j] = T(NAN);
 }
 
 // primtoflux (phys.c:16-55), UEVOLVE, every EOM factor = gdet

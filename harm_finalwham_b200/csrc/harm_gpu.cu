@@ -211,6 +211,7 @@ __device__ __forceinline__ void fv_diag_fixup(const double *pr0, const double *p
     }
     em_prepare<0>(pr0, m, q, e);
     primtoflux<0>(pr0, q, e, m, gam, Ui);
+    if (not_finite(Ui[UU])) put_poison(poison(pr0, q, e), 0, Ui);
   }
   {
     State q;
@@ -221,6 +222,7 @@ __device__ __forceinline__ void fv_diag_fixup(const double *pr0, const double *p
     }
     em_prepare<0>(pr, m, q, e);
     primtoflux<0>(pr, q, e, m, gam, Uf);
+    if (not_finite(Uf[UU])) put_poison(poison(pr, q, e), 0, Uf);
   }
 #pragma unroll
   for (int pl = 0; pl < NPR; pl++) {
@@ -256,6 +258,7 @@ __global__ void pi2u_kernel(Dims d, Params P, const double *__restrict__ p, cons
   }
   em_prepare<0>(pr, m, q, e);
   primtoflux<0>(pr, q, e, m, P.gam, U);
+  if (not_finite(U[UU])) put_poison(poison(pr, q, e), 0, U);
 #pragma unroll
   for (int pl = 0; pl < NPR; pl++) u[pl * d.nz + z] = U[pl];
 }
@@ -292,6 +295,28 @@ __device__ __forceinline__ void source_conn(C conn, const double *pbz, const Sta
   double full[NPR] = {0., dUconn[0], dUconn[1], dUconn[2], dUconn[3], 0., 0., 0.};
 #pragma unroll
   for (int pl = 0; pl < NPR; pl++) dUg[pl] = (pl >= UU && pl <= U3) ? 0. + m.g * full[pl] : 0.;
+}
+
+// The update's stores of a zone that is not finite: NaN components of U(pi)
+// (pi null: the finite-volume scheme keeps its own) and of the source, whose
+// every component takes in every element of T.  Out of line, as poison_face.
+static __device__ __noinline__ void poison_zone(long long nz, long long z, const double *pi, const double *pb,
+                                                const double *G, long long nij, long long ij, double *uf, double *ucum) {
+  double pr[NPR], nans[NPR] = {};
+  if (pi) {
+#pragma unroll
+    for (int v = 0; v < NPR; v++) pr[v] = pi[v * nz + z];
+    put_poison(poison_at(pr, G, nij, ij, G_CENT), 0, nans);
+  }
+#pragma unroll
+  for (int v = 0; v < NPR; v++) pr[v] = pb[v * nz + z];
+  const bool source = poison_at(pr, G, nij, ij, G_CENT) != 0;
+#pragma unroll
+  for (int v = UU; v <= U3; v++)
+    if (source || nans[v] != 0.) {
+      if (uf) uf[v * nz + z] = NAN;
+      ucum[v * nz + z] = NAN;
+    }
 }
 
 // What the update reads of one (i, j), in the order in which STAGE keeps it in
@@ -494,6 +519,12 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
       ucum[pl * nz + z] = Ucum[pl];
     }
     if (err) atomicOr(&sc->err, err);
+    uint32_t top = 0;
+#pragma unroll
+    for (int pl = 0; pl < NPR; pl++) top = max(top, hi_word(Uf[pl]) & 0x7fffffffu);
+    if (top >= 0x7ff00000u) {
+      poison_zone(nz, z, fv ? nullptr : pi, pb, G, d.nij, ij, write_uf ? uf : nullptr, ucum);
+    }
 }
 
 // FV: the finite-volume scheme, whose diag_fixup forms two more conserved
@@ -2960,6 +2991,7 @@ __global__ void __launch_bounds__(DIAG_BLOCK) diag_kernel(Dims d, Params P, Box 
       get_state(pr, m, q);
       em_prepare<0>(pr, m, q, e);
       primtoflux<0>(pr, q, e, m, P.gam, U);
+      if (not_finite(U[UU])) put_poison(poison(pr, q, e), 0, U);
     }
     double dV = P.dx1 * P.dx2 * P.dx3;
 #pragma unroll

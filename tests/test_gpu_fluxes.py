@@ -3,7 +3,8 @@ the update reads, and the three dt estimates, bit for bit (up to the sign of
 zero).  The states reach what the torus's flow rarely does: jumps in every
 primitive, constant stretches, exact zeros, and fields from 1e-30 down into
 the denormals, where shared reciprocals and the indicators read from
-exponents give way to the plain expressions.  WENO5 runs with segments of
+exponents give way to the plain expressions, and infinities, whose products
+with zeros the kernels leave out.  WENO5 runs with segments of
 many lengths: one cell, remainders, a whole line."""
 import numpy as np
 import pytest
@@ -34,12 +35,18 @@ def draw(pr, kind, seed):
         pr.p[...] = pr.p[:1, :1, :1]
         pr.p[pr.p.shape[0] // 2:, ..., 0] *= 1.0 + 1e-13
         pr.p[:, pr.p.shape[1] // 2:, :, 1] *= 1.0 + 3e-13
+    if kind == "odd":
+        # states whose fluxes are not finite though their wave speeds are
+        at = rng.random(pr.p.shape[:3])
+        pr.p[at < 0.02, 1] = -np.inf
+        for v in (5, 6, 7):
+            pr.p[(at > 0.96 + 0.01 * (v - 4)) & (at < 0.965 + 0.01 * (v - 4)), v] = 1e308
     pr.p = np.ascontiguousarray(pr.p)
 
 
-def check(pr, tiles=None):
+def check(pr, tiles=None, errors=(0,)):
     err, F, ndt = Oracle().fluxcalc(pr)
-    assert err == 0
+    assert err in errors
     with HarmGPU.from_problem(pr) as g:
         if tiles:
             g.set_tuning({"flux": 4, "weno": 3, "update": 3, "invert": 1,
@@ -62,6 +69,15 @@ def test_fluxes_of_drawn_states_match_oracle(n, lim, flux, kind):
     pr = problem_of(dom)
     draw(pr, kind, 1)
     check(pr)
+
+
+@pytest.mark.parametrize("lim,flux", [("WENO5", "HLL"), ("MC", "HLL"), ("PARA", "LAXF")])
+@pytest.mark.parametrize("n", [(19, 13, 11), (24, 17, 1)])
+def test_fluxes_that_are_not_finite_match_oracle(n, lim, flux):
+    dom = torus.fm_torus(*n, ng=6, lim=lim, flux=flux, seed=3)
+    pr = problem_of(dom)
+    draw(pr, "odd", 1)
+    check(pr, errors=(0, 32))  # 32: a wave speed that is not finite
 
 
 @pytest.mark.parametrize("lb", [1, 2, 7, 8, 9, 64])
