@@ -103,6 +103,7 @@ struct Scalars {
   int nsteps;                      // time steps taken since the last upload
   unsigned long long nfloor;       // zone floorings by fixup1zone (summed over a call's final substeps)
   unsigned int blocks_done;        // blocks of a bound kernel that are through (wraps to 0 with the last)
+  int nonfinite;                   // a stage of this call left an infinity or NaN in uf
 };
 
 __device__ __forceinline__ long long zix(const Dims &d, int i, int j, int k) {

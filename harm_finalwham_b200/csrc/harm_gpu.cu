@@ -366,6 +366,10 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
   const long long o1 = (long long)d.nt2 * d.nt3, o2 = d.nt3, o3 = 1;
   const long long ij = gix(d, i, j);
   const double *mine = geo;
+  // (0 times an infinity or NaN of an earlier stage is NaN: the accumulators
+  // are then read although the scheme's weight is 0)
+  const bool nonfinite = timeorder > 0 && sc->nonfinite;
+  const bool take_uf = read_uf || nonfinite, take_ucum = read_ucum || nonfinite;
   if constexpr (STAGE) {
     // (i, j) rows of the box from the block's first zone to its last
     const unsigned first = blockIdx.x * 128u / (unsigned)box.nk;
@@ -380,7 +384,7 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
     for (int v = 0; v < NPR; v++) {
       copy_async(own + v * 128 + threadIdx.x, pb + v * nz + z);
       if (!fv && pi != pb) copy_async(own + (NPR + v) * 128 + threadIdx.x, pi + v * nz + z);
-      if (read_ucum || (fv && timeorder == 0)) copy_async(own + (2 * NPR + v) * 128 + threadIdx.x, ucum + v * nz + z);
+      if (take_ucum || (fv && timeorder == 0)) copy_async(own + (2 * NPR + v) * 128 + threadIdx.x, ucum + v * nz + z);
     }
     copy_commit();
   }
@@ -511,8 +515,8 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
     double Uf[NPR], Ucum[NPR];
 #pragma unroll
     for (int pl = 0; pl < NPR; pl++) {
-      const double ufo = read_uf ? uf[pl * nz + z] : 0.0;
-      const double uco = read_ucum ? (STAGE ? own[(2 * NPR + pl) * 128 + threadIdx.x] : ucum[pl * nz + z]) : 0.0;
+      const double ufo = take_uf ? uf[pl * nz + z] : 0.0;
+      const double uco = take_ucum ? (STAGE ? own[(2 * NPR + pl) * 128 + threadIdx.x] : ucum[pl * nz + z]) : 0.0;
       Uf[pl] = CUf0 * Ui[pl] + CUf1 * ufo + CUf2 * dt * (dUr[pl] + dUg[pl]);
       Ucum[pl] = uco + (Cunew0 * Ui[pl] + Cunew1 * dt * (dUr[pl] + dUg[pl]) + Cunew2 * Uf[pl]);
       if (write_uf) uf[pl * nz + z] = Uf[pl];
@@ -523,6 +527,7 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
 #pragma unroll
     for (int pl = 0; pl < NPR; pl++) top = max(top, hi_word(Uf[pl]) & 0x7fffffffu);
     if (top >= 0x7ff00000u) {
+      if (write_uf) atomicOr(&sc->nonfinite, 1);
       poison_zone(nz, z, fv ? nullptr : pi, pb, G, d.nij, ij, write_uf ? uf : nullptr, ucum);
     }
 }
@@ -671,6 +676,7 @@ __global__ void reset_stage_kernel(Params P, Scalars *sc, int call) {
     sc->nfixed = 0;
     sc->overflow = 0;
     sc->nfloor = 0;
+    sc->nonfinite = 0;
   }
 }
 
@@ -2550,8 +2556,9 @@ static void launch_stage_advance(hgpu_ctx *x, int timeorder, bool folded = false
   const int fv = (x->cfg.doenoflux == HGPU_ENOFINITEVOLUME);
   double *ufv = (fv && finalstep) ? x->ucum : nullptr;
   // ulast and ucum enter a stage only where an earlier one left them other
-  // than zero, and uf is read by later stages and the intermediate inversion
-  // alone: what no one reads is not moved (RK2: 128 of 256 bytes a zone and step)
+  // than zero (or a stage left an infinity or NaN), and uf is read by later
+  // stages and the intermediate inversion alone: neither is moved where no one
+  // reads it.  ucum is stored in every stage.
   bool read_ucum = false;
   for (int o = 0; o < timeorder; o++) {
     const RKStage &E = rk_stage(x, o);

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 from harm_finalwham_b200 import torus
-from harm_finalwham_b200.gpu import HarmGPU
+from harm_finalwham_b200.gpu import HarmGPU, HarmGPUError
 from oracle.pyoracle import Oracle
 from tests.fixtures import same
 from tests.test_gpu_weno5 import problem_of
@@ -78,6 +78,37 @@ def test_fluxes_that_are_not_finite_match_oracle(n, lim, flux):
     pr = problem_of(dom)
     draw(pr, "odd", 1)
     check(pr, errors=(0, 32))  # 32: a wave speed that is not finite
+
+
+@pytest.mark.parametrize("scheme", [{}, {"timeorder": 3}, {"timeorder": 4}, {"timeorder": 4, "doenoflux": "ENOFINITEVOLUME"}])
+@pytest.mark.parametrize("v,value", [(0, 1.7e308), (1, 1e308), (5, np.nan), (7, np.inf)])
+@pytest.mark.parametrize("n", [(24, 17, 1), (12, 9, 33)])
+def test_a_zone_that_failed_in_one_stage_fails_as_the_oracles(n, v, value, scheme):
+    """0 times an infinity or NaN of an earlier stage is NaN: the scheme's
+    zero weights keep the zone failing in the later ones."""
+    dom = torus.fm_torus(*n, ng=6, lim="MC", flux="HLL", seed=3)
+    pr = problem_of(dom)
+    pr.timeorder = scheme.get("timeorder", 2)
+    pr.doenoflux = scheme.get("doenoflux", "NOENOFLUX")
+    pr.p[pr.g[0] + 8, pr.g[1] + 6, pr.g[2] + n[2] // 2, v] = value
+    pr.p = np.ascontiguousarray(pr.p)
+    orc = Oracle()
+    orc.bound_prim(pr)
+    pr.dt = 1e-3
+    q = pr.copy()
+    with HarmGPU.from_problem(pr) as g:
+        if scheme.get("doenoflux"):
+            # the conserved state of the zone itself
+            q.u = orc.pi2u(q)
+        st = orc.step(q, 1)
+        if st.err:
+            with pytest.raises(HarmGPUError):
+                g.step_ch(1)
+            return
+        g.step_ch(1)
+        p, pf, _t, _dt = g.download_state()
+    assert np.count_nonzero(q.pflag) > 0
+    assert same(p, q.p) and np.array_equal(pf, q.pflag)
 
 
 @pytest.mark.parametrize("lb", [1, 2, 7, 8, 9, 64])
