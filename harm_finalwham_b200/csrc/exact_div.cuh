@@ -18,9 +18,9 @@
 //     numbers can come to a middle).  Elsewhere the last rounding decides.
 //     The remainder is taken as b q - a so that a quotient +-0 by a positive
 //     divisor keeps the sign that the division gives.
-// The steps neither overflow nor lose bits to underflow for |b| in
-// [2^-200, 2^200) and a = +-0 or |a| in [2^-700, 2^700); any other operand,
-// infinities and NaN among them, takes the division itself.
+// The steps neither overflow nor lose bits to underflow for b in [2^-200,
+// 2^200) and a = +-0 or |a| in [2^-700, 2^700); any other operand, negative
+// divisors, infinities and NaN among them, takes the division itself.
 #pragma once
 #include <math.h>
 #include <stdint.h>
@@ -87,10 +87,10 @@ HG_HD double quot(double a, double b, double y) {
 // twice the biased exponent word of 2^e (the sign shifted out)
 constexpr uint32_t exp_word2(int e) { return (uint32_t)(1023 + e) << 21; }
 constexpr uint32_t kNumLo = exp_word2(-700), kNumRange = exp_word2(700) - exp_word2(-700);
-constexpr uint32_t kDenLo = exp_word2(-200), kDenRange = exp_word2(200) - exp_word2(-200);
+constexpr uint32_t kDenLo = exp_word2(-200) >> 1, kDenRange = (exp_word2(200) >> 1) - kDenLo;
 
-// whether rcp_rn holds for b
-HG_HD bool rcp_ok(double b) { return (hi_word(b) << 1) - kDenLo < kDenRange && lo_word(b) != 0xffffffffu; }
+// whether rcp_rn holds for b, and quot for it (a sign would leave the range)
+HG_HD bool rcp_ok(double b) { return hi_word(b) - kDenLo < kDenRange && lo_word(b) != 0xffffffffu; }
 
 // A divisor and its reciprocal.  FP32 (the mixed-precision path) divides.
 template <typename T>
