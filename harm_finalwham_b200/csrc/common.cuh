@@ -873,7 +873,7 @@ __global__ void __launch_bounds__(128, MB) fluxes_kernel(Dims d, Params P, FluxJ
     flux_boxes<2, RECON, T>(b - J.first[1], d, P, J.faces[2], pb, G, J.F[2], sc);
   else if (b < J.first[3])
     flux_boxes<3, RECON, T>(b - J.first[2], d, P, J.faces[3], pb, G, J.F[3], sc);
-  else
+  else if constexpr (sizeof(T) == 8)  // (of the FP64 unit; see launch_fluxes_t)
     bsqflags_zone((long long)(b - J.first[3]) * blockDim.x + threadIdx.x, d, J.pi, G, J.bsqf, sc);
 }
 

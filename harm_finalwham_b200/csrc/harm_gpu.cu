@@ -2397,7 +2397,11 @@ static void launch_fluxes_t(hgpu_ctx *x, const double *pb, bool bsq) {
     J.F[q] = x->F[q];
     J.first[q] = J.first[q - 1] + (n[q] > 1 ? J.faces[q].first[FACE_BOXES] : 0);
   }
-  J.first[4] = J.first[3] + (bsq ? grid_for(d.nz, 128) : 0);
+  // (the FP32 instances are built with contraction, which the flags' FP64
+  // arithmetic must not have: a zone at a limit would get another flag)
+  const bool ride = bsq && sizeof(TF) == 8;
+  if (bsq && !ride) LAUNCH(x, K_OTHER, bsqflags_kernel, grid_for(d.nz, 256), 256, d, x->p, x->G, x->bsqf, x->sc);
+  J.first[4] = J.first[3] + (ride ? grid_for(d.nz, 128) : 0);
   J.pi = x->p;
   J.bsqf = x->bsqf;
   if (J.first[4] == 0) return;

@@ -81,3 +81,28 @@ def test_mixed_weno5_within_1e5_of_fp64_at_scale():
           {k: f"{v:.2e}" for k, v in errs.items()})
     assert all(v <= 1e-5 for v in errs.values()), errs
     assert d32 < 1e-12
+
+
+@pytest.mark.parametrize("lim,ng", [("MC", 3), ("PARA", 3), ("WENO5", 6)])
+def test_bsq_flags_do_not_depend_on_the_precision(lim, ng):
+    # zones within a few roundings of b^2/rho = 20 or 18: the flags of a
+    # step's input state are FP64 arithmetic in both modes
+    dom = torus.fm_torus(24, 16, 8, ng=ng, lim=lim, flux="HLL", seed=5)
+    rng = np.random.default_rng(8)
+    dom.p[..., 5:8] += 1e-3 * rng.standard_normal(dom.p.shape[:3] + (3,))
+    nt, cent = dom.p.shape, torus.CENT
+    bsq = torus._bsq(dom.p, dom.gcov[:nt[0], :nt[1], cent][:, :, None], dom.gcon[:nt[0], :nt[1], cent][:, :, None])
+    limit = rng.choice([18.0, 20.0], size=bsq.shape)
+    dom.p[..., 0] = bsq / limit * (1.0 + 2.0 ** -52 * rng.integers(-3, 4, size=bsq.shape))
+    dom.p[..., 1] = 0.1 * dom.p[..., 0]
+    dom.p = np.ascontiguousarray(dom.p)
+    flags = {}
+    for precision in ("fp64", "mixed"):
+        with HarmGPU(*dom.n, dom.ng, dom.dx, lim=lim, flux="HLL", precision=precision, gam=dom.gam, cour=dom.cour) as g:
+            g.upload_geometry(dom.gcov, dom.gcon, dom.gcovpert, dom.gdet, dom.conn, dom.floors)
+            g.upload_state(dom.p, dom.pflag, 0.0, 1e-6)
+            g.step_ch(1)
+            flags[precision] = g.download_bsqflags()
+    counts = [np.count_nonzero(flags["fp64"][..., 0] == v) for v in (0, 1, 2)]
+    assert min(counts) > 100, counts
+    assert np.array_equal(flags["fp64"], flags["mixed"])
