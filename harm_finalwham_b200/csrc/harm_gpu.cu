@@ -1369,17 +1369,8 @@ __device__ __forceinline__ void fixup_compute(const FixJob &J, const Params &P, 
     double gamma = 1.0;
     if (gamma_calc(pr, m, &gamma)) err |= ERR_UTCALC_DISCR;
     if (gamma > P.gammamax) gamma = P.gammamax;
-    int startpl, endpl, looptype;
-    if (mypflag == UTOPRIMFAILU2AVG1 || mypflag == UTOPRIMFAILU2AVG2) {
-      startpl = UU;
-      endpl = UU;
-      looptype = 1;
-    } else {
-      startpl = RHO;
-      endpl = U3;
-      looptype = 0;
-    }
-    double mysum0[5] = {0, 0, 0, 0, 0}, mysum1[5] = {0, 0, 0, 0, 0}, lastmin[5] = {1E50, 1E50, 1E50, 1E50, 1E50};
+    const int looptype = (mypflag == UTOPRIMFAILU2AVG1 || mypflag == UTOPRIMFAILU2AVG2) ? 1 : 0;
+    double mysum0[5] = {0, 0, 0, 0, 0}, mysum1[5] = {0, 0, 0, 0, 0}, lastmin = 1E50;
     const int s1 = d.s1, s2 = d.s2, s3 = d.s3;
     const int rnx = (s1 == 1) ? 3 : 1, rny = (s2 == 1) ? 3 : 1;
     const int npow = s1 + s2 + s3;
@@ -1398,34 +1389,38 @@ __device__ __forceinline__ void fixup_compute(const FixJob &J, const Params &P, 
       int fa = pflag[za], fb = pflag[zb];
       int thisnotfail = (fa <= UTOPRIMNOFAIL) || (act_a && za < z && becomes_fixed(fa, finalstep));
       int thatnotfail = (fb <= UTOPRIMNOFAIL) || (act_b && zb < z && becomes_fixed(fb, finalstep));
-      numavg1 += (pv[(long long)UU * d.nz + za] > 0.0);
-      numavg1 += (pv[(long long)UU * d.nz + zb] > 0.0);
+      const double ua = pv[(long long)UU * d.nz + za], ub = pv[(long long)UU * d.nz + zb];
+      numavg1 += (ua > 0.0);
+      numavg1 += (ub > 0.0);
       numavg0 += thisnotfail + thatnotfail;
-      for (int pl = startpl; pl <= endpl; pl++) {
-        double va = pv[(long long)pl * d.nz + za], vb = pv[(long long)pl * d.nz + zb];
-        if (looptype == 0) {
-          double add = va * thisnotfail + vb * thatnotfail;
+      if (looptype == 0) {
+#pragma unroll
+        for (int pl = RHO; pl <= U3; pl++) {
+          const double va = pv[(long long)pl * d.nz + za], vb = pv[(long long)pl * d.nz + zb];
+          const double add = va * thisnotfail + vb * thatnotfail;
           if (qq % 2) mysum1[pl] += add;
           else mysum0[pl] += add;
-        } else {
-          if (va >= 0.0) lastmin[pl] = min_macro(lastmin[pl], va);
-          if (vb >= 0.0) lastmin[pl] = min_macro(lastmin[pl], vb);
         }
+      } else {
+        if (ua >= 0.0) lastmin = min_macro(lastmin, ua);
+        if (ub >= 0.0) lastmin = min_macro(lastmin, ub);
       }
     }
     int numavg;
     if (looptype == 0) {
       if (numavg0 != 0)
-        for (int pl = startpl; pl <= endpl; pl++) pr[pl] = (mysum0[pl] + mysum1[pl]) / ((double)(numavg0));
+#pragma unroll
+        for (int pl = RHO; pl <= U3; pl++) pr[pl] = (mysum0[pl] + mysum1[pl]) / ((double)(numavg0));
       numavg = numavg0;
     } else {
-      if (numavg1 != 0)
-        for (int pl = startpl; pl <= endpl; pl++) pr[pl] = lastmin[pl];
+      if (numavg1 != 0) pr[UU] = lastmin;
       numavg = numavg1;
     }
     if (mypflag == UTOPRIMFAILU2AVG2) numavg++;
     if (numavg == 0) {
-      for (int pl = startpl; pl <= endpl; pl++) {
+#pragma unroll
+      for (int pl = RHO; pl <= U3; pl++) {
+        if (looptype == 1 && pl != UU) continue;
         const double *pp = pv + (long long)pl * d.nz;
         double a41 = (0.25 * ((pp[zix(d, i, j + s2, k)] + pp[zix(d, i, j - s2, k)]) +
                               (pp[zix(d, i - s1, j, k)] + pp[zix(d, i + s1, j, k)])));
@@ -1494,17 +1489,24 @@ __global__ void fixup_scatter_kernel(FixJob J, Params P) {
 // checksolution from the candidates on and fixup_utoprim in one launch of one
 // cluster, whose hardware barrier stands where the kernels above end: seven
 // launches less a stage (with bound_kernel and the resets 246 -> 168 us a step
-// on 64x64).  Its 4096 threads do for the short lists of a flow; a larger
-// domain takes the kernels, which fill the GPU, and there seven launches are
-// under 1% of the step.  In a batch of strong 1D problems a good part of the
-// zones are candidates (128 problems, 77k zones: 88 ms to t = 0.2 with the
-// cluster, 79 with the kernels), so it has to be smaller by far.
-constexpr int FIX_CLUSTER = 8, FIX_THREADS = 512;
+// on 64x64).  A larger domain takes the kernels, which fill the GPU, and there
+// seven launches are under 1% of the step.
+// What it costs goes by the candidates, which only the device knows: no domain
+// up to the limit may lose more with long lists than with the launches that
+// short ones save.  Hence 16 blocks where the device takes such a cluster (8
+// is what every device of this architecture does).  Us a step, MC, RK2, with 0
+// / 10 / 50% of the zones fast: 16 blocks 586 / 940 / 1199 on 64x64x64, 451 /
+// 646 / 825 on 97x51x33, 221 / 286 / 343 on 256x256; 8 blocks 582 / 1174 /
+// 1695, 452 / 797 / 1137, 220 / 330 / 427; the kernels 631 / 738 / 769, 497 /
+// 586 / 590, 262 / 313 / 311.  Blocks of 1024 threads spill: 586 / 934 / 1161.
+// In a batch of strong 1D problems a good part of the zones are candidates
+// (128 problems, 77k zones: 88 ms to t = 0.2 with a cluster of 8, 79 with the
+// kernels), and there is no quiet flow to weigh them against.
+constexpr int FIX_THREADS = 512;
 constexpr long long kSmallDomain = 1LL << 18, kSmallBatch = 1LL << 13;
-__global__ void __cluster_dims__(FIX_CLUSTER, 1, 1) __launch_bounds__(FIX_THREADS)
-    fixup_small_kernel(FixJob J, Params P) {
+__global__ void __launch_bounds__(FIX_THREADS) fixup_small_kernel(FixJob J, Params P) {
   auto cluster = cooperative_groups::this_cluster();
-  const int a0 = blockIdx.x * FIX_THREADS + threadIdx.x, step = FIX_CLUSTER * FIX_THREADS;
+  const int a0 = blockIdx.x * FIX_THREADS + threadIdx.x, step = gridDim.x * FIX_THREADS;
   const int n = listed(*(volatile int *)&J.sc->ncand, J.cap);
   if (n > 0) {
     checksol_map(J, n, a0, step);
@@ -1772,6 +1774,31 @@ struct ProfEvent {
   cudaEvent_t a, b;
 };
 
+// a launch of fixup_small_kernel as one cluster of so many blocks
+struct FixLaunch {
+  cudaLaunchAttribute cluster;
+  cudaLaunchConfig_t cfg = {};
+  FixLaunch(int blocks, cudaStream_t stream) {
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = blocks;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(FIX_THREADS);
+    cfg.stream = stream;
+    cfg.attrs = &cluster;
+    cfg.numAttrs = 1;
+  }
+};
+// 16 blocks need leave and a device that can place them
+static int fix_cluster_size(cudaStream_t stream) {
+  int n = 0;
+  const FixLaunch l(16, stream);
+  const bool ok = cudaFuncSetAttribute(fixup_small_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&n, fixup_small_kernel, &l.cfg) == cudaSuccess && n > 0;
+  if (!ok) cudaGetLastError();
+  return ok ? 16 : 8;
+}
+
 struct hgpu_ctx {
   long long launches = 0;
   bool profiling = false;
@@ -1809,6 +1836,7 @@ struct hgpu_ctx {
   double *bondi_tab = nullptr;          // Bondi-integral boundaries' coordinate data
   double *progress = nullptr;                          // 4 doubles for hg_progress_async
   W5Tile w5[4];  // WENO5 tiling per direction
+  int fix_cluster = 8;  // blocks of fixup_small_kernel
   Box w5_state_box;  // zones whose dP/P state pieces some direction reads
   Box w5_shock_box;  // zones whose shock factors some direction reads
   int *istaging = nullptr;
@@ -2085,6 +2113,7 @@ int hgpu_create(const hgpu_config *cfg, hgpu_ctx **out) {
   }
   // the staged update hides its spills: 4 blocks, where the direct one takes 3
   x->tune.conserve = x->active_box.nk >= STAGE_MIN_NK ? 1 : 0;
+  x->fix_cluster = fix_cluster_size(x->stream);
   x->P.ffc = x->ffc;
   // post_fixup's lists and scratch live in the flux planes, which are read
   // for the last time by the conserved update before it and written by the
@@ -2592,6 +2621,11 @@ static void launch_stage_advance(hgpu_ctx *x, int timeorder, bool folded = false
   launch_bound(x, pf, true, false, folded && fused_gamma(x));
 }
 
+static void launch_fixup_small(hgpu_ctx *x, const FixJob &J) {
+  ProfScope ps__(x, K_CHECK_RESOLVE);
+  FixLaunch l(x->fix_cluster, x->stream);
+  cudaLaunchKernelEx(&l.cfg, fixup_small_kernel, J, x->P);
+}
 // fixup_checksolution and fixup_utoprim on pf with the context's flags
 static void launch_checksol_fixup(hgpu_ctx *x, double *pf, int finalstep, bool gamma_done = false) {
   const Dims &d = x->d;
@@ -2617,7 +2651,7 @@ static void launch_checksol_fixup(hgpu_ctx *x, double *pf, int finalstep, bool g
     LAUNCH(x, K_CHECK_GAMMA, checksol_gamma_kernel, grid_for(x->dq_box.size(), 128), 128, d, x->P, x->dq_box, gamma_job(x),
            pf, x->G, x->sc, x->pflag);
   if (small_fixup(x)) {
-    LAUNCH(x, K_CHECK_RESOLVE, fixup_small_kernel, FIX_CLUSTER, FIX_THREADS, J, x->P);
+    launch_fixup_small(x, J);
     return;
   }
   // grid-stride over the device-side candidate count; idle blocks exit at once

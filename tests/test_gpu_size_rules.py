@@ -24,16 +24,27 @@ def rough(pr, seed):
     pr.p = np.ascontiguousarray(pr.p)
 
 
-def run(n, ng=3, steps=1, **scheme):
+def boosted(pr, part):
+    """A part of the zones at Lorentz factors above 3, so that the lists of
+    candidates are longer than the cluster that takes them has threads."""
+    fast = np.random.default_rng(9).random(pr.p.shape[:3]) < part
+    g33 = pr.gcov[:pr.p.shape[0], :pr.p.shape[1], torus.CENT, 3, 3]
+    pr.p[..., 4] += fast * 3.0 / np.sqrt(g33)[:, :, None]
+    pr.p = np.ascontiguousarray(pr.p)
+
+
+def run(n, ng=3, steps=1, part=0.0, **scheme):
     dom = torus.fm_torus(*n, ng=ng, lim=scheme.get("lim", "MC"), flux=scheme.get("flux", "HLL"), seed=21)
     pr = problem_of(dom)
     pr.timeorder = scheme.get("timeorder", 2)
     pr.utoprim = scheme.get("utoprim", "2DFINAL")
     pr.doenoflux = scheme.get("doenoflux", "NOENOFLUX")
     rough(pr, 4)
+    if part:
+        boosted(pr, part)
     orc = Oracle()
     orc.bound_prim(pr)
-    pr.dt = 1e-3
+    pr.dt = 1e-5 if part else 1e-3
     q = pr.copy()
     with HarmGPU.from_problem(pr) as g:
         st = g.step_ch(steps)
@@ -54,6 +65,13 @@ def test_update_with_long_and_short_x3(n3, scheme):
 @pytest.mark.parametrize("n", [(63, 50, 63), (65, 49, 63), (66, 63, 63), (64, 64, 64), (65, 64, 64)])
 def test_domains_around_the_size_limits(n):
     assert run(n).nfixed > 0
+
+
+@pytest.mark.parametrize("part", [0.1, 0.5, 1.0])
+@pytest.mark.parametrize("n", [(63, 50, 33), (200, 180, 1)])
+def test_long_lists_in_one_cluster(n, part):
+    st = run(n, part=part)
+    assert part == 1.0 or st.nfixed > 2000
 
 
 @pytest.mark.parametrize("n", [(300, 1, 1), (90, 20, 1), (40, 9, 33)])
