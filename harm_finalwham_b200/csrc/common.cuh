@@ -313,7 +313,9 @@ template <> struct MinBlocks<float> {
 constexpr int kFluxMB[2] = {HG_MINB_FLUX, HG_MINB_FLUX - 1};
 constexpr int kWenoMB[2] = {HG_MINB_WENO, HG_MINB_WENO - 1};
 constexpr int kConserveMB[2] = {HG_MINB_UPDATE, HG_MINB_UPDATE + 1};
-// (1 and 2 name the inversion's variants for hgpu_tuning; they ask for 4 and 3 blocks)
+// (1 and 2 name the inversion's variants for hgpu_tuning: as many blocks as its
+// registers were cut for, 4 or, with Jon's inverter or the finite-volume scheme,
+// 3, and one less)
 constexpr int kInvertMB[2] = {HG_MINB_INVERT, 2};
 
 template <int DIR>

@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(128, MB) conserve_kernel(
 // ms a launch on 256x128x128.  With it, 3 blocks spill 140 B in the branch
 // of the floored zones: 83 -> 58 us a launch on 128x64x32 (RK4, Jon).
 template <int UV, int MB, bool FV>
-__global__ void __launch_bounds__(128, FV || UV == 8 || MB == 2 ? 3 : 4) invert_kernel(Dims d, Params P, Box box, const double *pb,
+__global__ void __launch_bounds__(128, (FV || UV == 8 ? 3 : 4) - (MB == 2)) invert_kernel(Dims d, Params P, Box box, const double *pb,
                                                                      double *pf, const double *__restrict__ uf,
                                                                      const double *__restrict__ ucum,
                                                                      const double *__restrict__ G,

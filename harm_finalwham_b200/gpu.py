@@ -415,8 +415,9 @@ class HarmGPU:
         return out
 
     def set_tuning(self, minb):
-        """hgpu_set_tuning: {"flux": 4, "weno": 3, "update": 3, "invert": 1} (blocks per SM), optionally
-        "weno_tiles": {dir: (cells per segment, lines)}."""
+        """hgpu_set_tuning: {"flux": 4 or 3, "weno": 4 or 3, "update": 3 or 4, "invert": 1 or 2} (blocks per SM; for
+        invert a name), optionally "weno_tiles": {dir: (cells per segment, lines)}.  A new context has 4, 4, 1 and
+        an update of 4 with 32 or more zones along x3, else 3: there the other value is the slower one."""
         tu = hgpu_tuning()
         tu.flux_minb, tu.weno_minb = int(minb["flux"]), int(minb["weno"])
         tu.update_minb, tu.invert_minb = int(minb["update"]), int(minb["invert"])

@@ -273,7 +273,9 @@ int hgpu_step_graph(hgpu_ctx *ctx, int nsteps, hgpu_stats *stats);
 /* Autotuner (no counterpart in the reference): for the FP64 flux, WENO5
    reconstruction, update and inversion kernels, times two resident-blocks-per-SM variants
    (registers per thread vs warps per SM) on this context's own state and
-   keeps the faster for later steps.  Results do not depend on the choice;
+   keeps the faster for later steps.  (The values are the blocks asked for, but
+   for invert, whose 1 and 2 name the two variants: 4 and 3 blocks, 3 and 2
+   with Jon's inverter or the finite-volume scheme.)  Results do not depend on the choice;
    the state is left as it was (for a batch context, every instance's t,
    dt, done flag and step count too).  *_ms: kernel milliseconds of one step per
    candidate (0 where a family does not apply: weno without WENO5; in the
