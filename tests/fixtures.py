@@ -1,12 +1,13 @@
 """Load the committed golden fixtures (tests/golden/*.npz) into oracle Problems,
 and summarise states into the compact records kept for the configurations
 too large to store whole (tests/golden/records/*.npz)."""
+import glob
 import hashlib
 import os
 
 import numpy as np
 
-from oracle.pyoracle import Problem
+from oracle.pyoracle import LIBDIR, Problem
 
 GOLDEN = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden")
 CASES = ["torus2d_16x16_mc_hll", "torus3d_12x12x6_mc_laxf", "torus2d_16x16_weno5_hll", "torus3d_12x12x6_weno5_laxf",
@@ -15,6 +16,18 @@ CASES = ["torus2d_16x16_mc_hll", "torus3d_12x12x6_mc_laxf", "torus2d_16x16_weno5
          "torus2d_16x16_para_hll_rk4_jon", "torus3d_12x12x6_weno5_laxf_jon", "torus2d_16x16_para_hll_rk4_jon_fv",
          "torus2d_16x16_mc_hll_fv", "torus3d_12x12x6_para_laxf_rk4_jon_fv", "torus3d_12x12x6_weno5_hll",
          "torus3d_12x12x6_mc_hll", "torus2d_16x16_mc_hll_beta1e-4"]
+
+
+def reference_binary(name):
+    """Path of a binary built from the reference's sources (oracle/_ref).
+    __graft_entry__.build makes all of them or, where the sources are absent,
+    none: then the test is skipped.  One missing among others is a failure."""
+    exe = os.path.join(LIBDIR, name)
+    if not glob.glob(os.path.join(LIBDIR, "harm_*")):
+        import pytest
+        pytest.skip("no reference binaries: the reference's sources were not there when build() ran")
+    assert os.path.exists(exe), f"{exe} is missing: __graft_entry__.build() builds it"
+    return exe
 
 
 def load(name):

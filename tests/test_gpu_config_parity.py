@@ -25,8 +25,8 @@ import numpy as np
 import pytest
 
 from harm_finalwham_b200.gpu import HarmGPU
-from oracle.pyoracle import LIBDIR, RefDump
-from tests.fixtures import load_record, summarise
+from oracle.pyoracle import RefDump
+from tests.fixtures import load_record, reference_binary, summarise
 
 pytestmark = pytest.mark.gpu
 
@@ -47,8 +47,7 @@ CONFIGS = {
 def reference_init(name):
     """Initial state and geometry written by the configuration's reference binary."""
     exe, ng = CONFIGS[name]
-    exe = os.path.join(LIBDIR, exe)
-    assert os.path.exists(exe), f"{exe} is missing: __graft_entry__.build() builds it"
+    exe = reference_binary(exe)
     rec = load_record(name)
     args = str(rec["harness_args"]).split()
     with tempfile.TemporaryDirectory() as tmp:

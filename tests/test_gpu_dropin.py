@@ -17,15 +17,14 @@ import tempfile
 import numpy as np
 import pytest
 
-from oracle.pyoracle import LIBDIR, RefDump
-from tests.fixtures import load, load_record, same
+from oracle.pyoracle import RefDump
+from tests.fixtures import load, load_record, reference_binary, same
 
 pytestmark = pytest.mark.gpu
 
 
 def run_shim(binary, nsteps, dumps, args=()):
-    exe = os.path.join(LIBDIR, binary)
-    assert os.path.exists(exe), f"{exe} is missing: __graft_entry__.build() builds it"
+    exe = reference_binary(binary)
     tmp = tempfile.TemporaryDirectory()
     out = os.path.join(tmp.name, "out")
     r = subprocess.run([exe] + list(args) + [out, str(nsteps)] + [str(d) for d in dumps], cwd=tmp.name,
@@ -89,8 +88,7 @@ def test_reference_bondi_flow_on_gpu_tracks_its_cpu_run():
     # with -DHARMGPU_GENERIC_BOUNDS; pow in the boundaries makes the bar a
     # tolerance (the device's own runs: tests/test_gpu_bondi_bc.py)
     pr, ref = load("bondi2d_16x16_mc_hll")
-    exe = os.path.join(LIBDIR, "harm_bondi_16x16x1_MC_HLL_jon_gpushim")
-    assert os.path.exists(exe), f"{exe} is missing: __graft_entry__.build() builds it"
+    exe = reference_binary("harm_bondi_16x16x1_MC_HLL_jon_gpushim")
     steps = sorted(ref)
     with tempfile.TemporaryDirectory() as tmp:
         with open(os.path.join(tmp, "bondigrid16.dat"), "wb") as f:
