@@ -524,7 +524,8 @@ def bench_ours(args, rank, world):
     dom_k = max(ktimes, key=lambda k: ktimes[k]["ms"])
     kt = ktimes[dom_k]
     avg_s = kt["ms"] / kt["launches"] / 1e3
-    alg = algorithmic_bytes(dom_k, n1, n2, n3, lim, tx=dom.ng if sc["doenoflux"] == "ENOFINITEVOLUME" else 1)
+    alg = algorithmic_bytes(dom_k, n1, n2, n3, lim, tx=dom.ng if sc["doenoflux"] == "ENOFINITEVOLUME" else 1,
+                            timeorder=sc["timeorder"], fv=sc["doenoflux"] == "ENOFINITEVOLUME")
     peaks, peaks_kind = measured_peaks()
     achieved = alg / avg_s / 1e9
     roof = {"kernel": dom_k, "bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
@@ -536,11 +537,12 @@ def bench_ours(args, rank, world):
     if fp64:
         roof["fp64"] = fp64
     # the whole step against the path's compulsory bytes: 392 B per
-    # zone-update (2 substeps x [read p_b 64 + read p^n 64 + write p_f 64 +
-    # pflag 4], state resident, metric per (i,j) amortised over x3), beside
-    # the DRAM bytes ncu counted for one step
+    # zone-update with RK2 (per substep read p_b 64 + read p^n 64 + write p_f
+    # 64 + pflag 4; state resident, metric per (i,j) amortised over x3; the
+    # finite-volume scheme's conserved state too), beside the DRAM bytes ncu
+    # counted for one step
     step_s = ms_max / args.steps / 1e3
-    step_alg = 392.0 * zones
+    step_alg = zones * sc["timeorder"] * (196.0 + (64.0 if sc["doenoflux"] == "ENOFINITEVOLUME" else 0.0))
     sdb = step_dram_bytes(args.workload)
     roof["step"] = {"algorithmic_bytes": step_alg, "achieved_gbs": step_alg / step_s / 1e9,
                     "frac": step_alg / step_s / 1e9 / peaks["hbm_gbs"], "dram_bytes_ncu": sdb,
@@ -793,7 +795,26 @@ def bench_serving(count=64, mean_gap_ms=2.0, seed=11, budget_bytes=32e9, max_act
                     "graph" % mean_gap_ms}
 
 
-def algorithmic_bytes(kernel, n1, n2, n3, lim="MC", tx=1):
+# per stage of each time order: whether uf's and ucum's old values enter it
+# (step_ch.c:442-562's weights of ulast, and of what earlier stages left in
+# ucum, that are not 0)
+RK_READS = {1: [(0, 0)], 2: [(0, 0), (0, 0)], 3: [(0, 0), (1, 0), (1, 0)], 4: [(0, 0), (0, 1), (0, 1), (0, 1)]}
+
+
+def update_bytes(ndim, timeorder, fv):
+    """Bytes a zone that the conserved update moves, mean over the stages: the
+    fluxes' five hydrodynamic components per direction, the EMFs, p_b, U's
+    source (p^n where it is another state; the stored U with the
+    finite-volume scheme), the accumulators."""
+    total = 0
+    for s, (uf, ucum) in enumerate(RK_READS[timeorder]):
+        total += 40 * ndim + 24 + 64 + 64 * (s > 0) + 64 * (uf + ucum)
+        total += 64 + 64 * (s < timeorder - 1)      # ucum; uf but for the last stage
+        total += 128 * (fv and s == 0)              # the stored U comes from ucum and is kept
+    return total / timeorder
+
+
+def algorithmic_bytes(kernel, n1, n2, n3, lim="MC", tx=1, timeorder=2, fv=False):
     """Compulsory HBM bytes per launch (FP64, state resident; per-(i,j) metric
     amortised over x3).  Units: faces for the flux kernels, zones otherwise.
     tx: transverse zones beyond the grid that the flux loops cover (1; all
@@ -813,19 +834,26 @@ def algorithmic_bytes(kernel, n1, n2, n3, lim="MC", tx=1):
     nd = [n for n in (n1, n2, n3) if n > 1]
     if kernel == "weno5":
         # output cells -1..n along the direction (mean over the directions):
-        # read 8 primitives and the 2 dP/P state pieces, write 16 face values
+        # read 8 primitives and the direction's shock factor, write 16 face values
         cells = sum(zones / n * (n + 2) for n in nd) / len(nd)
-        return cells * (64 + 16 + 128)
+        return cells * (64 + 8 + 128)
     if kernel == "w5_state":
         # zones -2..n+1: read 8 primitives, write 2 state pieces
         ext = 1.0
         for n in (n1, n2, n3):
             ext *= (n + 4) / n if n > 1 else 1.0
         return zones * ext * (64 + 16)
+    if kernel == "w5_shock":
+        # zones -1..n: read rho and the state pieces, write a factor per direction
+        ext = 1.0
+        for n in nd:
+            ext *= (n + 2) / n
+        return zones * ext * (8 + 16 + 8 * len(nd))
     if kernel == "update":
-        # mean of the two substeps: p(64) [+pk 64] + 5 F comps x3 dirs (120) + 3 EMFs (24)
-        # + uf/ucum write (128) [+read 128] + pf (64) + pflag (4)
-        return zones * (468 + 596) / 2.0
+        return zones * update_bytes(len(nd), timeorder, fv)
+    if kernel == "invert":
+        # read the conserved state and the guess, write p_f and the flag
+        return zones * (64 + 64 + 64 + 4)
     if kernel == "emf":
         return zones * (6 * 8 + 3 * 8)
     if kernel == "bound_ghost":
@@ -850,7 +878,8 @@ def fp64_roof(kt, kernel, args):
             "unit": "T FP64 instructions/s",
             "note": "DADD+DMUL+DFMA instructions per launch from ncu over the CUDA-event launch time; peak = "
                     "measured FP64 issue rate of this GPU (the FP64 path is built with -fmad=false for "
-                    "bit-identity, so its FMAs are those inside the IEEE division/sqrt sequences)"}
+                    "bit-identity: its FMAs are those of the divisions and roots and of the shared reciprocals "
+                    "that stand for divisions)"}
 
 
 _FP64_PEAK = None

@@ -1762,12 +1762,13 @@ W5Tile w5_tiling(const Dims &d, const Box &b, int dir) {
 // ---------------------------------------------------------------------------
 enum KernelId {
   K_RESET, K_FLUX, K_FLUX1, K_FLUX2, K_FLUX3, K_EMF, K_UPDATE, K_BOUND_GHOST, K_BOUND_PFLAG, K_CHECK_GAMMA,
-  K_CHECK_RESOLVE, K_FIX_COLLECT, K_FIX_COMPUTE, K_FIX_SCATTER, K_FINALIZE, K_WENO5, K_W5STATE, K_INVERT, K_OTHER, K_NKERNELS
+  K_CHECK_RESOLVE, K_FIX_COLLECT, K_FIX_COMPUTE, K_FIX_SCATTER, K_FINALIZE, K_WENO5, K_W5STATE, K_W5SHOCK, K_INVERT, K_OTHER, K_NKERNELS
 };
 static const char *kKernelNames[K_NKERNELS] = {
     "reset_stage",  "flux",           "flux_x1",         "flux_x2",       "flux_x3",       "emf",           "update",
     "bound_ghost",  "bound_pflag",   "checksol_gamma", "checksol_resolve", "fixup_collect",
-    "fixup_compute", "fixup_scatter",  "finalize",      "weno5",         "w5_state",      "invert",        "other"};
+    "fixup_compute", "fixup_scatter",  "finalize",      "weno5",         "w5_state",      "w5_shock",      "invert",
+    "other"};
 
 struct ProfEvent {
   int kid;
@@ -2357,7 +2358,7 @@ template <typename TW>
 static void launch_w5_state(hgpu_ctx *x, const double *pb) {
   LAUNCH(x, K_W5STATE, w5_state_kernel<TW>, grid_for(x->w5_state_box.size(), 128), 128, x->d, x->P, x->w5_state_box,
          pb, x->G, (TW *)x->w5pu);
-  LAUNCH(x, K_W5STATE, w5_shock_kernel<TW>, grid_for(x->w5_shock_box.size(), 256), 256, x->d, x->w5_shock_box, pb,
+  LAUNCH(x, K_W5SHOCK, w5_shock_kernel<TW>, grid_for(x->w5_shock_box.size(), 256), 256, x->d, x->w5_shock_box, pb,
          (const TW *)x->w5pu, (TW *)x->E);
 }
 
