@@ -2488,9 +2488,12 @@ static bool small_fixup(const hgpu_ctx *x) {
   return (long long)x->d.n1 * x->d.n2 * x->d.n3 <= (x->P.cell_inst ? kSmallBatch : kSmallDomain);
 }
 // Whether the bound kernel of a step also forms checksolution's Lorentz factors.
-// It saves a launch, and costs the active zones the heavier kernel: us a step
-// with / without, 64x64 155 / 168, 97x51x33 450 / 456, 128x64x32 (RK4) 2182 /
-// 2157, 256x128x128 13233 / 12980; a batch's kernel is light (72 / 77 ms).
+// It saves a launch, and costs the active zones the heavier kernel.  Us a step
+// with / without: 64x64 155 / 168, 300x300 283 / 296, 400x400 412 / 421,
+// 97x51x33 (163k) 425 / 427, 100x50x36 (180k) 444 / 441, 64x64x48 (197k) 455 /
+// 454, 96x64x36 (221k) 512 / 510, 64x64x64 554 / 554, 256x128x128 13233 /
+// 12980: from 1.6e5 to 2.6e5 zones within 0.7% either way, and the line lies
+// there.  A batch's kernel is light (72 / 77 ms).
 static bool fused_gamma(const hgpu_ctx *x) {
   return x->P.cell_inst || (long long)x->d.n1 * x->d.n2 * x->d.n3 <= 200000;
 }
