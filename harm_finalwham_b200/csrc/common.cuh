@@ -349,11 +349,12 @@ __device__ __forceinline__ long long dir_stride(const Dims &d) {
 // from each cell's own value and writes FP64 face values (the cell's value
 // plus the FP32 offset), which the FP64 Riemann kernel reads.
 //
-// Bound by instruction issue, FP64 first (FP64 pipe 65-67% active, 240 FP64
-// instructions a cell and primitive).  The form before this one staged tiles
-// of a line in shared memory, one stage at a time between barriers, and held
-// 1.7 other instructions (addresses, shared memory, selects, the branches of
-// its divisions) to an FP64 one: 2.63 -> 1.12 ms a launch on 256x128x128.
+// Bound by instruction issue, FP64 first (issue slots 58-68% and FP64 pipe
+// 56-60% active, about 200 FP64 instructions a cell and primitive).  Staging
+// tiles of a line in shared memory, one stage at a time between barriers,
+// holds 1.7 other instructions (addresses, shared memory, selects, the branches
+// of its divisions) to an FP64 one: 2.63 against 1.09 ms a launch on
+// 256x128x128.
 // The loop stays rolled: unrolled by 2 or 4, to spare the moves of its windows
 // (a fifth of its instructions), it ran 15% and 52% longer.
 // ---------------------------------------------------------------------------
