@@ -965,13 +965,15 @@ __device__ __forceinline__ void checksol_gamma(const Dims &d, const Params &P, c
 // POLEDEATH on the active first/last x2 rows.  A ghost zone that reads such a
 // row is in it itself and zeroes what it read, in any order; only the x1
 // ghosts' inflow check looks at u~2 before that, so the rows' first and last
-// zones, which those ghosts read, wait for the last block.
+// zones, which those ghosts read, wait for the last block; and where the other
+// x2 boundary reads a pole's row for ghosts that are not zeroed (defer), all of
+// its zones do.
 // close: that block also ends the step.  gamma: every zone's Lorentz factor for
 // checksolution follows from what its thread has just written or left, and
 // the threads of the pole rows become threads of all active zones.
 struct BoundJob {
   unsigned n[4];  // threads: x1 ghosts, x2 ghosts (active i), x3 ghosts (active i, j), active pole rows or zones
-  int corners, close;
+  int corners, defer, close;
   GammaJob gamma;
 };
 __global__ void __launch_bounds__(128) bound_kernel(Dims d, Params P, BoundJob J, double *p,
@@ -1017,7 +1019,7 @@ __global__ void __launch_bounds__(128) bound_kernel(Dims d, Params P, BoundJob J
       bound_ghost(d, P, i, j, k, p, G, sc, pflag);
     } else {
       pole = J.corners && ((j == 0 && P.bc[3] == HGPU_BC_POLARAXIS) || (j == d.n2 - 1 && P.bc[2] == HGPU_BC_POLARAXIS));
-      if (pole && i > 0 && i < d.n1 - 1) {
+      if (pole && i > 0 && i < d.n1 - 1 && !J.defer) {
         p[(long long)U2 * d.nz + z] *= 0;
         p[(long long)B2 * d.nz + z] *= 0.;
       }
@@ -1030,14 +1032,16 @@ __global__ void __launch_bounds__(128) bound_kernel(Dims d, Params P, BoundJob J
     }
   }
   if (!(J.corners || J.close) || !last_block(sc)) return;
-  if (J.corners)
-    for (unsigned c = threadIdx.x; c < (unsigned)d.n3 * 4; c += blockDim.x) {
-      const int k = (int)(c >> 2), up = (int)(c & 1), far = (int)((c >> 1) & 1);
-      if (P.bc[up ? 2 : 3] != HGPU_BC_POLARAXIS || (far && d.n1 == 1)) continue;
-      const long long z = zix(d, far ? d.n1 - 1 : 0, up ? d.n2 - 1 : 0, k);
+  if (J.corners) {
+    const unsigned columns = J.defer ? d.n1 : 2;
+    for (unsigned c = threadIdx.x; c < columns * 2 * d.n3; c += blockDim.x) {
+      const int k = (int)(c % d.n3), q = (int)(c / d.n3), up = q & 1, i = J.defer ? q >> 1 : (q >> 1) * (d.n1 - 1);
+      if (P.bc[up ? 2 : 3] != HGPU_BC_POLARAXIS || (q >> 1 && d.n1 == 1)) continue;
+      const long long z = zix(d, i, up ? d.n2 - 1 : 0, k);
       p[(long long)U2 * d.nz + z] *= 0;
       p[(long long)B2 * d.nz + z] *= 0.;
     }
+  }
   if (J.close) close_step(P, sc);
 }
 
@@ -2520,6 +2524,11 @@ static void launch_bound(hgpu_ctx *x, double *pv, bool flags = false, bool close
   J.n[1] = (unsigned)d.n1 * 2 * d.g2 * d.nt3;
   J.n[2] = (unsigned)d.n1 * d.n2 * 2 * d.g3;
   J.corners = d.n2 > 1 && (x->P.bc[2] == HGPU_BC_POLARAXIS || x->P.bc[3] == HGPU_BC_POLARAXIS);
+  // a periodic boundary reads the row of the other side, a reflecting one of a
+  // grid as narrow as its ghosts too
+  auto reads_far = [&](int bc) { return bc == HGPU_BC_PERIODIC || (bc == HGPU_BC_POLARAXIS_FLIP && d.n2 <= d.g2); };
+  J.defer = J.corners && ((x->P.bc[3] == HGPU_BC_POLARAXIS && reads_far(x->P.bc[2])) ||
+                          (x->P.bc[2] == HGPU_BC_POLARAXIS && reads_far(x->P.bc[3])));
   J.n[3] = gamma ? (unsigned)d.n1 * d.n2 * d.n3 : (J.corners ? (unsigned)d.n1 * 2 * d.n3 : 0);
   J.close = close;
   J.gamma = gj;
