@@ -2936,6 +2936,8 @@ static int utoprim_batch_impl(const double *U, const double *gcov, const double 
     if (iters) *iters = 0;
     return HGPU_OK;
   }
+  // (no device holds so many; below, the byte count of the one allocation cannot wrap)
+  if (n > (1LL << 40)) return HGPU_E_NOMEM;
   // one allocation: cudaMalloc and cudaFree take about 0.18 ms each here, and
   // one of either for every array was 2.5 ms of an 8 ms call on 1e5 zones
   double *base = nullptr;

@@ -168,3 +168,17 @@ def test_active_zone_transfers_keep_the_run_bit_identical(name):
         assert same(g.active(pg), pa) and np.array_equal(g.active(fg), fa) and tg == ta and dtg == dta
         ph, fh, _, _ = h.download_state()
         assert same(pg, ph)
+
+
+def test_an_inversion_batch_beyond_any_device_is_refused():
+    # 396 bytes a zone: a count at which the size of the one allocation wraps
+    import ctypes
+
+    from harm_finalwham_b200.gpu import load_library
+    L = load_library()
+    one = (ctypes.c_double * 16)()
+    flag = (ctypes.c_int * 1)()
+    n = 2 ** 64 // 396 + 1
+    rc = L.hgpu_utoprim_batch(one, one, one, one, one, flag, ctypes.c_longlong(n), ctypes.c_double(4.0 / 3.0),
+                              ctypes.c_double(100.0), None)
+    assert rc == 4  # HGPU_E_NOMEM
