@@ -666,7 +666,7 @@ __global__ void finalize_batch_kernel(Params P, int advance_time) {
 // one block: before a stage, or at the start of a call of steps (call: what
 // accumulates over a call, as clear_counters; each stage clears its counts)
 __global__ void reset_stage_kernel(Params P, Scalars *sc, int call) {
-  clear_ndt(P, sc, threadIdx.x, blockDim.x);
+  if (!call) clear_ndt(P, sc, threadIdx.x, blockDim.x);
   if (threadIdx.x != 0) return;
   if (!call) {
     clear_stage_counts(sc);
@@ -680,15 +680,13 @@ __global__ void reset_stage_kernel(Params P, Scalars *sc, int call) {
   }
 }
 
-// the dt update that closes a step, by the last kernel's last block; the dt
-// minima are left for the next step's first stage
+// the dt update that closes a step, by the last kernel's last block (the dt
+// minima stay, for who asks for them after the step)
 __device__ __forceinline__ void close_step(const Params &P, Scalars *sc) {
   if (P.cell_inst)
     for (int b = threadIdx.x; b < P.ninst; b += blockDim.x) finalize_inst(P, b, 1);
   else if (threadIdx.x == 0)
     finalize_one(P, sc, 1);
-  __syncthreads();
-  clear_ndt(P, sc, threadIdx.x, blockDim.x);
 }
 
 // whether this block is the last of the grid to come here: everything that
@@ -2697,9 +2695,11 @@ static void launch_stage(hgpu_ctx *x, int timeorder) {
 
 // One time step within a run of steps: the resets and the dt update ride on
 // kernels that are there anyway (before the first step of a run,
-// launch_reset(x, true); after the last the dt minima are cleared).
+// launch_reset(x, true)).  The first stage's EMFs clear the dt minima for the
+// last stage; a scheme of one stage has no such kernel before its faces.
 static void launch_step(hgpu_ctx *x) {
   const int norders = num_orders(x);
+  if (norders == 1) launch_reset(x);
   for (int o = 0; o < norders; o++) {
     launch_stage_advance(x, o, true);
     launch_stage_fixup(x, o, true);

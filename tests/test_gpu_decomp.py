@@ -157,3 +157,26 @@ def test_two_processes_through_the_collective_transport_match_whole_domain():
     assert _same_bits(p_s, p_w)
     assert np.array_equal(f_s, f_w)
     assert sum(out[r][4] for r in range(world)) == st_w.newton_iters
+
+
+@pytest.mark.parametrize("timeorder", [1, 2, 3])
+def test_dt_minima_after_a_whole_step_are_its_last_stages(timeorder):
+    import torch
+    dom = _torus((24, 16, 12), 3, "MC", "HLL", timeorder=timeorder)
+    out = []
+    for phases in (False, True):
+        ndt = torch.zeros(3, dtype=torch.int64, device="cuda")
+        with HarmGPU.from_problem(dom) as g:
+            g.bound_prim()
+            g.init_dt()
+            g.step_ch(1)
+            if phases:
+                for s in range(timeorder):
+                    assert g.L.hgpu_stage_advance(g.h, s) == 0 and g.L.hgpu_stage_fixup(g.h, s) == 0
+                # (one context holds the whole azimuth: its x3 ghosts are its own)
+            else:
+                g.step_ch(1)
+            assert g.L.hgpu_ndt_pack(g.h, ndt.data_ptr()) == 0
+            g.sync()
+            out.append(ndt.cpu().numpy().view(np.float64))
+    assert np.array_equal(out[0], out[1]) and np.all(out[0] < 1e49)  # (1e50: no face counted)
